@@ -34,6 +34,7 @@
 // written as zeros, the tensor memory is freed and kErrMmaWait is raised in
 // the caller's error word.
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <mutex>
 
@@ -81,9 +82,17 @@ __device__ __forceinline__ uint64_t sdesc(const void* p) {
          (1ull << 46);
 }
 
-// instruction descriptor: BF16 × BF16 → F32, both K-major, M = 128, N = 128
-__host__ __device__ constexpr uint32_t idesc(bool negA) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((negA ? 1u : 0u) << 13) | ((uint32_t)(kTN >> 3) << 17) |
+// Operand modes.  kF16 serves operands whose values are at most 1 (the scaled
+// eigenvectors), times 2¹⁰: hi = bf16(v), exact in FP16, and lo = fp16(v − hi),
+// three bits more than a BF16 lo at the same number of MMAs, so that what is
+// left out of v shrinks from 2⁻¹⁷ to 2⁻²⁰ of it; the product is scaled back by
+// 2⁻²⁰.  Fixed range, so not for image data.
+enum Mode { kBf16 = 0, kTf32 = 1, kF16 = 2 };
+constexpr float kF16Scale = 1024.f;
+
+// instruction descriptor: BF16 × BF16 (F16 × F16) → F32, both K-major, M = 128, N = 128
+__host__ __device__ constexpr uint32_t idesc(bool negA, bool f16 = false) {
+  return (1u << 4) | (f16 ? 0u : (1u << 7) | (1u << 10)) | ((negA ? 1u : 0u) << 13) | ((uint32_t)(kTN >> 3) << 17) |
          ((uint32_t)(kTM >> 4) << 24);
 }
 
@@ -144,6 +153,16 @@ __device__ __forceinline__ void split_pair(float x0, float x1, uint32_t& hi, uin
   const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
   const float2 hf = __bfloat1622float2(h);
   const __nv_bfloat162 l = __floats2bfloat162_rn(x0 - hf.x, x1 - hf.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+__device__ __forceinline__ void split_pair_f16(float x0, float x1, uint32_t& hi, uint32_t& lo) {
+  x0 *= kF16Scale;
+  x1 *= kF16Scale;
+  const float2 hf = __bfloat1622float2(__floats2bfloat162_rn(x0, x1));
+  const __half2 h = __floats2half2_rn(hf.x, hf.y);
+  const __half2 l = __floats2half2_rn(x0 - hf.x, x1 - hf.y);
   hi = *reinterpret_cast<const uint32_t*>(&h);
   lo = *reinterpret_cast<const uint32_t*>(&l);
 }
@@ -209,6 +228,7 @@ __device__ __forceinline__ void load_chunk(Chunk& ch, const cf* __restrict__ bas
 }
 
 // chunk → planar hi / lo tiles (re_h, re_l, im_h, im_l), conjugated when conj
+template <bool F16>
 __device__ __forceinline__ void store_chunk(const Chunk& ch, uint32_t* rh, uint32_t* rl,
                                             uint32_t* ih, uint32_t* il, bool conj) {
 #pragma unroll
@@ -219,19 +239,21 @@ __device__ __forceinline__ void store_chunk(const Chunk& ch, uint32_t* rh, uint3
     const cf a = ch.v[i][0], b = ch.v[i][1];
     const float ai = conj ? -a.y : a.y, bi = conj ? -b.y : b.y;
     uint32_t h, l;
-    split_pair(a.x, b.x, h, l);
+    if constexpr (F16) split_pair_f16(a.x, b.x, h, l);
+    else split_pair(a.x, b.x, h, l);
     rh[w] = h;
     rl[w] = l;
-    split_pair(ai, bi, h, l);
+    if constexpr (F16) split_pair_f16(ai, bi, h, l);
+    else split_pair(ai, bi, h, l);
     ih[w] = h;
     il[w] = l;
   }
 }
 
 // One operand chunk into stage `stage` (B operand when isB), conjugated when conj.
-template <bool TF>
+template <int MODE>
 __device__ __forceinline__ void store_operand(const Chunk& ch, uint32_t* stage, bool isB, bool conj) {
-  if constexpr (TF) {
+  if constexpr (MODE == kTf32) {
     uint32_t* re = stage + (isB ? 2 : 0) * kTfPlane;
     uint32_t* im = stage + (isB ? 3 : 1) * kTfPlane;
 #pragma unroll
@@ -245,20 +267,20 @@ __device__ __forceinline__ void store_operand(const Chunk& ch, uint32_t* stage, 
     }
   } else {
     const int o = isB ? BR_H : AR_H;
-    store_chunk(ch, stage + (o + 0) * (kTile / 2), stage + (o + 1) * (kTile / 2),
+    store_chunk<MODE == kF16>(ch, stage + (o + 0) * (kTile / 2), stage + (o + 1) * (kTile / 2),
                 stage + (o + 2) * (kTile / 2), stage + (o + 3) * (kTile / 2), conj);
   }
 }
 
 // The 12 MMAs of one 16-element K step t of stage s.
-template <bool GRAM>
+template <bool GRAM, bool F16>
 __device__ __forceinline__ void issue_step(const USmem& s, int st, int t, uint32_t dre, uint32_t dim,
                                            bool acc, bool bSameAsA) {
   const uint32_t* o = &s.op[st][0][0];
   auto A = [&](int k) { return sdesc(o + k * (kTile / 2) + t * 64); };   // +2 cores = 256 B = 64 words
   const int bro = bSameAsA ? AR_H : BR_H;   // B operands: same tiles as A on diagonal Gram tiles
   auto B = [&](int k) { return sdesc(o + (bro + (k - BR_H)) * (kTile / 2) + t * 64); };
-  constexpr uint32_t P = idesc(false), N = idesc(true);
+  constexpr uint32_t P = idesc(false, F16), N = idesc(true, F16);
   // real part
   umma(dre, A(AR_H), B(BR_H), P, acc);
   umma(dre, A(AR_H), B(BR_L), P, true);
@@ -285,10 +307,10 @@ __device__ __forceinline__ void issue_step(const USmem& s, int st, int t, uint32
 }
 
 // All MMAs of the chunk in stage st (first: the accumulators start from zero).
-template <bool GRAM, bool TF>
+template <bool GRAM, int MODE>
 __device__ __forceinline__ void issue_chunk(const USmem& s, int st, uint32_t dre, uint32_t dim,
                                             bool first, bool bSameAsA) {
-  if constexpr (TF) {
+  if constexpr (MODE == kTf32) {
     const uint32_t* o = &s.op[st][0][0];
     const int br = bSameAsA ? 0 : 2, bi = bSameAsA ? 1 : 3;
     constexpr uint32_t P = idesc_tf(false), N = idesc_tf(true);
@@ -309,8 +331,8 @@ __device__ __forceinline__ void issue_chunk(const USmem& s, int st, uint32_t dre
       }
     }
   } else {
-    issue_step<GRAM>(s, st, 0, dre, dim, !first, bSameAsA);
-    issue_step<GRAM>(s, st, 1, dre, dim, true, bSameAsA);
+    issue_step<GRAM, MODE == kF16>(s, st, 0, dre, dim, !first, bSameAsA);
+    issue_step<GRAM, MODE == kF16>(s, st, 1, dre, dim, true, bSameAsA);
   }
 }
 
@@ -339,7 +361,7 @@ struct Pending {
 // Main loop shared by both kernels: nch chunks; kofs(c, buf) fills s.kof[buf]
 // for chunk c (threads < 32); load(c, buf) loads chunk c's operands into
 // registers (A, and B unless bSameAsA); returns false when a wait timed out.
-template <bool GRAM, bool TF, class KOfs, class Load>
+template <bool GRAM, int MODE, class KOfs, class Load>
 __device__ __forceinline__ bool mainloop(USmem& s, int nch, Chunk& ca, Chunk& cb, bool conjA,
                                          bool conjB, bool bSameAsA, const KOfs& kofs,
                                          const Load& load, int polls) {
@@ -355,15 +377,15 @@ __device__ __forceinline__ bool mainloop(USmem& s, int nch, Chunk& ca, Chunk& cb
       else ok = false;
     }
     if (ok) {
-      store_operand<TF>(ca, &s.op[st][0][0], false, conjA);
-      if (!bSameAsA) store_operand<TF>(cb, &s.op[st][0][0], true, conjB);
+      store_operand<MODE>(ca, &s.op[st][0][0], false, conjA);
+      if (!bSameAsA) store_operand<MODE>(cb, &s.op[st][0][0], true, conjB);
     }
     fence_async_smem();
     __syncthreads();
     if (c + 1 < nch) load(c + 1, (c + 1) & 1);
     if (tid == 0 && ok) {
       tc_fence_after();
-      issue_chunk<GRAM, TF>(s, st, s.tmem, s.tmem + kTN, c == 0, bSameAsA);
+      issue_chunk<GRAM, MODE>(s, st, s.tmem, s.tmem + kTN, c == 0, bSameAsA);
       umma_commit(&s.bar[st]);
       pend.committed(c);
     }
@@ -406,10 +428,12 @@ __device__ __forceinline__ void tmem_free(USmem& s) {
 }
 
 // ---------------------------------------------------------------------------
-template <bool TF>
+// kcols (or null): the patch's contraction stops at kcols[ip] values (the
+// eigenvectors beyond the rank are zero).
+template <int MODE>
 __global__ void __launch_bounds__(kThr, 1)
     k_gram_umma(const cf* __restrict__ img, PatchMap m, cf* __restrict__ out, int nsplit,
-                int lchunk, DevWait dw) {
+                int lchunk, const int* __restrict__ kcols, DevWait dw) {
   extern __shared__ __align__(1024) unsigned char smraw[];
   USmem& s = *reinterpret_cast<USmem*>(smraw);
   int t = blockIdx.x, ta = 0;
@@ -425,7 +449,7 @@ __global__ void __launch_bounds__(kThr, 1)
   const int64_t ts = tstride(m);
   const int a0 = ta * kTM, b0 = tb * kTN;
   const int l_begin = split * lchunk;
-  const int l_end = min(m.L, l_begin + lchunk);
+  const int l_end = min(kcols ? kcols[ip] : m.L, l_begin + lchunk);
   const int n = m.n;
   const int nch = l_end > l_begin ? (l_end - l_begin + kKc - 1) / kKc : 0;
   tmem_alloc(s);
@@ -451,7 +475,7 @@ __global__ void __launch_bounds__(kThr, 1)
     load_chunk(ca, base, s.rowA, s.kof[buf]);
     if (!diag) load_chunk(cb, base, s.rowB, s.kof[buf]);
   };
-  const bool ok = mainloop<true, TF>(s, nch, ca, cb, cj, cj, diag, kofs, load, dw.polls);
+  const bool ok = mainloop<true, MODE>(s, nch, ca, cb, cj, cj, diag, kofs, load, dw.polls);
   cf* G = out + ((nsplit > 1) ? (int64_t)split * n * n : ip * (int64_t)n * n);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int a = a0 + (warp & 3) * 32 + lane;
@@ -475,7 +499,8 @@ __global__ void __launch_bounds__(kThr, 1)
         for (int j = 0; j < 16; ++j) {
           const int b = b0 + col + j;
           if (b < n) {
-            const cf v = make_float2(re[j], im[j]);
+            constexpr float sc = MODE == kF16 ? 1.f / (kF16Scale * kF16Scale) : 1.f;
+            const cf v = make_float2(re[j] * sc, im[j] * sc);
             G[(int64_t)b * n + a] = v;
             if (!diag) G[(int64_t)a * n + b] = cconj(v);
           }
@@ -487,7 +512,7 @@ __global__ void __launch_bounds__(kThr, 1)
 }
 
 // ---------------------------------------------------------------------------
-template <bool TF>
+template <int MODE>
 __global__ void __launch_bounds__(kThr, 1)
     k_rebuild_umma(const cf* __restrict__ img, const cf* __restrict__ W, PatchMap m,
                    cf* __restrict__ out, int direct, DevWait dw) {
@@ -535,7 +560,7 @@ __global__ void __launch_bounds__(kThr, 1)
     }
     load_chunk(cb, img + org, s.rowB, s.kof[buf]);
   };
-  const bool ok = mainloop<false, TF>(s, nch, ca, cb, true, m.tall != 0, false, kofs, load, dw.polls);
+  const bool ok = mainloop<false, MODE>(s, nch, ca, cb, true, m.tall != 0, false, kofs, load, dw.polls);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int a = a0 + (warp & 3) * 32 + lane;
   // on a time-out the output tile is written as zeros and the error raised
@@ -589,28 +614,26 @@ int umma_prepare() {
   MSLR_CUDA_TRY(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(mu);
   if (dev < 64 && done[dev]) return MSLR_OK;
-  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_gram_umma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(USmem)));
-  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_rebuild_umma<false>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(USmem)));
-  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_gram_umma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(USmem)));
-  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_rebuild_umma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(USmem)));
+  for (const void* k : {reinterpret_cast<const void*>(&k_gram_umma<kBf16>), reinterpret_cast<const void*>(&k_gram_umma<kTf32>),
+                        reinterpret_cast<const void*>(&k_gram_umma<kF16>), reinterpret_cast<const void*>(&k_rebuild_umma<kBf16>),
+                        reinterpret_cast<const void*>(&k_rebuild_umma<kTf32>)})
+    MSLR_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(USmem)));
   if (dev < 64) done[dev] = true;
   return MSLR_OK;
 }
 
 int gram_umma_launch(const cf* img, const PatchMap& m, int64_t np, cf* out_or_part, int nsplit,
-                     int lchunk, const DevWait& dw, cudaStream_t st, bool tf32) {
+                     int lchunk, const DevWait& dw, cudaStream_t st, bool tf32, const int* kcols) {
   if (int rc = umma_prepare()) return rc;
   const int T = (m.n + kTM - 1) / kTM;
   const int ntri = T * (T + 1) / 2;
   const dim3 grid(ntri, (unsigned)np, nsplit);
   if (tf32)
-    k_gram_umma<true><<<grid, kThr, sizeof(USmem), st>>>(img, m, out_or_part, nsplit, lchunk, dw);
+    k_gram_umma<kTf32><<<grid, kThr, sizeof(USmem), st>>>(img, m, out_or_part, nsplit, lchunk, kcols, dw);
+  else if (kcols)
+    k_gram_umma<kF16><<<grid, kThr, sizeof(USmem), st>>>(img, m, out_or_part, nsplit, lchunk, kcols, dw);
   else
-    k_gram_umma<false><<<grid, kThr, sizeof(USmem), st>>>(img, m, out_or_part, nsplit, lchunk, dw);
+    k_gram_umma<kBf16><<<grid, kThr, sizeof(USmem), st>>>(img, m, out_or_part, nsplit, lchunk, nullptr, dw);
   MSLR_CUDA_TRY(cudaGetLastError());
   return MSLR_OK;
 }
@@ -620,9 +643,9 @@ int rebuild_umma_launch(const cf* img, const cf* W, const PatchMap& m, int64_t n
   if (int rc = umma_prepare()) return rc;
   const dim3 grid((m.n + kTM - 1) / kTM, (m.L + kTN - 1) / kTN, (unsigned)np);
   if (tf32)
-    k_rebuild_umma<true><<<grid, kThr, sizeof(USmem), st>>>(img, W, m, out, direct, dw);
+    k_rebuild_umma<kTf32><<<grid, kThr, sizeof(USmem), st>>>(img, W, m, out, direct, dw);
   else
-    k_rebuild_umma<false><<<grid, kThr, sizeof(USmem), st>>>(img, W, m, out, direct, dw);
+    k_rebuild_umma<kBf16><<<grid, kThr, sizeof(USmem), st>>>(img, W, m, out, direct, dw);
   MSLR_CUDA_TRY(cudaGetLastError());
   return MSLR_OK;
 }

@@ -58,7 +58,8 @@ __device__ __forceinline__ cf m_elem(const PatchMap& m, const cf* __restrict__ i
 // umma_supported: the 32-bit offset tables of those kernels cover this map.
 bool umma_supported(const PatchMap& m);
 int gram_umma_launch(const cf* img, const PatchMap& m, int64_t np, cf* out_or_part, int nsplit,
-                     int lchunk, const DevWait& dw, cudaStream_t st, bool tf32 = false);
+                     int lchunk, const DevWait& dw, cudaStream_t st, bool tf32 = false,
+                     const int* kcols = nullptr);
 int rebuild_umma_launch(const cf* img, const cf* W, const PatchMap& m, int64_t np, cf* out,
                         int direct, const DevWait& dw, cudaStream_t st, bool tf32 = false);
 int umma_prepare();

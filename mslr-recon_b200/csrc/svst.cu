@@ -312,8 +312,9 @@ struct WorkPtrs {
 
 // Gram matrices of all patches described by m into w.gram.
 // Tensor cores (tc, tuned form: split-precision BF16 mma) or FP32 SIMT.
+// kcols (tensor cores only): per-patch contraction lengths, operands at most 1 in magnitude.
 int svst_gram(const cf* in, const PatchMap& m, int64_t np, const WorkPtrs& w, int nsplit, int tc,
-              const DevWait& dw, cudaStream_t st, uint64_t* launches) {
+              const DevWait& dw, cudaStream_t st, uint64_t* launches, const int* kcols = nullptr) {
   if (launches) *launches += (nsplit > 1 ? 2 : 1);
   const int n = m.n;
   const int T = (n + kTile - 1) / kTile;
@@ -321,7 +322,7 @@ int svst_gram(const cf* in, const PatchMap& m, int64_t np, const WorkPtrs& w, in
   const int lchunk = (nsplit > 1) ? ((m.L + nsplit - 1) / nsplit + 31) / 32 * 32 : m.L;
   cf* dst = (nsplit > 1) ? w.part : w.gram;
   if (tc && umma_supported(m)) {
-    if (int rc = gram_umma_launch(in, m, np, dst, nsplit, lchunk, dw, st, tc == 2)) return rc;
+    if (int rc = gram_umma_launch(in, m, np, dst, nsplit, lchunk, dw, st, tc == 2, kcols)) return rc;
   } else {
     k_gram<<<dim3(ntri, (unsigned)np, nsplit), 256, 0, st>>>(in, m, dst, nsplit, lchunk);
   }
@@ -357,7 +358,7 @@ int svst_form_w(const WorkPtrs& w, int n, int64_t np, int tc, const DevWait& dw,
   vm.L = n;
   vm.nvox = n;
   vm.mstride = (int64_t)n * n;
-  return svst_gram(reinterpret_cast<const cf*>(w.zv), vm, np, w, 1, tc, dw, st, launches);
+  return svst_gram(reinterpret_cast<const cf*>(w.zv), vm, np, w, 1, tc, dw, st, launches, w.rank);
 }
 
 // Gram → eig → W → (rebuild into out or pbuf) for all patches described by m.
