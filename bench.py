@@ -489,11 +489,12 @@ def main():
         phases["normal_op_kernel_ms"] = kms
         phases["normal_op_launches_per_kernel"] = nl
     if kms and "pfwd" in kms:
+        fr = Nt * -(-Nc // ch) / nl   # frames per launch
         per = RL.four_pass_kernels(pb["N"], ch, fr)
         names = {"pfwd": "k_pfwd (forward plane pass: coil map x summed image, DFT_y, DFT_x)",
-                 "zmask": "k_zmask (z pass: DFT_z, k-space mask, inverse DFT_z)",
-                 "padj": "k_padj (inverse plane pass: inverse DFT_y, DFT_x, x conj(coil map))",
-                 "csum": "k_csum (coil combine into g)"}
+                 "zmask": "k_lcol (z pass: DFT_z, k-space mask, inverse DFT_z)",
+                 "padj": "k_padj (inverse plane pass: inverse DFT_x, DFT_y)",
+                 "csum": "k_csum (coil combine into g: sum of conj(coil map) x image)"}
         dom = max(("pfwd", "zmask", "padj"), key=lambda k: kms[k])
         tdom = kms[dom] / 1e3
         byts, fl = per[dom]["bytes"], per[dom]["flops"]

@@ -193,9 +193,9 @@ class MSLRContext:
     def normal_profile(self, X: torch.Tensor, out=None, stream=None):
         """One normal operator with events around every kernel of every chunk:
         returns ({kernel: average ms per launch}, launches of each).  Kernels of
-        the four-pass form: "pfwd" (forward plane pass), "zmask" (z pass with
-        the mask), "padj" (inverse plane pass), "csum" (coil combine); of the
-        three-kernel form: "zfwd", "xy", "zadj"."""
+        the register-line form: "pfwd" (forward plane pass), "zmask" (z pass
+        with the mask), "padj" (inverse plane pass), "csum" (coil combine); of
+        the three-kernel form: "zfwd", "xy", "zadj"."""
         import ctypes as C
         if X.dim() == 4:
             X = X.unsqueeze(0)

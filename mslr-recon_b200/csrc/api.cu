@@ -86,6 +86,7 @@ static void free_ctx(mslr_ctx* c) {
   if (c->d_gbuf) cudaFree(c->d_gbuf);
   if (c->d_vjpw) cudaFree(c->d_vjpw);
   if (c->d_xsum) cudaFree(c->d_xsum);
+  if (c->d_mz) cudaFree(c->d_mz);
   if (c->d_pthr) cudaFree(c->d_pthr);
   if (c->sn_stream) cudaStreamDestroy(c->sn_stream);
   if (c->sn_fork) cudaEventDestroy(c->sn_fork);
@@ -599,8 +600,9 @@ int mslr_get_tuning(const mslr_ctx* ctx, int32_t* values, int32_t cap, int32_t* 
   std::vector<int32_t> v = {ctx->spec_ch, ctx->spec_fr};
   for (const auto& g : ctx->scales) v.push_back(g.nsplit_tuned > 0 ? g.nsplit_tuned : 0);
   v.push_back(ctx->spec_lanes);
-  v.push_back(ctx->spec_zmask_var == 1 ? 1 : 2);
-  v.push_back(ctx->spec_zmask_warps[ctx->spec_zmask_var]);
+  // the z pass: two or more resident CTAs per SM of four warps, not tuned
+  v.push_back(2);
+  v.push_back(4);
   for (const auto& g : ctx->scales) v.push_back(g.n > 384 || g.eig_big ? 1024 : 384);
   *count = (int32_t)v.size();
   for (int32_t i = 0; i < cap && i < (int32_t)v.size(); ++i) values[i] = v[i];

@@ -91,23 +91,18 @@ struct Ctx {
   int spec_ch = 6;        // coils per group of the specialised normal operator (autotuned)
   int spec_fr = 2;        // frames per chunk (autotuned)
   int spec_zfwd_ctas = 0; // resident CTAs of the specialised forward z kernel
-  // four-pass form of the specialised normal operator (default; MSLR_SENSE_PATH=3
-  // selects the three-kernel form): resident CTAs of its kernels, and the
-  // summed image Σ_k X_k of all frames that its forward plane pass reads
-  bool spec_four = true;
-  int spec_pfwd_ctas = 0, spec_zmask_ctas = 0, spec_padj_ctas = 0;
-  // z-mask kernel variant: 0 two CTAs per SM (64 registers), 1 one CTA per SM
-  // (MSLR_ZMASK_CTAS=1), 2 two CTAs per SM with fewer warps (more registers)
-  int spec_zmask_var = 0;
-  int spec_zmask_ctas_v[3] = {0, 0, 0};   // resident CTAs of each variant
-  int spec_zmask_warps[3] = {0, 0, 0};    // warps per CTA of each variant
-  // chunks of the four-pass form alternate between two streams ("lanes",
+  // MSLR_SENSE_PATH=3: the three-kernel form of sense_spec.cu for the normal operator
+  bool spec_three = false;
+  // chunks of the register-line form alternate between two streams ("lanes",
   // each with its own k-space buffer) when spec_lanes == 2 (the default;
   // MSLR_SENSE_LANES=1 keeps one), so one chunk's kernels overlap the other's
   int spec_lanes = 1;
   cudaStream_t sn_stream = nullptr;
   cudaEvent_t sn_fork = nullptr, sn_join = nullptr;
-  cf* d_xsum = nullptr;   // (Nt, nvox)
+  cf* d_xsum = nullptr;   // (Nt, nvox) summed image Σ_k X_k
+  // register-line SENSE kernels (sense_line.cu): every axis a 5-smooth length of 8..96
+  bool line = false;
+  uint32_t* d_mz = nullptr;   // sample bits over z: (Nt, ⌈Nz/32⌉, Ny·Nx)
   bool xy_tc = false;     // tensor-core plane pass (DFT products on tcgen05)
   uint32_t* d_dft = nullptr;   // its split-BF16 DFT matrix tiles
   // graph-captured POGM step (tuned form): captured on a private stream the
@@ -202,6 +197,16 @@ bool sense_spec_setup(Ctx* c);
 int normal_op_spec(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool subtract,
                    cudaStream_t st);
 
+// ---- sense_line.cu (tuned form, 5-smooth axes) -------------------------------------
+bool sense_line_setup(Ctx* c);
+int sense_line_bind(Ctx* c, cudaStream_t st);
+int normal_op_line(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool subtract,
+                   cudaStream_t st);
+int sense_forward_line(Ctx* c, const cf* x, cf* y, cudaStream_t st);
+int sense_adjoint_line(Ctx* c, const cf* y, cf* x, cudaStream_t st);
+int image_sum(Ctx* c, const cf* X, int ns, int64_t sstride, cf* out, cudaStream_t st);   // Σ_k X_k (sense_spec.cu)
+int prof_mark(Ctx* c, cudaStream_t st);
+
 // ---- svst.cu -----------------------------------------------------------------
 int svst_setup(Ctx* c);   // workspaces (create time)
 // img_out = patchSVST(img_in) for scale s with threshold (*thr_dev) * lam
@@ -268,7 +273,6 @@ int set_scalar(double* dst, double v, cudaStream_t st);
 // ---- autotuner (api.cu; sense_spec.cu, svst.cu) ---------------------------------
 int tune_sense_chunks(Ctx* c, cudaStream_t st);
 int tune_svst_splits(Ctx* c, cudaStream_t st);
-int tune_sense_variants(Ctx* c, cudaStream_t st);
 int tune_eig_variants(Ctx* c, cudaStream_t st);
 int autotune(Ctx* c, cudaStream_t st);
 // milliseconds per call of fn(), timed with events on st after one warm-up call

@@ -344,6 +344,7 @@ int sense_setup_tables(Ctx* c) {
   if (c->tuned()) {
     c->fast = sense_fast_setup(c);
     c->spec = c->fast && sense_spec_setup(c);
+    c->line = sense_line_setup(c);
   }
   c->Ffast = 1;
   return MSLR_OK;
@@ -372,6 +373,7 @@ int sense_bind(Ctx* c, const cf* smaps, const cf* y, const int32_t* idx, int bas
   k_modmaps<<<1184, 256, 0, st>>>(smaps, c->d_smaps_mod, c->d_mod[0], c->d_mod[1], c->d_mod[2], d);
   MSLR_CUDA_TRY(cudaGetLastError());
   c->bound = true;
+  if (c->line && (rc = sense_line_bind(c, st))) return rc;
   rc = sense_adjoint(c, y, c->d_ahy, st);
   if (!rc) rc = data_norm2(c, y, &c->ynorm2, st);   // ‖y‖² for dc_cost (cost.cu)
   if (rc) {
@@ -382,6 +384,7 @@ int sense_bind(Ctx* c, const cf* smaps, const cf* y, const int32_t* idx, int bas
 }
 
 int sense_forward(Ctx* c, const cf* x, cf* y, cudaStream_t st) {
+  if (c->line) return sense_forward_line(c, x, y, st);
   if (c->fast) return sense_forward_fast(c, x, y, st);
   const Dims d = dims_of(c);
   const float s = (float)(1.0 / std::sqrt((double)c->nvox));
@@ -402,6 +405,7 @@ int sense_forward(Ctx* c, const cf* x, cf* y, cudaStream_t st) {
 }
 
 int sense_adjoint(Ctx* c, const cf* y, cf* x, cudaStream_t st) {
+  if (c->line) return sense_adjoint_line(c, y, x, st);
   if (c->fast) return sense_adjoint_fast(c, y, x, st);
   const Dims d = dims_of(c);
   const float s = (float)(1.0 / std::sqrt((double)c->nvox));
@@ -425,6 +429,7 @@ int sense_adjoint(Ctx* c, const cf* y, cf* x, cudaStream_t st) {
 int normal_op(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool subtract,
               cudaStream_t st) {
   if (c->spec) return normal_op_spec(c, X, ns, sstride, g, subtract, st);
+  if (c->line) return normal_op_line(c, X, ns, sstride, g, subtract, st);
   if (c->fast) return normal_op_fast(c, X, ns, sstride, g, subtract, st);
   const Dims d = dims_of(c);
   const float scale = (float)(1.0 / (double)c->nvox);

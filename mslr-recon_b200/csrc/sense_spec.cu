@@ -1,4 +1,6 @@
-// sense_spec.cu — shape-specialised tuned SENSE normal operator.
+// sense_spec.cu — shape-specialised SENSE normal operator in three kernels
+// (MSLR_SENSE_PATH=3; the default is the register-line form of sense_line.cu)
+// and its tensor-core plane pass (MSLR_XY_PATH=tc).
 //
 // Same decomposition as sense_fast.cu (z pass | xy pass with the k-space mask
 // | z pass with the coil combine; the centring identity is in the header of
@@ -76,43 +78,11 @@ struct Shape {
   static constexpr int ev(int n) { return (n + 1) & ~1; }
   // warps of the adjoint z kernel (two CTAs per SM): at most 16
   static constexpr int ZW2 = mn(16, cdiv(NX, AZ::LPW));
-  // fewer warps for the z-mask kernel's third variant (more registers per
-  // thread at two CTAs per SM): the most, at most 12, whose compute warps
-  // divide the slab's line groups evenly (warp 0 then only moves slabs)
-  static constexpr int zwm(int g) {
-    int w = 12;
-    while (w > 2 && g % (w - 1) != 0) --w;
-    return (w > 2) ? w : mn(12, g);
-  }
-  static constexpr int ZWm = mn(ZW2, zwm(cdiv(NX, AZ::LPW)));
   static constexpr size_t smem_zfwd = sizeof(cf) * (4 * (size_t)S + ev(NZ)) + 3 * sizeof(uint64_t);
   static constexpr size_t smem_zadj = sizeof(cf) * (2 * (size_t)S + ev(NZ)) + sizeof(uint64_t);
   static constexpr size_t smem_xy =
       sizeof(cf) * (2 * (size_t)PL + ev(NX) + ev(NY)) + MW * sizeof(uint32_t) + sizeof(uint64_t);
-  // four-pass form.  The plane kernels' work plane W (filled and read only by
-  // their own passes, never by a bulk copy) has an odd row stride PW, and the
-  // lines of a warp are spread over the plane (line l of group g is row or
-  // column g + D·l, D = n / LPW): with NX = 90 the column passes' strided
-  // accesses then fall on distinct shared-memory banks far more often than
-  // with rows of 90 complex values at neighbouring lines.
-  static constexpr int PW = NX | 1;
-  static constexpr int spread(int n, int lpw) { return (n % lpw == 0) ? n / lpw : 0; }
-  static constexpr int DC = spread(NX, AY::LPW);   // column lines (x) of the plane passes
-  static constexpr int DR = spread(NY, AX::LPW);   // row lines (y)
-  static constexpr size_t smem_pfwd =
-      sizeof(cf) * (2 * (size_t)PL + (size_t)PW * NY + ev(NX) + ev(NY)) + sizeof(uint64_t);
-  static constexpr size_t smem_zmask =
-      sizeof(cf) * (2 * (size_t)S + 2 * ev(NZ)) + 8 * NZ * sizeof(uint32_t) + 2 * sizeof(uint64_t);
-  static constexpr size_t smem_padj =
-      sizeof(cf) * ((size_t)PL + (size_t)PW * NY + ev(NX) + ev(NY)) + sizeof(uint64_t);
 };
-
-// line l of a warp's group → row / column index (identity when D == 0)
-template <int LPW, int D>
-__device__ __forceinline__ int line_at(int l) {
-  if constexpr (D > 0) return (l / LPW) + D * (l % LPW);
-  return l;
-}
 
 // xs[z][x] · S'_c[z][x], both in shared memory (line = x, element = z)
 template <int NX>
@@ -402,20 +372,6 @@ __global__ void __launch_bounds__(Sh::ZW2 * 32, 2)
   cluster.sync();
 }
 
-// ===========================================================================
-// Four-pass form of the normal operator (the default).  Per chunk of frames
-// and group of coils, with T[f][cc][z][y][x] the chunk's per-coil k-space:
-//   k_pfwd   unit (cc, z, f): S'_c ⊙ x̄ on plane z → DFT_y → DFT_x → T
-//            (x̄ = Σ_k X_k, summed once per operator by k_xsum)
-//   k_zmask  unit (cc, f, y): the z slab of T → DFT_z → mask → bDFT_z → T,
-//            in place, slabs in and out by bulk copies
-//   k_padj   unit (cc, z, f): plane of T → bDFT_y → bDFT_x → × conj(S'_c) → T
-//   k_csum   g (=, −A'y, or +=) scale · Σ_cc T[f][cc], coils summed in order
-// The plane passes take their planes by TMA (the next unit's while the current
-// one runs its row passes); every unit is one plane or slab, so the launches
-// fill all SMs evenly and no CTA waits on another.
-// ===========================================================================
-
 // x̄[i] = Σ_k X[k][i] over ns scales (in order), n elements, pairs per thread
 __global__ void k_xsum(const cf* __restrict__ X, int ns, int64_t sstride, cf* __restrict__ out,
                        int64_t n) {
@@ -443,383 +399,6 @@ __global__ void k_xsum(const cf* __restrict__ X, int ns, int64_t sstride, cf* __
     cf v = X[i];
     for (int k = 1; k < ns; ++k) v = cadd(v, X[i + k * sstride]);
     out[i] = v;
-  }
-}
-
-// a[i] · b[i], both in shared memory (line l, element e at line_at(l)·SL + e·SE)
-template <int SL, int SE, int LPW = 1, int D = 0>
-struct LdMul {
-  const cf* a;
-  const cf* b;
-  __device__ __forceinline__ cf operator()(int l, int e) const {
-    const int i = line_at<LPW, D>(l) * SL + e * SE;
-    return cmul(a[i], b[i]);
-  }
-};
-// element e of line l at b[line_at(l)·SL + e·SE]
-template <int SL, int SE, int LPW, int D>
-struct SmM {
-  cf* b;
-  __device__ __forceinline__ cf operator()(int l, int e) const { return b[line_at<LPW, D>(l) * SL + e * SE]; }
-  __device__ __forceinline__ void operator()(int l, int e, cf v) const { b[line_at<LPW, D>(l) * SL + e * SE] = v; }
-};
-// dst[i] = conj(s[i]) · v, row layout (line = row line_at(l), element = x); s in global memory
-template <int NX, int LPW = 1, int D = 0>
-struct StMulC {
-  cf* dst;
-  const cf* s;
-  __device__ __forceinline__ void operator()(int l, int e, cf v) const {
-    const int i = line_at<LPW, D>(l) * NX + e;
-    dst[i] = cmulc(__ldg(s + i), v);
-  }
-};
-// k-space mask of one z slab (line = kx, element = kz): row kz's bits start at
-// bit (kz·PL + y·NX) & 31 of the four words w[4·kz ..]
-template <int NX, int PL>
-struct MaskZ {
-  const uint32_t* w;
-  int ybit;   // y·NX
-  __device__ __forceinline__ cf operator()(int l, int e, cf v) const {
-    const int b = ((e * PL + ybit) & 31) + l;
-    return ((w[4 * e + (b >> 5)] >> (b & 31)) & 1u) ? v : make_float2(0.f, 0.f);
-  }
-};
-
-// Pass groups of the plane kernels, out of line (each keeps its own index
-// arithmetic, within the 128-register budget of 16 warps).  The second pass
-// of each axis reads its twiddles from a table (build_tab); W has row stride
-// Sh::PW and the lines of a group are spread (Sh::DC, Sh::DR).
-template <class Sh>
-__device__ __noinline__ void pf_cols(const cf* xs, const cf* sc, cf* W, const cf* tby, int l0) {
-  using AY = typename Sh::AY;
-  using Cols = SmM<1, Sh::PW, AY::LPW, Sh::DC>;
-  spec::wpass<Sh::NY, AY::R0, 1, false, AY::LPW, false>(
-      l0, Sh::NX, tby, LdMul<1, Sh::NX, AY::LPW, Sh::DC>{xs, sc}, Cols{W});
-  spec::wpass<Sh::NY, AY::R1, AY::R0, false, AY::LPW, true, true>(l0, Sh::NX, tby, Cols{W}, Cols{W});
-}
-template <class Sh>
-__device__ __noinline__ void pf_rows(cf* W, const cf* tbx, int l0, cf* dst) {
-  using AX = typename Sh::AX;
-  using Rows = SmM<Sh::PW, 1, AX::LPW, Sh::DR>;
-  using Out = SmM<Sh::NX, 1, AX::LPW, Sh::DR>;
-  spec::wpass<Sh::NX, AX::R0, 1, false, AX::LPW, true>(l0, Sh::NY, tbx, Rows{W}, Rows{W});
-  spec::wpass<Sh::NX, AX::R1, AX::R0, false, AX::LPW, false, true>(l0, Sh::NY, tbx, Rows{W}, Out{dst});
-}
-template <class Sh>
-__device__ __noinline__ void pa_cols(const cf* P, cf* W, const cf* tby, int l0) {
-  using AY = typename Sh::AY;
-  using In = SmM<1, Sh::NX, AY::LPW, Sh::DC>;
-  using Cols = SmM<1, Sh::PW, AY::LPW, Sh::DC>;
-  spec::wpass<Sh::NY, AY::R1, 1, true, AY::LPW, false>(l0, Sh::NX, tby, In{const_cast<cf*>(P)}, Cols{W});
-  spec::wpass<Sh::NY, AY::R0, AY::R1, true, AY::LPW, true, true>(l0, Sh::NX, tby, Cols{W}, Cols{W});
-}
-template <class Sh>
-__device__ __noinline__ void pa_rows(cf* W, const cf* tbx, int l0, cf* dst, const cf* sc) {
-  using AX = typename Sh::AX;
-  using Rows = SmM<Sh::PW, 1, AX::LPW, Sh::DR>;
-  spec::wpass<Sh::NX, AX::R1, 1, true, AX::LPW, true>(l0, Sh::NY, tbx, Rows{W}, Rows{W});
-  spec::wpass<Sh::NX, AX::R0, AX::R1, true, AX::LPW, false, true>(
-      l0, Sh::NY, tbx, Rows{W}, StMulC<Sh::NX, AX::LPW, Sh::DR>{dst, sc});
-}
-
-// Forward plane pass of one coil group, persistent over units u = (cc
-// fastest, then z, then frame f of the chunk): the summed image plane and the
-// coil-map plane arrive by TMA; DFT_y over the columns of their product, then
-// DFT_x over the rows, written to T[f][cc][z].
-template <class Sh>
-__global__ void __launch_bounds__(Sh::XYW * 32, 1)
-    k_pfwd(const cf* __restrict__ xsum, int t0, int nf, int cc0, int ch, const cf* __restrict__ smod,
-           cf* __restrict__ T, const cf* __restrict__ twx_g, const cf* __restrict__ twy_g,
-           int* __restrict__ err) {
-  using AX = typename Sh::AX;
-  using AY = typename Sh::AY;
-  constexpr int NX = Sh::NX, NY = Sh::NY, NZ = Sh::NZ, PL = Sh::PL;
-  constexpr int64_t NVOX = Sh::NVOX;
-  extern __shared__ __align__(128) unsigned char smraw[];
-  cf* XS = reinterpret_cast<cf*>(smraw);
-  cf* SB = XS + PL;
-  cf* W = SB + PL;                  // row stride Sh::PW
-  cf* tbx = W + Sh::PW * NY;        // twiddle tables of the second x and y passes
-  cf* tby = tbx + Sh::ev(NX);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(tby + Sh::ev(NY));
-  const int tid = threadIdx.x, warp = tid >> 5, nw = blockDim.x >> 5;
-  const int units = ch * NZ * nf;
-  auto issue = [&](int u) {
-    const int cc = u % ch, r = u / ch, z = r % NZ, f = r / NZ;
-    spec::mbar_expect_tx(bar, 2u * PL * (unsigned)sizeof(cf));
-    spec::bulk_g2s(XS, xsum + (int64_t)(t0 + f) * NVOX + (int64_t)z * PL, PL * (unsigned)sizeof(cf), bar);
-    spec::bulk_g2s(SB, smod + (int64_t)(cc0 + cc) * NVOX + (int64_t)z * PL, PL * (unsigned)sizeof(cf), bar);
-  };
-  if (tid == 0) {
-    spec::mbar_init(bar, 1);
-    spec::mbar_fence_init();
-  }
-  spec::build_tab<NX, AX::R1>(tbx, twx_g);
-  spec::build_tab<NY, AY::R1>(tby, twy_g);
-  __syncthreads();
-  int u = blockIdx.x;
-  if (tid == 0 && u < units) issue(u);
-  unsigned par = 0;
-  bool bad = false;
-  for (; u < units; u += gridDim.x) {
-    if (!bad && !spec::mbar_wait(bar, par)) bad = true;
-    par ^= 1u;
-    if (!bad) {
-#pragma unroll 1
-      for (int g = warp; g * AY::LPW < NX; g += nw) pf_cols<Sh>(XS, SB, W, tby, g * AY::LPW);
-    }
-    __syncthreads();   // columns done: XS, SB free
-    const int nxt = u + (int)gridDim.x;
-    if (tid == 0 && nxt < units) {
-      spec::fence_proxy_async();
-      issue(nxt);
-    }
-    if (!bad) {
-      const int cc = u % ch, r = u / ch, z = r % NZ, f = r / NZ;
-      cf* dst = T + ((int64_t)f * ch + cc) * NVOX + (int64_t)z * PL;
-#pragma unroll 1
-      for (int g = warp; g * AX::LPW < NY; g += nw) pf_rows<Sh>(W, tbx, g * AX::LPW, dst);
-    }
-    __syncthreads();   // rows done: W free
-  }
-  if (__syncthreads_or(bad) && tid == 0) atomicOr(err, kErrWait);
-}
-
-// z pass with the k-space mask, in place on T, persistent over slabs u = (cc
-// fastest, then frame, then y): each slab (NZ rows of NX) comes in by bulk
-// copies into one of two buffers, runs DFT_z, the mask and bDFT_z (the last
-// forward and first inverse radix passes fused around the mask), and goes back
-// by bulk copies; the other buffer's slab is in flight meanwhile.  The mask
-// words of the next slab are staged (double-buffered) while the current one
-// finishes, so a unit needs one block barrier.  MINB: CTAs per SM the
-// register budget is set for.
-template <class Sh, int MINB, int NW = Sh::ZW2>
-__global__ void __launch_bounds__(NW * 32, MINB)
-    k_zmask(cf* __restrict__ T, const uint32_t* __restrict__ mask, int nwords, int t0, int nf, int ch,
-            const cf* __restrict__ twz_g, int* __restrict__ err) {
-  using AZ = typename Sh::AZ;
-  constexpr int NX = Sh::NX, NY = Sh::NY, NZ = Sh::NZ, S = Sh::S, PL = Sh::PL;
-  constexpr int64_t NVOX = Sh::NVOX;
-  constexpr int kGroups = Sh::cdiv(NX, AZ::LPW);   // line groups of a slab
-  constexpr bool kCopyWarp = NW > 1 && kGroups % (NW - 1) == 0;
-  extern __shared__ __align__(128) unsigned char smraw[];
-  cf* SL = reinterpret_cast<cf*>(smraw);          // two slab buffers
-  cf* tf = SL + 2 * S;                            // twiddle tables: forward (the fused pass)
-  cf* ti = tf + Sh::ev(NZ);                       // and inverse (the last pass)
-  uint32_t* MB = reinterpret_cast<uint32_t*>(ti + Sh::ev(NZ));   // 2 × 4 words per kz
-  uint64_t* bar = reinterpret_cast<uint64_t*>(MB + 8 * NZ);
-  const int tid = threadIdx.x, warp = tid >> 5, nw = blockDim.x >> 5, lane = tid & 31;
-  const int units = ch * nf * NY;
-  auto slab = [&](int u) {
-    const int cc = u % ch, r = u / ch, f = r % nf, y = r / nf;
-    return T + ((int64_t)f * ch + cc) * NVOX + (int64_t)y * NX;
-  };
-  if (tid == 0) {
-    spec::mbar_init(&bar[0], 1);
-    spec::mbar_init(&bar[1], 1);
-    spec::mbar_fence_init();
-  }
-  // mask words of slab u into mb: row kz spans bits [kz·PL + y·NX, + NX) of frame t0 + f
-  auto stage_mask = [&](int u, uint32_t* mb) {
-    const int r = u / ch, f = r % nf, y = r / nf;
-    const uint32_t* mrow = mask + (int64_t)(t0 + f) * nwords;
-    for (int i = tid; i < 4 * NZ; i += blockDim.x) {
-      const int kz = i >> 2;
-      const int w = (int)(((int64_t)kz * PL + (int64_t)y * NX) >> 5) + (i & 3);
-      mb[i] = (w < nwords) ? __ldg(mrow + w) : 0u;
-    }
-  };
-  spec::build_tab<NZ, AZ::R1>(tf, twz_g);
-  spec::build_tab<NZ, AZ::R0>(ti, twz_g);
-  if ((int)blockIdx.x < units) stage_mask(blockIdx.x, MB);
-  __syncthreads();
-  if (warp == 0) {
-    for (int q = 0; q < 2; ++q) {
-      const int u = blockIdx.x + q * (int)gridDim.x;
-      if (u < units) rows_g2s(SL + q * S, slab(u), NZ, NX, PL, &bar[q]);
-    }
-  }
-  bool bad = false;
-  int k = 0;
-  for (int u = blockIdx.x; u < units; u += gridDim.x, ++k) {
-    const int b = k & 1;
-    const int y = (u / ch) / nf;
-    if (!bad && !spec::mbar_wait(&bar[b], (unsigned)((k >> 1) & 1))) bad = true;
-    cf* P = SL + b * S;
-    if (!bad) {
-      const cf* tfc = opaque(tf);
-      const cf* tic = opaque(ti);
-      using Cols = SmC<1, NX>;   // line = x, element = z
-      const MaskZ<NX, PL> msk{MB + b * 4 * NZ, y * NX};
-      // when the line groups divide evenly over the other warps, warp 0 only
-      // moves slabs (its bulk stores and loads then overlap the others' passes)
-      const int cw = kCopyWarp ? 1 : 0;
-#pragma unroll 1
-      for (int g = warp - cw; g >= 0 && g * AZ::LPW < NX; g += nw - cw) {
-        spec::wpass<NZ, AZ::R0, 1, false, AZ::LPW, true>(g * AZ::LPW, NX, tfc, Cols{P}, Cols{P});
-        spec::wsandwich<NZ, AZ::R1, AZ::LPW, true, true>(g * AZ::LPW, NX, tfc, Cols{P}, Cols{P}, msk);
-        spec::wpass<NZ, AZ::R0, AZ::R1, true, AZ::LPW, true, true>(g * AZ::LPW, NX, tic, Cols{P}, Cols{P});
-      }
-    }
-    if (u + (int)gridDim.x < units) stage_mask(u + (int)gridDim.x, MB + (b ^ 1) * 4 * NZ);
-    spec::fence_proxy_async();   // this thread's slab writes, before the bulk copies read them
-    __syncthreads();   // slab done; the next slab's mask words visible
-    if (warp == 0) {
-      if (!bad) {
-        spec::fence_proxy_async();
-        cf* dst = slab(u);
-        for (int z = lane; z < NZ; z += 32)
-          spec::bulk_s2g(dst + (int64_t)z * PL, P + z * NX, NX * (unsigned)sizeof(cf));
-        spec::bulk_commit();
-      }
-      const int u2 = u + 2 * (int)gridDim.x;
-      if (u2 < units) {
-        spec::bulk_wait_read();   // this buffer's rows have left shared memory
-        __syncwarp();
-        rows_g2s(P, slab(u2), NZ, NX, PL, &bar[b]);
-      }
-    }
-  }
-  if (warp == 0) spec::bulk_wait_all();
-  if (__syncthreads_or(bad) && tid == 0) atomicOr(err, kErrWait);
-}
-
-// Inverse plane pass, persistent over units u = (cc fastest, then z, then f):
-// plane z of T[f][cc] by TMA, bDFT_y over the columns, bDFT_x over the rows,
-// × conj(S'_c), written back in place.
-template <class Sh>
-__global__ void __launch_bounds__(Sh::XYW * 32, 1)
-    k_padj(cf* __restrict__ T, int nf, int cc0, int ch, const cf* __restrict__ smod,
-           const cf* __restrict__ twx_g, const cf* __restrict__ twy_g, int* __restrict__ err) {
-  using AX = typename Sh::AX;
-  using AY = typename Sh::AY;
-  constexpr int NX = Sh::NX, NY = Sh::NY, NZ = Sh::NZ, PL = Sh::PL;
-  constexpr int64_t NVOX = Sh::NVOX;
-  extern __shared__ __align__(128) unsigned char smraw[];
-  cf* P = reinterpret_cast<cf*>(smraw);
-  cf* W = P + PL;                   // row stride Sh::PW
-  cf* tbx = W + Sh::PW * NY;        // twiddle tables of the second x and y inverse passes
-  cf* tby = tbx + Sh::ev(NX);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(tby + Sh::ev(NY));
-  const int tid = threadIdx.x, warp = tid >> 5, nw = blockDim.x >> 5;
-  const int units = ch * NZ * nf;
-  auto plane = [&](int u) {
-    const int cc = u % ch, r = u / ch, z = r % NZ, f = r / NZ;
-    return T + ((int64_t)f * ch + cc) * NVOX + (int64_t)z * PL;
-  };
-  if (tid == 0) {
-    spec::mbar_init(bar, 1);
-    spec::mbar_fence_init();
-  }
-  spec::build_tab<NX, AX::R0>(tbx, twx_g);
-  spec::build_tab<NY, AY::R0>(tby, twy_g);
-  __syncthreads();
-  int u = blockIdx.x;
-  if (tid == 0 && u < units) {
-    spec::mbar_expect_tx(bar, PL * (unsigned)sizeof(cf));
-    spec::bulk_g2s(P, plane(u), PL * (unsigned)sizeof(cf), bar);
-  }
-  unsigned par = 0;
-  bool bad = false;
-  for (; u < units; u += gridDim.x) {
-    if (!bad && !spec::mbar_wait(bar, par)) bad = true;
-    par ^= 1u;
-    if (!bad) {
-#pragma unroll 1
-      for (int g = warp; g * AY::LPW < NX; g += nw) pa_cols<Sh>(P, W, tby, g * AY::LPW);
-    }
-    __syncthreads();   // columns done: P free
-    const int nxt = u + (int)gridDim.x;
-    if (tid == 0 && nxt < units) {
-      spec::fence_proxy_async();
-      spec::mbar_expect_tx(bar, PL * (unsigned)sizeof(cf));
-      spec::bulk_g2s(P, plane(nxt), PL * (unsigned)sizeof(cf), bar);
-    }
-    if (!bad) {
-      const int cc = u % ch, z = (u / ch) % NZ;
-      const cf* sc = smod + (int64_t)(cc0 + cc) * NVOX + (int64_t)z * PL;
-      cf* dst = plane(u);
-#pragma unroll 1
-      for (int g = warp; g * AX::LPW < NY; g += nw) pa_rows<Sh>(W, tbx, g * AX::LPW, dst, sc);
-    }
-    __syncthreads();   // rows done: W free
-  }
-  if (__syncthreads_or(bad) && tid == 0) atomicOr(err, kErrWait);
-}
-
-// Coil combine of a chunk: out[t0 + f] (mode 0: scale·Σ − A'y when subtract,
-// else scale·Σ; mode 1: out += scale·Σ) with Σ over the ch coils of T[f] in
-// coil order.  Pairs of values per thread when every pointer is 16-byte aligned.
-__global__ void k_csum(const cf* __restrict__ T, int nf, int ch, int64_t nvox, cf* __restrict__ out,
-                       const cf* __restrict__ ahy, int t0, float scale, int mode, int subtract) {
-  const int64_t step = (int64_t)gridDim.x * blockDim.x;
-  const bool vec = ((reinterpret_cast<uintptr_t>(T) | reinterpret_cast<uintptr_t>(out) |
-                     reinterpret_cast<uintptr_t>(ahy)) & 15) == 0 && (nvox % 2) == 0;
-  if (vec) {
-    const int64_t h = nvox / 2, n2 = (int64_t)nf * h;
-    const float4* t4 = reinterpret_cast<const float4*>(T);
-    float4* o4 = reinterpret_cast<float4*>(out) + (int64_t)t0 * h;
-    const float4* a4 = reinterpret_cast<const float4*>(ahy) + (int64_t)t0 * h;
-    if (ch == 6) {   // the compiled coil group: the six coil loads and g / A'y issued together
-      for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < h; o += step) {
-#pragma unroll 2
-        for (int f = 0; f < nf; ++f) {
-          const float4* src = t4 + (int64_t)f * 6 * h + o;
-          const int64_t i = (int64_t)f * h + o;
-          float4 w[6];
-#pragma unroll
-          for (int c = 0; c < 6; ++c) w[c] = src[c * h];
-          const float4 g = mode ? o4[i] : subtract ? a4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-          float4 sm = w[0];
-#pragma unroll
-          for (int c = 1; c < 6; ++c) {
-            sm.x += w[c].x;
-            sm.y += w[c].y;
-            sm.z += w[c].z;
-            sm.w += w[c].w;
-          }
-          float4 v = make_float4(sm.x * scale, sm.y * scale, sm.z * scale, sm.w * scale);
-          if (mode) v = make_float4(g.x + v.x, g.y + v.y, g.z + v.z, g.w + v.w);
-          else if (subtract) v = make_float4(v.x - g.x, v.y - g.y, v.z - g.z, v.w - g.w);
-          o4[i] = v;
-        }
-      }
-      return;
-    }
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n2; i += step) {
-      const int64_t f = i / h, o = i - f * h;
-      const float4* src = t4 + f * ch * h + o;
-      float4 s = src[0];
-      for (int c = 1; c < ch; ++c) {
-        const float4 w = src[c * h];
-        s.x += w.x;
-        s.y += w.y;
-        s.z += w.z;
-        s.w += w.w;
-      }
-      float4 v = make_float4(s.x * scale, s.y * scale, s.z * scale, s.w * scale);
-      if (mode) {
-        const float4 g = o4[i];
-        v = make_float4(g.x + v.x, g.y + v.y, g.z + v.z, g.w + v.w);
-      } else if (subtract) {
-        const float4 a = a4[i];
-        v = make_float4(v.x - a.x, v.y - a.y, v.z - a.z, v.w - a.w);
-      }
-      o4[i] = v;
-    }
-    return;
-  }
-  const int64_t n = (int64_t)nf * nvox;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += step) {
-    const int64_t f = i / nvox, o = i - f * nvox;
-    const cf* src = T + f * ch * nvox + o;
-    cf s = src[0];
-    for (int c = 1; c < ch; ++c) s = cadd(s, src[c * nvox]);
-    const int64_t oi = (int64_t)t0 * nvox + i;
-    cf v = cscale(s, scale);
-    if (mode) v = cadd(out[oi], v);
-    else if (subtract) v = csub(v, ahy[oi]);
-    out[oi] = v;
   }
 }
 
@@ -1103,14 +682,6 @@ struct SpecOps {
   const void* zadj;
   int zfwd_threads, xy_threads, zadj_threads;
   size_t smem_zfwd, smem_zadj, smem_xy;
-  // four-pass form
-  const void* pfwd;
-  const void* zmask;     // two CTAs per SM (64 registers)
-  const void* zmask1;    // one CTA per SM (more registers, MSLR_ZMASK_CTAS=1)
-  const void* zmaskm;    // two CTAs per SM with Sh::ZWm warps (more registers per thread)
-  int zmaskm_threads;
-  const void* padj;
-  size_t smem_pfwd, smem_zmask, smem_padj;
   const void* xy_tc;                       // tensor-core plane pass (square planes), or null
   size_t smem_xy_tc;
   std::vector<uint32_t> (*dft)();          // its DFT tiles
@@ -1130,15 +701,6 @@ SpecOps ops_of() {
             Sh::smem_zfwd,
             Sh::smem_zadj,
             Sh::smem_xy,
-            reinterpret_cast<const void*>(&k_pfwd<Sh>),
-            reinterpret_cast<const void*>(&k_zmask<Sh, 2>),
-            reinterpret_cast<const void*>(&k_zmask<Sh, 1>),
-            reinterpret_cast<const void*>(&k_zmask<Sh, 2, Sh::ZWm>),
-            Sh::ZWm * 32,
-            reinterpret_cast<const void*>(&k_padj<Sh>),
-            Sh::smem_pfwd,
-            Sh::smem_zmask,
-            Sh::smem_padj,
             nullptr,
             0,
             nullptr};
@@ -1200,49 +762,10 @@ bool sense_spec_setup(Ctx* c) {
     c->spec_fr = fr;
   }
   c->spec_zfwd_ctas = per_sm_z * c->nsm;
-  // four-pass form (default; MSLR_SENSE_PATH=3 keeps the three-kernel form)
-  {
-    const char* sp = std::getenv("MSLR_SENSE_PATH");
-    c->spec_four = !(sp && std::string(sp) == "3");
-  }
-  if (c->spec_four) {
-    const char* zc = std::getenv("MSLR_ZMASK_CTAS");
-    c->spec_zmask_var = (zc && std::string(zc) == "1") ? 1 : 0;
-    int a = 0, b = 0, b1 = 0, bm = 0, d = 0;
-    if (cudaFuncSetAttribute(o->pfwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)o->smem_pfwd) ||
-        cudaFuncSetAttribute(o->zmask, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)o->smem_zmask) ||
-        cudaFuncSetAttribute(o->zmask1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)o->smem_zmask) ||
-        cudaFuncSetAttribute(o->zmaskm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)o->smem_zmask) ||
-        cudaFuncSetAttribute(o->padj, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)o->smem_padj) ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, o->pfwd, o->xy_threads, o->smem_pfwd) ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, o->zmask, o->zadj_threads, o->smem_zmask) ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, o->zmask1, o->zadj_threads, o->smem_zmask) ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bm, o->zmaskm, o->zmaskm_threads, o->smem_zmask) ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, o->padj, o->xy_threads, o->smem_padj) ||
-        a < 1 || b < 1 || b1 < 1 || bm < 1 || d < 1 ||
-        dalloc(c, (void**)&c->d_xsum, (size_t)c->Nt * c->nvox * sizeof(cf))) {
-      cudaGetLastError();
-      c->spec_four = false;
-    } else {
-      c->spec_pfwd_ctas = a * c->nsm;
-      c->spec_zmask_ctas_v[0] = b * c->nsm;
-      c->spec_zmask_ctas_v[1] = b1 * c->nsm;
-      c->spec_zmask_ctas_v[2] = bm * c->nsm;
-      c->spec_zmask_warps[0] = c->spec_zmask_warps[1] = o->zadj_threads / 32;
-      c->spec_zmask_warps[2] = o->zmaskm_threads / 32;
-      c->spec_zmask_ctas = c->spec_zmask_ctas_v[c->spec_zmask_var];
-      c->spec_padj_ctas = d * c->nsm;
-      // two lanes by default (measured 8.65 → 7.77 ms for a 40-frame operator
-      // at 90×90×60 × 18 coils); MSLR_SENSE_LANES=1 keeps one
-      const char* ln = std::getenv("MSLR_SENSE_LANES");
-      if (!(ln && std::string(ln) == "1") &&
-          !cudaStreamCreateWithFlags(&c->sn_stream, cudaStreamNonBlocking) &&
-          !cudaEventCreateWithFlags(&c->sn_fork, cudaEventDisableTiming) &&
-          !cudaEventCreateWithFlags(&c->sn_join, cudaEventDisableTiming))
-        c->spec_lanes = 2;
-      cudaGetLastError();
-    }
-  }
+  // MSLR_SENSE_PATH=3 selects this file's three-kernel form for the normal
+  // operator (else the register-line form of sense_line.cu runs)
+  const char* sp = std::getenv("MSLR_SENSE_PATH");
+  c->spec_three = sp && std::string(sp) == "3";
   // tensor-core plane pass only on request (MSLR_XY_PATH=tc): at 90×90 its
   // padded split-BF16 DFT products (12 MMAs of 128×96×16 per K step, four
   // products per plane, serialised with their epilogues) take longer than the
@@ -1261,8 +784,15 @@ bool sense_spec_setup(Ctx* c) {
   return true;
 }
 
+int image_sum(Ctx* c, const cf* X, int ns, int64_t sstride, cf* out, cudaStream_t st) {
+  k_xsum<<<4 * c->nsm, 512, 0, st>>>(X, ns, sstride, out, (int64_t)c->Nt * c->nvox);
+  MSLR_CUDA_TRY(cudaGetLastError());
+  c->launches += 1;
+  return MSLR_OK;
+}
+
 // Records a profiling event on st when the context is profiling.
-static int prof_mark(Ctx* c, cudaStream_t st) {
+int prof_mark(Ctx* c, cudaStream_t st) {
   if (!c->prof_on) return MSLR_OK;
   if (c->prof_n == (int)c->prof_ev.size()) {
     cudaEvent_t e;
@@ -1273,100 +803,11 @@ static int prof_mark(Ctx* c, cudaStream_t st) {
   return MSLR_OK;
 }
 
-// Four-pass normal operator (see k_pfwd ... k_csum): Σ_k X_k once, then per
-// coil group and chunk of frames the four kernels; consecutive chunks
-// alternate between two streams ("lanes", each with its own k-space buffer),
-// so that one chunk's memory-bound coil combine and its kernels' last waves
-// overlap the next chunk's kernels.
-static int normal_op_four(Ctx* c, const SpecOps* o, const cf* X, int ns, int64_t sstride, cf* g,
-                          bool subtract, cudaStream_t st) {
-  const float scale = (float)(1.0 / (double)c->nvox);
-  const int Nc = c->Nc;
-  const int Ch = std::max(1, std::min(Nc, c->spec_ch));             // coils per group
-  int F = std::max(1, c->spec_fr);                                  // frames per chunk
-  while (F > 1 && (int64_t)F * Ch > (int64_t)c->F * Nc) --F;        // within the k-space buffer
-  const int64_t nvox = c->nvox;
-  // the summed image: X itself for one 16-byte aligned image, else Σ_k X_k
-  const cf* xs = X;
-  if (ns > 1 || (reinterpret_cast<uintptr_t>(X) & 15)) {
-    k_xsum<<<4 * c->nsm, 512, 0, st>>>(X, ns, sstride, c->d_xsum, (int64_t)c->Nt * nvox);
-    MSLR_CUDA_TRY(cudaGetLastError());
-    c->launches += 1;
-    xs = c->d_xsum;
-  }
-  int nwords = c->nwords;
-  const cf* smod = c->d_smaps_mod;
-  const uint32_t* mask = c->d_mask;
-  const cf* ahy = c->d_ahy;
-  cf* T = c->d_T;
-  int* err = c->d_err;
-  const int sub = subtract ? 1 : 0;
-  const int zv = c->spec_zmask_var;
-  const void* zk = zv == 1 ? o->zmask1 : zv == 2 ? o->zmaskm : o->zmask;
-  const int zthreads = zv == 2 ? o->zmaskm_threads : o->zadj_threads;
-  c->prof_kernels = 4;
-  // two lanes: chunk j of every group on lane j % 2 (so the += of later
-  // groups stays ordered after the first group's chunk of the same frames),
-  // each lane with its own k-space buffer
-  const int64_t chunk_imgs = (int64_t)F * Ch;
-  const bool lanes = c->spec_lanes == 2 && !c->prof_on && 2 * chunk_imgs <= (int64_t)c->F * Nc &&
-                     c->Nt > F;
-  cudaStream_t side = c->sn_stream;
-  if (lanes) {
-    MSLR_CUDA_TRY(cudaEventRecord(c->sn_fork, st));
-    MSLR_CUDA_TRY(cudaStreamWaitEvent(side, c->sn_fork, 0));
-  }
-  cudaStream_t st0 = st;
-  for (int cc0 = 0; cc0 < Nc; cc0 += Ch) {
-    int ch = std::min(Ch, Nc - cc0);
-    const int mode = cc0 > 0 ? 1 : 0;
-    for (int t0 = 0, j = 0; t0 < c->Nt; t0 += F, ++j) {
-      int f = std::min(F, c->Nt - t0);
-      const int lane = lanes ? (j & 1) : 0;
-      st = lane ? side : st0;
-      T = c->d_T + lane * chunk_imgs * nvox;
-      const int planes = ch * c->N[2] * f;
-      if (int rc = prof_mark(c, st)) return rc;
-      {
-        const int grid = std::max(1, std::min(planes, c->spec_pfwd_ctas));
-        void* args[] = {(void*)&xs, (void*)&t0, (void*)&f, (void*)&cc0, (void*)&ch, (void*)&smod,
-                        (void*)&T,  (void*)&c->d_tw[0], (void*)&c->d_tw[1], (void*)&err};
-        MSLR_CUDA_TRY(cudaLaunchKernel(o->pfwd, dim3(grid), dim3(o->xy_threads), args, o->smem_pfwd, st));
-      }
-      if (int rc = prof_mark(c, st)) return rc;
-      {
-        const int slabs = ch * f * c->N[1];
-        const int grid = std::max(1, std::min(slabs, c->spec_zmask_ctas));
-        void* args[] = {(void*)&T, (void*)&mask, (void*)&nwords, (void*)&t0, (void*)&f, (void*)&ch,
-                        (void*)&c->d_tw[2], (void*)&err};
-        MSLR_CUDA_TRY(cudaLaunchKernel(zk, dim3(grid), dim3(zthreads), args, o->smem_zmask, st));
-      }
-      if (int rc = prof_mark(c, st)) return rc;
-      {
-        const int grid = std::max(1, std::min(planes, c->spec_padj_ctas));
-        void* args[] = {(void*)&T,  (void*)&f, (void*)&cc0, (void*)&ch, (void*)&smod,
-                        (void*)&c->d_tw[0], (void*)&c->d_tw[1], (void*)&err};
-        MSLR_CUDA_TRY(cudaLaunchKernel(o->padj, dim3(grid), dim3(o->xy_threads), args, o->smem_padj, st));
-      }
-      if (int rc = prof_mark(c, st)) return rc;
-      k_csum<<<4 * c->nsm, 512, 0, st>>>(T, f, ch, nvox, g, ahy, t0, scale, mode, sub);
-      MSLR_CUDA_TRY(cudaGetLastError());
-      if (int rc = prof_mark(c, st)) return rc;
-      c->launches += 4;
-    }
-  }
-  if (lanes) {   // join the side lane back into the caller's stream
-    MSLR_CUDA_TRY(cudaEventRecord(c->sn_join, side));
-    MSLR_CUDA_TRY(cudaStreamWaitEvent(st0, c->sn_join, 0));
-  }
-  return MSLR_OK;
-}
-
 int normal_op_spec(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool subtract,
                    cudaStream_t st) {
   const SpecOps* o = find_ops(c->N[0], c->N[1], c->N[2]);
   if (!o) return fail(MSLR_ERR_UNSUPPORTED, "no specialised SENSE kernels for this shape");
-  if (c->spec_four && !c->xy_tc) return normal_op_four(c, o, X, ns, sstride, g, subtract, st);
+  if (c->line && !c->spec_three && !c->xy_tc) return normal_op_line(c, X, ns, sstride, g, subtract, st);
   c->prof_kernels = 3;
   float scale = (float)(1.0 / (double)c->nvox);
   const int Nc = c->Nc, Ny = c->N[1], Nz = c->N[2];
@@ -1439,76 +880,46 @@ int normal_op_spec(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool sub
   return MSLR_OK;
 }
 
-// Autotuner: coils per group × frames per chunk of the specialised normal
-// operator, timed on the bound context (A'A applied to A'y).  Larger chunks
-// mean fewer launches; the chunk's k-space (Ch·F images) and the group's coil
-// maps should stay in L2.  Clusters of the adjoint z kernel hold Ch CTAs, so
-// Ch ≤ 8.
+// Autotuner: coils per group × frames per chunk of the normal operator, and
+// (register-line form) one or two lanes of chunks, timed on the bound context
+// (A'A applied to A'y).  Larger chunks mean fewer launches; the chunk's
+// k-space should stay in L2.  The three-kernel form's clusters hold one coil
+// per CTA, so groups have at most eight coils.
 int tune_sense_chunks(Ctx* c, cudaStream_t st) {
-  if (!c->spec) return MSLR_OK;
-  // the three-kernel form's clusters hold one coil per CTA (at most 8); the
-  // four-pass form takes any group size
-  const bool four = c->spec_four && !c->xy_tc;
-  std::vector<int> chs = {2, 3, 4, 6, 8};
-  if (four) chs.insert(chs.end(), {9, 12, 18});
+  const bool three = c->spec && (c->spec_three || c->xy_tc);
+  if (!three && !c->line) return MSLR_OK;
   const int64_t E = (int64_t)c->Nt * c->nvox;
+  const int max_lanes = !three && c->sn_stream ? 2 : 1;
   float best = 1e30f;
-  int bch = c->spec_ch, bfr = c->spec_fr;
-  for (int ch : chs) {
+  int bch = c->spec_ch, bfr = c->spec_fr, bl = c->spec_lanes;
+  for (int ch : {2, 3, 4, 6, 8}) {
     if (ch > c->Nc) continue;
     for (int fr = 1; fr <= 4; ++fr) {
       if ((int64_t)fr * ch > (int64_t)c->F * c->Nc || fr > c->Nt || fr * ch > 24) continue;
       c->spec_ch = ch;
       c->spec_fr = fr;
-      float ms = 0.f;
-      int rc = time_ms(st, 2, &ms, [&] { return normal_op_spec(c, c->d_ahy, 1, E, c->d_G, false, st); });
-      if (rc) return rc;
-      if (ms < best) {
-        best = ms;
-        bch = ch;
-        bfr = fr;
+      for (int lanes = 1; lanes <= max_lanes; ++lanes) {
+        if (!three) c->spec_lanes = lanes;
+        float ms = 0.f;
+        int rc = time_ms(st, 2, &ms, [&] { return normal_op(c, c->d_ahy, 1, E, c->d_G, false, st); });
+        if (rc) return rc;
+        if (ms < best) {
+          best = ms;
+          bch = ch;
+          bfr = fr;
+          bl = c->spec_lanes;
+        }
       }
     }
   }
   c->spec_ch = bch;
   c->spec_fr = bfr;
-  return MSLR_OK;
-}
-
-// Autotuner, four-pass form: one or two lanes (streams) for the chunks, and
-// the z-mask kernel variant — two CTAs per SM (64 registers), one CTA per SM
-// (more registers, fewer slabs in flight), or two CTAs per SM of fewer warps
-// (more registers per thread) — timed on the chosen chunk shape.
-int tune_sense_variants(Ctx* c, cudaStream_t st) {
-  if (!c->spec || !c->spec_four || c->xy_tc) return MSLR_OK;
-  const int64_t E = (int64_t)c->Nt * c->nvox;
-  const int max_lanes = c->sn_stream ? 2 : 1;
-  float best = 1e30f;
-  int bl = c->spec_lanes, bz = c->spec_zmask_var;
-  for (int lanes = 1; lanes <= max_lanes; ++lanes) {
-    for (int z1 = 0; z1 <= 2; ++z1) {
-      c->spec_lanes = lanes;
-      c->spec_zmask_var = z1;
-      c->spec_zmask_ctas = c->spec_zmask_ctas_v[z1];
-      float ms = 0.f;
-      int rc = time_ms(st, 2, &ms, [&] { return normal_op_spec(c, c->d_ahy, 1, E, c->d_G, false, st); });
-      if (rc) return rc;
-      if (ms < best) {
-        best = ms;
-        bl = lanes;
-        bz = z1;
-      }
-    }
-  }
   c->spec_lanes = bl;
-  c->spec_zmask_var = bz;
-  c->spec_zmask_ctas = c->spec_zmask_ctas_v[bz];
   return MSLR_OK;
 }
 
 int autotune(Ctx* c, cudaStream_t st) {
   int rc = tune_sense_chunks(c, st);
-  if (!rc) rc = tune_sense_variants(c, st);
   if (!rc) rc = tune_svst_splits(c, st);
   if (!rc) rc = tune_eig_variants(c, st);
   if (c->gexec) {   // the captured iteration holds the old launch shapes

@@ -84,8 +84,8 @@ def _fft_flops(n: int) -> float:
 
 
 def four_pass_kernels(N, ch: int, f: int) -> dict:
-    """Per-launch algorithmic bytes and flops of the four kernels of one chunk
-    (ch coils × f frames) of the four-pass SENSE normal operator."""
+    """Per-launch algorithmic bytes and flops of the four kernels of one launch
+    (ch coils × f frames) of the register-line SENSE normal operator."""
     Nx, Ny, Nz = N
     pl = Nx * Ny
     nvox = pl * Nz
@@ -99,11 +99,10 @@ def four_pass_kernels(N, ch: int, f: int) -> dict:
         # the chunk's k-space read and written, the frames' sampling bits
         "zmask": {"bytes": 2 * ch * f * img + mask_bits,
                   "flops": ch * f * Ny * Nx * 2 * _fft_flops(Nz)},
-        # the chunk's k-space read and written, the group's coil maps read
-        "padj": {"bytes": 2 * ch * f * img + ch * img,
-                 "flops": planes * (_fft_flops(pl) + 6.0 * pl)},
-        # the chunk's k-space read, g (or A'y) read, g written
-        "csum": {"bytes": ch * f * img + 2 * f * img, "flops": ch * f * nvox * 2.0},
+        # the chunk's k-space read and written
+        "padj": {"bytes": 2 * ch * f * img, "flops": planes * _fft_flops(pl)},
+        # the chunk's k-space and the group's coil maps read, g (or A'y) read, g written
+        "csum": {"bytes": ch * f * img + ch * img + 2 * f * img, "flops": ch * f * nvox * 8.0},
     }
 
 
