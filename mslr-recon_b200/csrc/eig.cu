@@ -34,11 +34,14 @@
 // Zero patches give no eigenvalue above β² and Ṽ = 0, hence W = 0 (the
 // reference's zero-norm skip, src/recon.jl:185).
 //
-// Split stage (thresholded SVSTs with 64 <= n <= 384): three launches instead
-// of one, so that each phase runs at the occupancy it needs — phase 1 and the
-// WY blocks' T factors (two CTAs per SM), phases 2–3 (four CTAs per SM, all
-// patches resident at once), and phases 4–5 as k_wy_apply: 32 eigenvectors
-// of one patch per CTA, held in registers through every block update.
+// Split stage (thresholded SVSTs with 33 <= n <= 384): three launches instead
+// of one, so that each phase has the shape it needs — phase 1 and the WY
+// blocks' T factors (k_tri_reg: the matrix in registers, n <= 128; k_tri_big:
+// panels), phases 2–3 (four CTAs per SM, all patches resident at once), and
+// phases 4–5 as k_wy_apply: 32 eigenvectors of one patch per CTA, held in
+// registers through every block update.  Phase 1 measured against k_eig's:
+// one patch of side 64 351 → 88 µs, 40 of 128 834 → 244 µs, 2250 of 128 8.0 →
+// 3.9 ms, 486 of 300 12.7 → 8.8 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -408,15 +411,15 @@ __device__ void wy_factors(cf* A, int n, const float* taur, const float* taui, c
       sYb[row * kNb + jj] = y;
     }
     __syncthreads();
-    if (tid < kNb * kNb) {   // Yᴴ Y
-      const int a = tid / kNb, b = tid - a * kNb;
+    for (int t = tid; t < kNb * kNb; t += kT) {   // Yᴴ Y
+      const int a = t / kNb, b = t - a * kNb;
       float sr = 0.f, si = 0.f;
       for (int row = k0 + 1; row < n; ++row) {
         const cf ya = sYb[row * kNb + a], yb = sYb[row * kNb + b];
         sr += ya.x * yb.x + ya.y * yb.y;
         si += ya.x * yb.y - ya.y * yb.x;
       }
-      sYY[tid] = make_float2(sr, si);
+      sYY[t] = make_float2(sr, si);
     }
     __syncthreads();
     if (tid < 32) {   // lane a owns row a of T
@@ -1129,6 +1132,701 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
   }
 }
 
+// ---- tridiagonalisation with the matrix in registers (n <= 128) -------------------
+// Phase 1 for Gram sides up to 32·NT: NT × NT warps hold the whole Hermitian
+// matrix, one 32 × 32 tile per warp, lane (rg, cg) rows rg + 8t and columns
+// cg + 4u of it (32 values).  A step is what k_eig's is — the previous
+// rank-2 update applied on the fly while y = A v is formed — but nothing but
+// vectors moves: the tile pass is six packed FMAs per value on registers with
+// the column's (v, w) from shared memory, and both triangles are stored, so a
+// row's sum is a thread's own and needs no transposed partial sums.
+// Two barriers a step: the column x and its norm's partial sums before the
+// tile pass (which works on the unscaled reflector u = (α − β, x), v = u / (α
+// − β), so no second round publishes v), and the partial sums of A u and of
+// uᴴ A u after it (so no third one reduces vᴴ y).
+// With the matrix in L2 a step cost 5.6 µs whatever n was (n = 64, one
+// patch: 351 µs), the latency of its round trips and four barriers.
+// Tile of warp w: row w / NT, column (w + w / NT) mod NT, so that the tiles
+// left in play when the leading ones are done stay spread over the SM's four
+// schedulers.
+template <int NT>
+struct TriVec {
+  static constexpr int NP = 32 * NT, LD = NP + 1;
+  float4 dw[NP], dv[NP];  // the pending update of column j: (wp.x, wp.x, wp.y, wp.y), (vp.x, vp.x, vp.y, vp.y)
+  float4 sx[NP];          // this step's column x below the subdiagonal: (x.x, x.y, x.y, x.x)
+  cf scol[NP];            // next column, before the pending update
+  cf part[NT][NP];        // per tile column: partial sums of A u
+  float red0[4], redt[16];
+  cf x1;
+};
+
+// The n steps of the n × n Hermitian matrix at A (column stride ld, n <= 32·NT,
+// lower triangle read): d, e and τ; reflectors below A's subdiagonal and, when
+// given, in Y (unit entry and zeros included).  NT·NT warps.
+template <int NT>
+__device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, double* dd, double* ee, cf* taus,
+                                          cf* Y) {
+  constexpr int NP = 32 * NT, LD = TriVec<NT>::LD;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int I = warp / NT, J = (warp + I) % NT;
+  const int rg = lane >> 2, cg = lane & 3;
+
+  // the tile, from the lower triangle
+  cf a[4][8];
+#pragma unroll
+  for (int t = 0; t < 4; ++t)
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int r = I * 32 + rg + 8 * t, c = J * 32 + cg + 4 * u;
+      cf v = make_float2(0.f, 0.f);
+      if (r < n && c < n) {
+        v = r >= c ? __ldcg(A + (int64_t)c * ld + r) : __ldcg(A + (int64_t)r * ld + c);
+        if (r < c) v.y = -v.y;
+        if (r == c) v.y = 0.f;
+      }
+      a[t][u] = v;
+    }
+  const int i = tid;                 // row of the vector phases
+  const bool own = tid < NP;         // (the first NT warps)
+  if (own) {
+    m.dw[i] = m.dv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    m.scol[i] = (i < n) ? __ldcg(A + i) : make_float2(0.f, 0.f);
+  }
+  const int row = I * 32 + rg + 8 * cg;   // row whose sum this lane ends with
+  cf vpi = make_float2(0.f, 0.f), wpi = vpi, vpk = vpi, wpk = vpi;
+  for (int k = 0; k < n - 1; ++k) {
+    // column k with the pending update; its norm below the subdiagonal
+    cf x = make_float2(0.f, 0.f);
+    if (own) {
+      if (i >= k && i < n) x = csub(m.scol[i], cadd(cmul(vpi, cconj(wpk)), cmul(wpi, cconj(vpk))));
+      if (i == k) dd[k] = (double)x.x;
+      if (i == k + 1) m.x1 = x;
+      if (i <= k + 1) x = make_float2(0.f, 0.f);
+      m.sx[i] = make_float4(x.x, x.y, x.y, x.x);
+      const float q = warp_sum(cabs2(x));
+      if (lane == 0) m.red0[warp] = q;
+    }
+    __syncthreads();
+    float xn = 0.f;
+#pragma unroll
+    for (int q = 0; q < NT; ++q) xn += m.red0[q];
+    // zlarfg, by every thread on the same values: Hᴴ (α, x) = (β, 0), H = I − τ v vᴴ, β real
+    const float ar = m.x1.x, ai = m.x1.y;
+    float bt = ar;
+    cf tau = make_float2(0.f, 0.f), scal = make_float2(1.f, 0.f), u1 = scal;
+    const bool refl = !(xn == 0.f && ai == 0.f);
+    if (refl) {
+      bt = -copysignf(sqrtf(ar * ar + ai * ai + xn), ar);
+      const float ib = 1.f / bt;
+      tau = make_float2((bt - ar) * ib, -ai * ib);
+      u1 = make_float2(ar - bt, ai);
+      const float id = 1.f / (u1.x * u1.x + ai * ai);
+      scal = make_float2(u1.x * id, -ai * id);
+    }
+    // A ← A − (vp wpᴴ + wp vpᴴ), A u on the tiles still in play
+    float tq = 0.f;
+    if (I * 32 + 31 > k && J * 32 + 31 > k) {
+      const int c0 = J * 32 + cg;
+      {
+        cf r1[4], r2[4], r3[4], r4[4];   // −(vp), −(vp rotated), −(wp), −(wp rotated) of the rows
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const float4 w = m.dw[I * 32 + rg + 8 * t], v = m.dv[I * 32 + rg + 8 * t];
+          r1[t] = make_float2(-v.x, -v.z);
+          r2[t] = make_float2(-v.z, v.x);
+          r3[t] = make_float2(-w.x, -w.z);
+          r4[t] = make_float2(-w.z, w.x);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {   // a −= vp conj(wp_j) + wp conj(vp_j)
+          const float4 w = m.dw[c0 + 4 * u], v = m.dv[c0 + 4 * u];
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            cf e = a[t][u];
+            e = __ffma2_rn(r1[t], make_float2(w.x, w.y), e);
+            e = __ffma2_rn(r2[t], make_float2(w.z, w.w), e);
+            e = __ffma2_rn(r3[t], make_float2(v.x, v.y), e);
+            a[t][u] = __ffma2_rn(r4[t], make_float2(v.z, v.w), e);
+          }
+        }
+      }
+      cf y[4];
+      {
+        cf P[4], Q[4];   // (Σ a.x x.x, Σ a.y x.y), (Σ a.x x.y, Σ a.y x.x)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) P[t] = Q[t] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const float4 v = m.sx[c0 + 4 * u];
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            P[t] = __ffma2_rn(a[t][u], make_float2(v.x, v.y), P[t]);
+            Q[t] = __ffma2_rn(a[t][u], make_float2(v.z, v.w), Q[t]);
+          }
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) y[t] = make_float2(P[t].x - P[t].y, Q[t].x + Q[t].y);
+      }
+      if (J == (k + 1) >> 5) {   // column k + 1: entry u1 of u, and the next step's column
+        const int us = ((k + 1) & 31) >> 2;
+        cf nx[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) nx[t] = a[t][0];
+#pragma unroll
+        for (int u = 1; u < 8; ++u)
+          if (u == us) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) nx[t] = a[t][u];
+          }
+        if (cg == ((k + 1) & 3)) {
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            m.scol[I * 32 + rg + 8 * t] = nx[t];
+            y[t] = cadd(y[t], cmul(nx[t], u1));
+          }
+        }
+      }
+      // sums over the four column groups; lane cg ends with row t = cg
+      const bool h2 = cg & 2, h1 = cg & 1;
+      cf z0 = h2 ? y[2] : y[0], z1 = h2 ? y[3] : y[1];
+      const cf o0 = h2 ? y[0] : y[2], o1 = h2 ? y[1] : y[3];
+      z0.x += __shfl_xor_sync(0xffffffffu, o0.x, 2);
+      z0.y += __shfl_xor_sync(0xffffffffu, o0.y, 2);
+      z1.x += __shfl_xor_sync(0xffffffffu, o1.x, 2);
+      z1.y += __shfl_xor_sync(0xffffffffu, o1.y, 2);
+      cf z = h1 ? z1 : z0;
+      const cf o = h1 ? z0 : z1;
+      z.x += __shfl_xor_sync(0xffffffffu, o.x, 1);
+      z.y += __shfl_xor_sync(0xffffffffu, o.y, 1);
+      m.part[J][row] = z;
+      const float4 xr = m.sx[row];
+      const cf ur = row == k + 1 ? u1 : make_float2(xr.x, xr.y);
+      tq = warp_sum(ur.x * z.x + ur.y * z.y);   // uᴴ A u is real
+    }
+    if (lane == 0) m.redt[warp] = tq;
+    __syncthreads();
+    if (own) {
+      // y = A v of this row and of row k + 1 (the next pivot row), in tile order
+      cf y = make_float2(0.f, 0.f), y1 = y;
+      const int q0 = (k + 1) >> 5;
+#pragma unroll
+      for (int q = 0; q < NT; ++q)
+        if (q >= q0) {
+          y = cadd(y, m.part[q][i]);
+          y1 = cadd(y1, m.part[q][k + 1]);
+        }
+      float t = 0.f;
+#pragma unroll
+      for (int q = 0; q < NT * NT; ++q) t += m.redt[q];
+      const float c = 0.5f * (tau.x * tau.x + tau.y * tau.y) * (scal.x * scal.x + scal.y * scal.y) * t;
+      const cf vi = i == k + 1 ? make_float2(1.f, 0.f) : cmul(x, scal);   // 0 for i <= k and i >= n
+      if (i == k + 1) {
+        ee[k] = (double)bt;
+        taus[k] = tau;
+      }
+      if (Y) Y[k * LD + i] = vi;
+      if (i >= k + 2 && i < n) A[(int64_t)k * ld + i] = vi;   // reflector kept below the subdiagonal
+      vpi = vpk = wpi = wpk = make_float2(0.f, 0.f);
+      if (refl) {
+        const cf ts = cmul(tau, scal);
+        const cf t1 = cmul(ts, y1), ty = cmul(ts, y);
+        vpk = make_float2(1.f, 0.f);
+        wpk = make_float2(t1.x - c, t1.y);
+        if (i > k && i < n) {
+          vpi = vi;
+          wpi = make_float2(ty.x - c * vi.x, ty.y - c * vi.y);
+        }
+      }
+      m.dv[i] = make_float4(vpi.x, vpi.x, vpi.y, vpi.y);
+      m.dw[i] = make_float4(wpi.x, wpi.x, wpi.y, wpi.y);
+    }
+    // what the next step's first phase reads was written before the last
+    // barrier or is this thread's own
+  }
+  if (own && i == n - 1) {
+    const cf x = csub(m.scol[i], cadd(cmul(vpi, cconj(wpi)), cmul(wpi, cconj(vpi))));
+    dd[n - 1] = (double)x.x;
+    ee[n - 1] = 0.0;
+  }
+  __syncthreads();
+}
+
+// Row `lane` of the T factor (zlarft, forward columnwise) of one WY block by
+// one warp: tau of its nb reflectors, G the products Yᴴ Y above the diagonal,
+// column by column; into the block's upper slots of A.
+__device__ __forceinline__ void wy_tfactor(cf* A, int n, int blk, const cf* tau, int nb, const cf* G) {
+  const int lane = threadIdx.x & 31;
+  cf t[kNb];
+#pragma unroll
+  for (int jj = 0; jj < kNb; ++jj) {
+    const cf tj = jj < nb ? tau[jj] : make_float2(0.f, 0.f);
+    cf sacc = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int b = 0; b < jj; ++b) sacc = cadd(sacc, cmul(t[b], G[jj * (jj - 1) / 2 + b]));
+    const cf v = cmul(tj, sacc);
+    t[jj] = lane == jj ? tj : lane < jj ? make_float2(-v.x, -v.y) : make_float2(0.f, 0.f);
+  }
+  if (lane < kNb) {
+#pragma unroll
+    for (int jj = 0; jj < kNb; ++jj) A[upper_slot(n, blk * kNb * kNb + lane * kNb + jj)] = t[jj];
+  }
+}
+// entry e of a block's G: column jj, row b < jj
+__device__ __forceinline__ void g_entry(int e, int* jj, int* b) {
+  int j = 1;
+  while ((j + 1) * j / 2 <= e) ++j;
+  *jj = j;
+  *b = e - j * (j - 1) / 2;
+}
+
+template <int NT>
+struct TriSmem {
+  TriVec<NT> v;
+  double dd[32 * NT], ee[32 * NT];
+  cf tau[32 * NT];
+  cf Y[32 * NT * TriVec<NT>::LD];   // reflectors, Y[k·LD + i]
+  cf G[NT * 2][120];                // per WY block: Yᴴ Y above the diagonal
+};
+
+template <int NT>
+__global__ void __launch_bounds__(NT * NT * 32, NT == 4 ? 1 : NT == 3 ? 2 : NT == 2 ? 4 : 8) k_tri_reg(EigArgs g) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  TriSmem<NT>& m = *reinterpret_cast<TriSmem<NT>*>(smraw);
+  int s = 0;
+  while (s + 1 < g.nseg && (int64_t)blockIdx.x >= g.seg[s + 1].first) ++s;
+  const Seg& S = g.seg[s];
+  const int n = S.n;
+  const int64_t ip = (int64_t)blockIdx.x - S.first;
+  constexpr int kThreads = NT * NT * 32, LD = TriVec<NT>::LD;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  cf* A = S.gram + ip * (int64_t)n * n;
+  tri_steps<NT>(A, n, n, m.v, m.dd, m.ee, m.tau, m.Y);
+  double* side = S.side + ip * 6 * (int64_t)n;
+  for (int q = tid; q < n; q += kThreads) {
+    side[q] = m.dd[q];
+    side[n + q] = m.ee[q];
+  }
+  // the T factors of all WY blocks, from the last reflector down: the products
+  // Yᴴ Y of every block at once, then one warp per block
+  const int nref = n - 1, nblk = (nref + kNb - 1) / kNb;
+  for (int q = tid; q < nblk * 120; q += kThreads) {
+    const int blk = q / 120, e = q - blk * 120;
+    int jj, b;
+    g_entry(e, &jj, &b);
+    const int kend = nref - blk * kNb, k0 = max(0, kend - kNb);
+    float sr = 0.f, si = 0.f;
+    if (jj < kend - k0) {
+      const cf* ya = m.Y + (k0 + b) * LD;
+      const cf* yb = m.Y + (k0 + jj) * LD;
+#pragma unroll 8
+      for (int row = k0 + jj + 1; row < n; ++row) {
+        sr += ya[row].x * yb[row].x + ya[row].y * yb[row].y;
+        si += ya[row].x * yb[row].y - ya[row].y * yb[row].x;
+      }
+    }
+    m.G[blk][e] = make_float2(sr, si);
+  }
+  __syncthreads();
+  for (int blk = warp; blk < nblk; blk += kThreads / 32) {
+    const int kend = nref - blk * kNb, k0 = max(0, kend - kNb);
+    wy_tfactor(A, n, blk, m.tau + k0, kend - k0, m.G[blk]);
+  }
+}
+
+// ---- blocked tridiagonalisation (128 < n <= 384) --------------------------------------
+// The leading n − 128 columns in panels of eight with the matrix in L2, the
+// trailing 128 × 128 block in registers (tri_steps).  Within a panel the
+// matrix is only read: column k gets its pending updates from the panel's V
+// and W in shared memory, and y = A u − V (Wᴴ u) − W (Vᴴ u); the rank-16 update
+// of the trailing lower triangle follows at the panel's end.  k_eig reads and
+// writes the triangle every step instead, and spends most of its time on
+// per-tile bookkeeping (486 patches of side 300: 12.7 ms).
+// The matrix–vector product reads the lower triangle once, in groups of 64
+// rows × 8 columns (lane = two rows, eight 16-byte loads in flight): each value
+// serves its row (kept in the lane while the warp's groups stay in one 64-row
+// chunk) and its column (a shuffle transpose of the group's eight sums).
+// So that no value needs a test, the diagonal 64 × 64 blocks are kept with
+// zeros above the diagonal and half the diagonal (each half counts once in the
+// row's and once in the column's sum).
+// Each warp takes an equal share of the groups, chunk by chunk, and every
+// partial sum has its own slot, added up in a fixed order.  One 512-thread CTA
+// per SM, so that the working set, 148 triangles, stays in L2.
+constexpr int kPb = 8;            // panel width
+constexpr int kBigT = 512;
+constexpr int kBigW = kBigT / 32;
+constexpr int kTail = 128;        // trailing block in registers
+constexpr int kChunks = kSmallT / 64;
+
+struct BigSmem {
+  union {
+    struct {
+      float4 vw[kPb][kSmallT];                      // the panel's (v, w), by row
+      cf rowp[kChunks][kBigW][64];                  // row sums: chunk, warp
+      cf colp[kChunks][kSmallT];                    // column sums: chunk
+      float4 sx[kSmallT];                           // u: (x.x, x.y, x.y, x.x)
+      float4 g[kPb];                                // (Vᴴ u, Wᴴ u)
+      float red0[kBigW], redt[kBigW];
+      cf x1;
+    } p;
+    TriVec<4> t;
+    struct {
+      cf Y[4][kSmallT * kNb];                       // four WY blocks' reflectors, [row][reflector]
+      cf G[4][120];
+    } y;
+  };
+  double dd[kSmallT], ee[kSmallT];
+  cf tau[kSmallT];
+};
+
+// Groups of 64 rows × 8 columns of the lower triangle from column o on, chunk
+// by chunk (chunk q: rows 64q …), the first chunk being the one of row o.
+__device__ __forceinline__ int groups_of(int o, int q, int n) {   // of chunk q
+  return min(8 * (q + 1), (n + 7) >> 3) - (o >> 3);
+}
+__device__ __forceinline__ int groups_before(int o, int q) {   // of the chunks before q (none of them the last)
+  const int q0 = o >> 6;
+  return 4 * (q * (q + 1) - q0 * (q0 + 1)) - (q - q0) * (o >> 3);
+}
+__device__ __forceinline__ int groups_all(int o, int n) {
+  const int ql = (n - 1) >> 6;
+  return groups_before(o, ql) + groups_of(o, ql, n);
+}
+struct GroupIt {
+  int q, base, cnt;
+  // moves on to the chunk of group gi; the group's first column
+  __device__ __forceinline__ int col(int o, int n, int gi) {
+    while (gi >= base + cnt) {
+      base += cnt;
+      ++q;
+      cnt = groups_of(o, q, n);
+    }
+    return (o & ~7) + 8 * (gi - base);
+  }
+};
+
+// rows r (even) and r + 1 of a column; rows at or beyond n read the last ones
+template <bool EVEN>
+__device__ __forceinline__ void load2(cf* a0, cf* a1, const cf* col, int r, int n) {
+  if constexpr (EVEN) {
+    const float4 v = __ldcg(reinterpret_cast<const float4*>(col + min(r, n - 2)));
+    *a0 = make_float2(v.x, v.y);
+    *a1 = make_float2(v.z, v.w);
+  } else {
+    *a0 = __ldcg(col + min(r, n - 1));
+    *a1 = __ldcg(col + min(r + 1, n - 1));
+  }
+}
+
+template <bool EVEN>
+__global__ void __launch_bounds__(kBigT, 1) k_tri_big(EigArgs g) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  BigSmem& m = *reinterpret_cast<BigSmem*>(smraw);
+  int s = 0;
+  while (s + 1 < g.nseg && (int64_t)blockIdx.x >= g.seg[s + 1].first) ++s;
+  const Seg& S = g.seg[s];
+  const int n = S.n;
+  const int64_t ip = (int64_t)blockIdx.x - S.first;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  cf* A = S.gram + ip * (int64_t)n * n;
+  const int i = tid;   // row of the vector phases
+  const int nchunk = (n + 63) >> 6;
+  for (int c = warp; c < n; c += kBigW) {   // the diagonal blocks (see above)
+    cf* col = A + (int64_t)c * n;
+    for (int r = (c & ~63) + lane; r < c; r += 32) col[r] = make_float2(0.f, 0.f);
+    if (lane == 0) col[c] = make_float2(0.5f * __ldcg(&col[c].x), 0.f);
+  }
+  __syncthreads();
+  int k = 0;
+  while (n - k > kTail) {
+    const int p0 = k, pe = min(p0 + kPb, n - kTail);   // this panel's columns
+    cf xraw = (i >= p0 && i < n) ? __ldcg(A + (int64_t)p0 * n + i) : make_float2(0.f, 0.f);
+    for (; k < pe; ++k) {
+      const int np = k - p0;
+      // column k with the panel's updates so far
+      cf x = make_float2(0.f, 0.f);
+      if (i >= k && i < n) {
+        x = xraw;
+        if (i == k) x.x *= 2.f;
+#pragma unroll 4
+        for (int p = 0; p < np; ++p) {
+          const float4 a = m.p.vw[p][i], b = m.p.vw[p][k];   // − v conj(w_k) − w conj(v_k)
+          x.x -= a.x * b.z + a.y * b.w + a.z * b.x + a.w * b.y;
+          x.y -= a.y * b.z - a.x * b.w + a.w * b.x - a.z * b.y;
+        }
+      }
+      if (k + 1 < pe && i > k && i < n) xraw = __ldcg(A + (int64_t)(k + 1) * n + i);   // the next column
+      if (i == k) m.dd[k] = (double)x.x;
+      if (i == k + 1) m.p.x1 = x;
+      if (i <= k + 1) x = make_float2(0.f, 0.f);
+      if (i < kSmallT) m.p.sx[i] = make_float4(x.x, x.y, x.y, x.x);
+      {
+        const float q = warp_sum(cabs2(x));
+        if (lane == 0) m.p.red0[warp] = q;
+      }
+      __syncthreads();
+      float xn = 0.f;
+#pragma unroll
+      for (int q = 0; q < kBigW; ++q) xn += m.p.red0[q];
+      // zlarfg as in tri_steps: u = (α − β, x), v = scal · u
+      const float ar = m.p.x1.x, ai = m.p.x1.y;
+      float bt = ar;
+      cf tau = make_float2(0.f, 0.f), scal = make_float2(1.f, 0.f), u1 = scal;
+      const bool refl = !(xn == 0.f && ai == 0.f);
+      if (refl) {
+        bt = -copysignf(sqrtf(ar * ar + ai * ai + xn), ar);
+        const float ib = 1.f / bt;
+        tau = make_float2((bt - ar) * ib, -ai * ib);
+        u1 = make_float2(ar - bt, ai);
+        const float id = 1.f / (u1.x * u1.x + ai * ai);
+        scal = make_float2(u1.x * id, -ai * id);
+      }
+      const int o = k + 1;
+      if (i == o) m.p.sx[o] = make_float4(u1.x, u1.y, u1.y, u1.x);
+      __syncthreads();
+      // Wᴴ u and Vᴴ u of the panel's earlier columns, one per warp
+      if (warp < np) {
+        cf gw = make_float2(0.f, 0.f), gv = gw;
+        for (int r = o + lane; r < n; r += 32) {
+          const float4 q = m.p.sx[r];
+          const cf u = make_float2(q.x, q.y);
+          const float4 a = m.p.vw[warp][r];
+          const cf v = make_float2(a.x, a.y), w = make_float2(a.z, a.w);
+          gw.x += w.x * u.x + w.y * u.y;
+          gw.y += w.x * u.y - w.y * u.x;
+          gv.x += v.x * u.x + v.y * u.y;
+          gv.y += v.x * u.y - v.y * u.x;
+        }
+        gw.x = warp_sum(gw.x);
+        gw.y = warp_sum(gw.y);
+        gv.x = warp_sum(gv.x);
+        gv.y = warp_sum(gv.y);
+        if (lane == 0) m.p.g[warp] = make_float4(gv.x, gv.y, gw.x, gw.y);
+      }
+      // A u over this warp's groups, the next group's values on their way
+      float tq = 0.f;
+      {
+        const int G = groups_all(o, n);
+        const int ge = (warp + 1) * G / kBigW;
+        int gi = warp * G / kBigW;
+        GroupIt it{o >> 6, 0, groups_of(o, o >> 6, n)};
+        int c0 = it.col(o, n, gi), q = it.q, cur = -1, r = 0;
+        cf u0 = make_float2(0.f, 0.f), uu = u0;         // u of the lane's two rows
+        cf P0 = u0, Q0 = u0, P1 = u0, Q1 = u0;           // row sums (Σ a.x u.x, Σ a.y u.y), (Σ a.x u.y, Σ a.y u.x)
+        cf a0[8], a1[8];
+        if (gi < ge) {
+#pragma unroll
+          for (int b = 0; b < 8; ++b)
+            load2<EVEN>(&a0[b], &a1[b], A + (int64_t)min(c0 + b, n - 1) * n, 64 * q + 2 * lane, n);
+        }
+        auto flush = [&]() {
+          if (cur < 0) return;
+          const cf y0 = make_float2(P0.x - P0.y, Q0.x + Q0.y), y1 = make_float2(P1.x - P1.y, Q1.x + Q1.y);
+          *reinterpret_cast<float4*>(&m.p.rowp[cur][warp][2 * lane]) = make_float4(y0.x, y0.y, y1.x, y1.y);
+          tq += u0.x * y0.x + u0.y * y0.y + uu.x * y1.x + uu.y * y1.y;
+        };
+        for (; gi < ge; ++gi) {
+          if (q != cur) {
+            flush();
+            cur = q;
+            r = 64 * q + 2 * lane;
+            const float4 q0 = r < n ? m.p.sx[r] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 q1 = r + 1 < n ? m.p.sx[r + 1] : make_float4(0.f, 0.f, 0.f, 0.f);
+            u0 = make_float2(q0.x, q0.y);
+            uu = make_float2(q1.x, q1.y);
+            P0 = Q0 = P1 = Q1 = make_float2(0.f, 0.f);
+          }
+          int nq = q, nc0 = c0;
+          if (gi + 1 < ge) {
+            nc0 = it.col(o, n, gi + 1);
+            nq = it.q;
+          }
+          const cf* nxt = A + (int64_t)nc0 * n;
+          const int nr = 64 * nq + 2 * lane;
+          float cr[8], ci[8];
+          const cf s0 = make_float2(u0.y, u0.x), s1 = make_float2(uu.y, uu.x);
+#pragma unroll
+          for (int b = 0; b < 8; ++b) {
+            // u of columns before o, of columns at or beyond n and of such rows is zero
+            const float4 v = m.p.sx[c0 + b];
+            const cf e0 = a0[b], e1 = a1[b];
+            load2<EVEN>(&a0[b], &a1[b], nxt + (int64_t)min(b, n - 1 - nc0) * n, nr, n);
+            P0 = __ffma2_rn(e0, make_float2(v.x, v.y), P0);
+            Q0 = __ffma2_rn(e0, make_float2(v.z, v.w), Q0);
+            P1 = __ffma2_rn(e1, make_float2(v.x, v.y), P1);
+            Q1 = __ffma2_rn(e1, make_float2(v.z, v.w), Q1);
+            const cf pc = __ffma2_rn(e1, uu, __fmul2_rn(e0, u0)), qc = __ffma2_rn(e1, s1, __fmul2_rn(e0, s0));
+            cr[b] = pc.x + pc.y;   // conj(a) u
+            ci[b] = qc.x - qc.y;
+          }
+          col_sums(cr, ci, lane);
+          if ((lane & 3) == 0) {
+            const int c = c0 + (lane >> 2);
+            m.p.colp[q][c] = make_float2(cr[0], ci[0]);
+            const float4 v = m.p.sx[c];
+            tq += v.x * cr[0] + v.y * ci[0];
+          }
+          q = nq;
+          c0 = nc0;
+        }
+        flush();
+      }
+      tq = warp_sum(tq);
+      if (lane == 0) m.p.redt[warp] = tq;
+      __syncthreads();
+      // y = A u − V (Wᴴ u) − W (Vᴴ u); uᴴ y; w
+      {
+        float t = 0.f;
+#pragma unroll
+        for (int q = 0; q < kBigW; ++q) t += m.p.redt[q];
+        for (int p = 0; p < np; ++p) {
+          const float4 a = m.p.g[p];
+          t -= 2.f * (a.x * a.z + a.y * a.w);
+        }
+        const float c = 0.5f * (tau.x * tau.x + tau.y * tau.y) * (scal.x * scal.x + scal.y * scal.y) * t;
+        cf vi = make_float2(0.f, 0.f), wi = vi;
+        if (i > k && i < n) {
+          cf y = make_float2(0.f, 0.f);
+          // group x belongs to warp ⌈16 (x + 1) / G⌉ − 1 (G >= 16: no warp is without groups)
+          const int q = i >> 6, G = groups_all(o, n), gb = groups_before(o, q);
+          const int w0 = (kBigW * (gb + 1) + G - 1) / G - 1;
+          const int w1 = (kBigW * (gb + groups_of(o, q, n)) + G - 1) / G - 1;
+          for (int w = w0; w <= w1; ++w) y = cadd(y, m.p.rowp[q][w][i & 63]);
+          for (int q2 = q; q2 < nchunk; ++q2) y = cadd(y, m.p.colp[q2][i]);
+#pragma unroll 4
+          for (int p = 0; p < np; ++p) {
+            const float4 a = m.p.vw[p][i], b = m.p.g[p];
+            y = csub(y, cadd(cmul(make_float2(a.x, a.y), make_float2(b.z, b.w)),
+                             cmul(make_float2(a.z, a.w), make_float2(b.x, b.y))));
+          }
+          vi = i == o ? make_float2(1.f, 0.f) : cmul(x, scal);
+          if (i == o) {
+            m.ee[k] = (double)bt;
+            m.tau[k] = tau;
+          } else {
+            A[(int64_t)k * n + i] = vi;   // reflector kept below the subdiagonal
+          }
+          if (refl) {
+            const cf ty = cmul(cmul(tau, scal), y);
+            wi = make_float2(ty.x - c * vi.x, ty.y - c * vi.y);
+          }
+          if (!refl) vi = make_float2(0.f, 0.f);
+        }
+        if (i < kSmallT) {
+          m.p.vw[np][i] = make_float4(vi.x, vi.y, wi.x, wi.y);
+        }
+      }
+      __syncthreads();
+    }
+    // A ← A − V Wᴴ − W Vᴴ on the trailing lower triangle, groups as above
+    {
+      const int np = pe - p0, o = pe;
+      const int G = groups_all(o, n);
+      const float dh = n - pe == kTail ? 1.f : 0.5f;   // the trailing block goes on with its whole diagonal
+      GroupIt it{o >> 6, 0, groups_of(o, o >> 6, n)};
+      for (int gi = warp; gi < G; gi += kBigW) {
+        const int c0 = it.col(o, n, gi), r = 64 * it.q + 2 * lane;
+        cf a0[8], a1[8];
+#pragma unroll
+        for (int b = 0; b < 8; ++b) load2<EVEN>(&a0[b], &a1[b], A + (int64_t)min(c0 + b, n - 1) * n, r, n);
+        if (c0 + 8 > 64 * it.q) {   // the whole diagonal
+#pragma unroll
+          for (int b = 0; b < 8; ++b) {
+            if (r == c0 + b) a0[b].x *= 2.f;
+            if (r + 1 == c0 + b) a1[b].x *= 2.f;
+          }
+        }
+        const int rs = min(r, kSmallT - 2);
+#pragma unroll 2
+        for (int p = 0; p < np; ++p) {
+          const float4 x0 = m.p.vw[p][rs], x1 = m.p.vw[p][rs + 1];
+#pragma unroll
+          for (int b = 0; b < 8; ++b) {
+            const float4 c = m.p.vw[p][min(c0 + b, kSmallT - 1)];
+            auto upd = [&](cf& e, const float4& x) {   // e −= v conj(w_c) + w conj(v_c)
+              e.x = fmaf(-x.x, c.z, e.x);
+              e.y = fmaf(-x.y, c.z, e.y);
+              e.x = fmaf(-x.y, c.w, e.x);
+              e.y = fmaf(x.x, c.w, e.y);
+              e.x = fmaf(-x.z, c.x, e.x);
+              e.y = fmaf(-x.w, c.x, e.y);
+              e.x = fmaf(-x.w, c.y, e.x);
+              e.y = fmaf(x.z, c.y, e.y);
+            };
+            upd(a0[b], x0);
+            upd(a1[b], x1);
+          }
+        }
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+          const int c = c0 + b;
+          if (c < o || c >= n) continue;
+          if (r == c) a0[b] = make_float2(dh * a0[b].x, 0.f);
+          if (r + 1 == c) a1[b] = make_float2(dh * a1[b].x, 0.f);
+          cf* d = A + (int64_t)c * n + r;
+          if (EVEN && r >= c && r + 1 < n) {
+            *reinterpret_cast<float4*>(d) = make_float4(a0[b].x, a0[b].y, a1[b].x, a1[b].y);
+          } else {
+            if (r >= c && r < n) d[0] = a0[b];
+            if (r + 1 >= c && r + 1 < n) d[1] = a1[b];
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  tri_steps<4>(A + (int64_t)k * n + k, n, n - k, m.t, m.dd + k, m.ee + k, m.tau + k, nullptr);
+  double* side = S.side + ip * 6 * (int64_t)n;
+  for (int q = tid; q < n; q += kBigT) {
+    side[q] = m.dd[q];
+    side[n + q] = m.ee[q];
+  }
+  // T factors, four WY blocks at a time
+  const int nref = n - 1, nblk = (nref + kNb - 1) / kNb;
+  for (int b0 = 0; b0 < nblk; b0 += 4) {
+    const int nb4 = min(4, nblk - b0);
+    __syncthreads();
+    for (int q = warp; q < nb4 * kNb; q += kBigW) {   // one reflector per warp
+      const int bl = q >> 4, jj = q & 15;
+      const int kend = nref - (b0 + bl) * kNb, k0 = max(0, kend - kNb), kk = k0 + jj;
+      cf* y = m.y.Y[bl] + jj;
+      for (int r = k0 + lane; r < n; r += 32) {
+        cf v = make_float2(0.f, 0.f);
+        if (kk < kend) {
+          if (r == kk + 1) v = make_float2(1.f, 0.f);
+          else if (r > kk + 1) v = __ldcg(A + (int64_t)kk * n + r);
+        }
+        y[r * kNb] = v;
+      }
+    }
+    __syncthreads();
+    if (tid < nb4 * 120) {
+      const int bl = tid / 120, e = tid - bl * 120;
+      int jj, b;
+      g_entry(e, &jj, &b);
+      const int kend = nref - (b0 + bl) * kNb, k0 = max(0, kend - kNb);
+      const cf* y = m.y.Y[bl];
+      float sr = 0.f, si = 0.f;
+#pragma unroll 8
+      for (int r = k0 + jj + 1; r < n; ++r) {
+        const cf ya = y[r * kNb + b], yb = y[r * kNb + jj];
+        sr += ya.x * yb.x + ya.y * yb.y;
+        si += ya.x * yb.y - ya.y * yb.x;
+      }
+      m.y.G[bl][e] = make_float2(sr, si);
+    }
+    __syncthreads();
+    if (warp < nb4) {
+      const int blk = b0 + warp, kend = nref - blk * kNb, k0 = max(0, kend - kNb);
+      wy_tfactor(A, n, blk, m.tau + k0, kend - k0, m.y.G[warp]);
+    }
+  }
+}
+
+template <int NT>
+void tri_reg_launch(const EigArgs& a, unsigned grid, cudaStream_t st) {
+  k_tri_reg<NT><<<grid, NT * NT * 32, sizeof(TriSmem<NT>), st>>>(a);
+}
+
 // ---- split stage, third launch: Ṽ = conj(Q Z) diag(√h) -------------------------
 // One CTA per (32 eigenvectors, patch); warp w holds rows w, w + 16, … of its
 // 32 vectors in registers (lane = vector) through all WY blocks, taken from
@@ -1324,9 +2022,13 @@ int eig2_prepare(int nmax) {
   MSLR_CUDA_TRY(cudaFuncSetAttribute(k_eig<kT, 1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   MSLR_CUDA_TRY(cudaFuncSetAttribute(k_eig<kSmallT, 2, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, small));
   MSLR_CUDA_TRY(cudaFuncSetAttribute(k_eig<kT, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_eig<kSmallT, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, small));
   MSLR_CUDA_TRY(cudaFuncSetAttribute(k_eig<kSmallT, kPairsMinB, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)(228 * 1024 / kPairsMinB - 1024)));
+  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_tri_reg<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TriSmem<3>)));
+  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_tri_reg<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TriSmem<4>)));
+  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_tri_big<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BigSmem)));
+  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_tri_big<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BigSmem)));
+  static_assert(sizeof(BigSmem) <= 227 * 1024, "shared memory of the blocked tridiagonalisation");
   const int wy = (int)wy_apply_smem(kSmallT);
   MSLR_CUDA_TRY(cudaFuncSetAttribute(k_wy_apply<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, wy));
   MSLR_CUDA_TRY(cudaFuncSetAttribute(k_wy_apply<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, wy));
@@ -1340,15 +2042,15 @@ int eig2_prepare(int nmax) {
 namespace {
 
 // The split stage applies to thresholded SVSTs (not the values-only or
-// all-eigenpairs modes) with a side buffer and 64 <= n <= 384 (the
-// back-transform's register tile; the T factors fit the upper triangle).
+// all-eigenpairs modes) with a side buffer and 33 <= n <= 384 (the
+// back-transform's register tile) whose T factors fit the upper triangle.
 // MSLR_EIG_SPLIT=0 keeps the one-launch stage everywhere (for comparisons).
 bool split_ok(const EigSegment& e) {
   static const bool off = [] {
     const char* v = std::getenv("MSLR_EIG_SPLIT");
     return v && v[0] == '0';
   }();
-  if (off || !e.side || e.nuc || e.lam_out || e.n < 64 || e.n > kSmallT) return false;
+  if (off || !e.side || e.nuc || e.lam_out || e.n <= 32 || e.n > kSmallT) return false;
   const int64_t nblk = (e.n - 1 + kNb - 1) / kNb;
   return nblk * kNb * kNb <= (int64_t)e.n * (e.n - 1) / 2;
 }
@@ -1366,7 +2068,29 @@ int wy_apply_launch(const EigArgs& a, int nmax, int64_t total, cudaStream_t st) 
   return MSLR_OK;
 }
 
-// One launch (or, for the split stage, three) over segments that all take the
+// Phase 1 of the split stage for one segment: the matrix in registers up to
+// 128, the blocked form above (16-byte loads need an even side and a 16-byte
+// aligned buffer); the autotuner's 1024-thread variant keeps the step-by-step form.
+void tri_launch(const EigArgs& a, bool big, cudaStream_t st) {
+  const Seg& S = a.seg[0];
+  const int n = S.n;
+  const unsigned grid = (unsigned)S.np;
+  if (big) {
+    k_eig<kT, 1, 1><<<grid, kT, vec_bytes(n) + wy_bytes(n, kT) + 128, st>>>(a);
+  } else if (n <= 64) {
+    tri_reg_launch<2>(a, grid, st);
+  } else if (n <= 96) {
+    tri_reg_launch<3>(a, grid, st);
+  } else if (n <= kTail) {
+    tri_reg_launch<4>(a, grid, st);
+  } else if (n % 2 == 0 && (reinterpret_cast<uintptr_t>(S.gram) & 15) == 0) {
+    k_tri_big<true><<<grid, kBigT, sizeof(BigSmem), st>>>(a);
+  } else {
+    k_tri_big<false><<<grid, kBigT, sizeof(BigSmem), st>>>(a);
+  }
+}
+
+// One launch (or, for the split stage, two and one per segment) over segments that all take the
 // same CTA variant.
 int eig_launch_group(const std::vector<const EigSegment*>& segs, const double* thr, int thr_per_patch,
                      cudaStream_t st, uint64_t* launches) {
@@ -1400,16 +2124,18 @@ int eig_launch_group(const std::vector<const EigSegment*>& segs, const double* t
   const int threads = big ? kT : kSmallT;
   if (split) {
     a.rz = 0;
-    const size_t sm1 = vec_bytes(nmax) +
-                       std::max(threads <= kSmallT ? part_bytes(nmax) : (size_t)0, wy_bytes(nmax, threads)) + 128;
-    if (threads == kSmallT)
-      k_eig<kSmallT, 2, 1><<<(unsigned)total, kSmallT, sm1, st>>>(a);
-    else
-      k_eig<kT, 1, 1><<<(unsigned)total, kT, sm1, st>>>(a);
+    for (int q = 0; q < a.nseg; ++q) {   // phase 1, per segment: the kernel follows its n
+      EigArgs one = a;
+      one.nseg = 1;
+      one.seg[0] = a.seg[q];
+      one.seg[0].first = 0;
+      tri_launch(one, threads == kT, st);
+      if (launches) *launches += 1;
+    }
     k_eig<kSmallT, kPairsMinB, 2><<<(unsigned)total, kSmallT, vec_bytes(nmax) + 128, st>>>(a);
     wy_apply_launch(a, nmax, total, st);
     MSLR_CUDA_TRY(cudaGetLastError());
-    if (launches) *launches += 3;
+    if (launches) *launches += 2;
     return MSLR_OK;
   }
   a.rz = stage_cols(nmax, threads);
