@@ -34,7 +34,7 @@
 // Zero patches give no eigenvalue above β² and Ṽ = 0, hence W = 0 (the
 // reference's zero-norm skip, src/recon.jl:185).
 //
-// Split stage (thresholded SVSTs with 33 <= n <= 384): three launches instead
+// Split stage (33 <= n <= 384): three launches (two for the values alone) instead
 // of one, so that each phase has the shape it needs — phase 1 and the WY
 // blocks' T factors (k_tri_reg: the matrix in registers, n <= 128; k_tri_big:
 // panels), phases 2–3 (four CTAs per SM, all patches resident at once), and
@@ -443,11 +443,9 @@ __device__ void wy_factors(cf* A, int n, const float* taur, const float* taui, c
   }
 }
 
-// MODE 0: the whole stage in one launch.  The split stage (three launches):
-// MODE 1 tridiagonalises and writes d, e to the side buffer and the WY
-// blocks' T factors to the Gram's upper triangle; MODE 2 computes the
-// eigenpairs of T from the side buffer (vectors into zv, FP32, [row][vector],
-// λ and h back to the side buffer); k_wy_apply then forms Ṽ.
+// MODE 0: the whole stage in one launch.  MODE 1: phase 1 of the split stage
+// (1024-thread variant) — d and e to the side buffer and the WY blocks' T
+// factors to the Gram's upper triangle.
 template <int MAXT, int MINB, int MODE>
 __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -495,17 +493,6 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
 
   const int i = tid;   // row owned by this thread (n <= kT)
   const int warp = tid >> 5, lane = tid & 31, nwarp = kT >> 5;
-  if constexpr (MODE == 2) {   // T from the side buffer (the same FP64 values phase 1 keeps)
-    const double* side = S.side + ip * 6 * (int64_t)n;
-    for (int q = tid; q < n; q += kT) {
-      dd[q] = side[q];
-      const double e = side[n + q];
-      ee[q] = e;
-      ee2[q] = e * e;
-    }
-    (void)nwarp;
-    __syncthreads();
-  } else {
   // ---- 1. tridiagonalisation with delayed rank-2 updates ---------------------
   for (int q = tid; q < npad; q += kT) {
     sv[q] = make_float2(0.f, 0.f);
@@ -758,7 +745,6 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
     wy_factors(A, n, taur, taui, sY, tid, kT);
     return;
   }
-  }   // phase 1 (MODE != 2)
 
   // ---- 2. eigenvalues above β² (FP64 multisection) ----------------------------
   if (tid == 0) {
@@ -890,15 +876,14 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
     }
   }
   __syncthreads();
-  if (MODE == 0 && S.nuc) {   // nuclear norm of the patch (src/recon.jl:138-146): Σ σ_i = Σ √λ_i
+  if (S.nuc) {   // nuclear norm of the patch (src/recon.jl:138-146): Σ σ_i = Σ √λ_i
     const double sq = (tid < r) ? sqrt(fmax(lam[tid], 0.0)) : 0.0;
     const double tot = block_sum_d(sq, redd);
     if (tid == 0) S.nuc[ip] = tot;
     return;
   }
-  if (r == 0) {   // (the split stage's back-transform writes the zero columns itself)
-    if (MODE == 0)
-      for (int64_t q = tid; q < (int64_t)n * n; q += kT) Z[q] = make_float2(0.f, 0.f);
+  if (r == 0) {
+    for (int64_t q = tid; q < (int64_t)n * n; q += kT) Z[q] = make_float2(0.f, 0.f);
     return;
   }
 
@@ -995,16 +980,6 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
       s0 = t;
     }
   }
-  if constexpr (MODE == 2) {   // the eigenvalues and √-weights for the back-transform
-    double* side = S.side + ip * 6 * (int64_t)n;
-    float* sh = reinterpret_cast<float*>(side + 4 * (int64_t)n);
-    for (int q = tid; q < r; q += kT) {
-      side[3 * n + q] = lam[q];
-      sh[q] = hv[q];
-    }
-    return;
-  }
-
   // ---- 4. V = H_0 ⋯ H_{n-2} Z, blocks of kNb reflectors from the last ---------
   // Staged vectors (few): every thread takes part — S = Yᴴ Z by (output, row
   // group) partial sums added in a fixed order, S ← T S, then Z −= Y S by
@@ -1827,6 +1802,299 @@ void tri_reg_launch(const EigArgs& a, unsigned grid, cudaStream_t st) {
   k_tri_reg<NT><<<grid, NT * NT * 32, sizeof(TriSmem<NT>), st>>>(a);
 }
 
+// ---- split stage, second launch: eigenpairs of T --------------------------------------
+// Phases 2–3 from d and e of the side buffer.
+//   Eigenvalues: multisection on FP64 Sturm counts of T scaled by a power of two
+// to norm at most 1.  The count is the number of sign changes of the leading
+// minors p_i = (d_i − x) p_{i−1} − e²_{i−1} p_{i−2} (Givens' sequence; computed
+// it is that of a T with a few relative roundings, as the quotient form is),
+// rescaled every eight steps: three FP64 operations a step and one of them on
+// the critical path, where the quotients p_i / p_{i−1} need a division each.
+// Couplings are kept at or above 1e-30 of the norm so that no two consecutive
+// minors vanish.  A group of g threads per eigenvalue counts below g points of
+// its bracket a round (two or three points a thread measured no faster).
+//   Vectors: twisted factorisation T − λ = L₊D₊L₊ᵀ = U₋D₋U₋ᵀ with the
+// multipliers l_j = e_j / D₊_j and m_j = e_{j−1} / D₋_j kept (two divisions a
+// row instead of four); γ_k = d_k − λ − e_{k−1} l_{k−1} − e_k m_{k+1}, z_k = 1 at
+// the smallest |γ_k|, z_j = −l_j z_{j+1} above it and −m_j z_{j−1} below.
+// Against the quotient form with FP32 first rounds: 486 full-rank sides of 300
+// 3.60 → 1.78 ms, one of 64 87 → 32 µs, 40 of 128 493 → 170 µs.
+
+// the reciprocal by two Newton steps from the hardware's approximation (|q| >= 1e-290)
+__device__ __forceinline__ double recip(double q) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(q));
+  y = fma(y, fma(-q, y, 1.0), y);
+  return fma(y, fma(-q, y, 1.0), y);
+}
+
+// eigenvalues below x: de[i] = (d_i, e²_{i−1}) of the scaled T
+__device__ __forceinline__ int sturm_count(const double2* de, int n, double x) {
+  double p0 = 1.0, p1 = de[0].x - x;
+  int cnt = (unsigned)__double2hiint(p1) >> 31;
+  auto step = [&](double2 t) {
+    const double p2 = fma(t.x - x, p1, -(t.y * p0));
+    cnt += (unsigned)(__double2hiint(p2) ^ __double2hiint(p1)) >> 31;
+    p0 = p1;
+    p1 = p2;
+  };
+  int i = 1;
+  for (; i + 8 <= n; i += 8) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) step(de[i + u]);
+    // the larger of the two back to [1, 2)
+    const int e0 = (__double2hiint(p0) >> 20) & 0x7ff, e1 = (__double2hiint(p1) >> 20) & 0x7ff;
+    const double sc = __hiloint2double((2046 - max(max(e0, e1), 1)) << 20, 0);
+    p0 *= sc;
+    p1 *= sc;
+  }
+  for (; i < n; ++i) step(de[i]);
+  return cnt;
+}
+
+// TH threads, n <= TH
+template <int TH>
+__global__ void __launch_bounds__(TH, kPairsMinB) k_pairs(EigArgs g) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  int s = 0;
+  while (s + 1 < g.nseg && (int64_t)blockIdx.x >= g.seg[s + 1].first) ++s;
+  const Seg& S = g.seg[s];
+  const int n = S.n;
+  const int64_t ip = (int64_t)blockIdx.x - S.first;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr int kThr = TH;
+  cf* Z = S.zv + ip * (int64_t)n * n;
+  double* AUX = S.aux + ip * (int64_t)n * n;
+  double* side = S.side + ip * 6 * (int64_t)n;
+  const bool full = S.lam_out != nullptr;
+  const double beta = full ? 0.0 : g.thr[g.thr_per_patch ? (int64_t)blockIdx.x : 0] * S.lam;
+
+  double2* de = reinterpret_cast<double2*>(smraw);   // scaled (d_i, e²_{i−1})
+  double* dd = reinterpret_cast<double*>(de + n);
+  double* ee = dd + n;
+  double* lam = ee + n;
+  double* redd = lam + n;                            // 64 doubles
+  float* hv = reinterpret_cast<float*>(redd + 64);
+  __shared__ int s_r;
+  for (int q = tid; q < n; q += kThr) {
+    dd[q] = side[q];
+    ee[q] = side[n + q];
+  }
+  __syncthreads();
+  // Gershgorin's interval
+  double gl = 1e300, gu = -1e300;
+  for (int q = tid; q < n; q += kThr) {
+    const double rr = (q > 0 ? fabs(ee[q - 1]) : 0.0) + (q < n - 1 ? fabs(ee[q]) : 0.0);
+    gl = fmin(gl, dd[q] - rr);
+    gu = fmax(gu, dd[q] + rr);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    gl = fmin(gl, __shfl_xor_sync(0xffffffffu, gl, o));
+    gu = fmax(gu, __shfl_xor_sync(0xffffffffu, gu, o));
+  }
+  if (lane == 0) {
+    redd[warp] = gl;
+    redd[32 + warp] = gu;
+  }
+  __syncthreads();
+  for (int w = 0; w < kThr / 32; ++w) {
+    gl = fmin(gl, redd[w]);
+    gu = fmax(gu, redd[32 + w]);
+  }
+  const double tnorm = fmax(fabs(gl), fabs(gu));
+  // power of two with norm · sc in [1/2, 1) (1 for a zero or non-finite T)
+  const int tex = (__double2hiint(tnorm) >> 20) & 0x7ff;
+  const bool sane = tex > 64 && tex < 1983;
+  const double sc = sane ? __hiloint2double((2045 - tex) << 20, 0) : 1.0;
+  const double isc = sane ? __hiloint2double((tex + 1) << 20, 0) : 1.0;
+  const double pad = 2.0 * 2.220446049250313e-16 * n;
+  gl = gl * sc - pad;
+  gu = gu * sc + pad;
+  for (int q = tid; q < n; q += kThr) {
+    const double e = q > 0 ? ee[q - 1] * sc : 0.0;
+    de[q] = make_double2(dd[q] * sc, fmax(e * e, 1e-60));
+  }
+  __syncthreads();
+  const double thr2 = beta * beta * sc;
+  if (tid == 0) {
+    s_r = full ? n : !(tnorm > 0.0) || thr2 >= gu ? 0 : n - sturm_count(de, n, thr2);
+    S.rank[ip] = s_r;
+  }
+  __syncthreads();
+  const int r = s_r;
+  {
+    if (!full) gl = fmax(gl, thr2);
+    int gsz = 1;
+    while (gsz < 32 && 2 * gsz * r <= kThr) gsz <<= 1;
+    const int e = tid / gsz, sl = tid & (gsz - 1);
+    if (warp * 32 < r * gsz) {   // whole warps, for the shuffles
+      const int kth = n - 1 - e;   // e-th largest = kth smallest
+      const double frac = (double)(sl + 1) / (double)(gsz + 1);
+      double lo = gl, hi = gu;
+      bool done = e >= r;
+      for (int it = 0; it < 200; ++it) {
+        // 4e-13 of the norm is well below what the vectors need (their error is |λ̂ − λ| / gap)
+        if (!done && !(hi - lo > 4e-13)) done = true;
+        if (!__any_sync(0xffffffffu, !done)) break;
+        const double x = lo + (hi - lo) * frac;
+        double nlo = lo, nhi = hi;
+        const int c = sturm_count(de, n, x);
+        if (x > lo && x < hi) {
+          if (c > kth) nhi = x;   // the eigenvalue is below x
+          else nlo = x;
+        }
+        for (int o = 1; o < gsz; o <<= 1) {
+          nlo = fmax(nlo, __shfl_xor_sync(0xffffffffu, nlo, o));
+          nhi = fmin(nhi, __shfl_xor_sync(0xffffffffu, nhi, o));
+        }
+        if (!done) {
+          if (!(nhi - nlo < hi - lo) || !(nlo < nhi)) {
+            done = true;
+          } else {
+            lo = nlo;
+            hi = nhi;
+          }
+        }
+      }
+      if (e < r && sl == 0) {
+        const double lm = 0.5 * (lo + hi) * isc;
+        lam[e] = lm;
+        const double sg = sqrt(fmax(lm, 0.0));
+        hv[e] = (sg > beta && sg > 0.0) ? (float)((sg - beta) / sg) : 0.f;
+      }
+    }
+  }
+  __syncthreads();
+  if (S.nuc) {   // nuclear norm of the patch (src/recon.jl:138-146): Σ σ_i = Σ √λ_i
+    const double sq = (tid < r) ? sqrt(fmax(lam[tid], 0.0)) : 0.0;
+    const double tot = block_sum_d(sq, redd);
+    if (tid == 0) S.nuc[ip] = tot;
+    return;
+  }
+  if (r == 0) return;   // the back-transform writes the zero columns itself
+
+  // eigenvectors of T: l in AUX, m in the vector's slots read as doubles
+  // ([row][vector], row stride n), replaced by z in place
+  const int64_t zs = n;
+  if (tid < r) {
+    const double lm = lam[tid];
+    const double pivmin = fmax(2.2250738585072014e-308 * fmax(tnorm * tnorm, 1.0), 1e-290);
+    double* zd = reinterpret_cast<double*>(Z) + tid;
+    double* dp = AUX + tid;
+    auto piv = [&](double q) { return fabs(q) < pivmin ? -pivmin : q; };
+    {   // both factorisations, one from either end
+      double qf = piv(dd[0] - lm), qb = piv(dd[n - 1] - lm);
+      for (int j = 0; j + 1 < n; ++j) {
+        const int jb = n - 1 - j;
+        const double ef = ee[j], eb = ee[jb - 1];
+        const double l = ef * recip(qf), m = eb * recip(qb);
+        dp[(int64_t)j * zs] = l;
+        zd[(int64_t)jb * zs] = m;
+        qf = piv(fma(-ef, l, dd[j + 1] - lm));
+        qb = piv(fma(-eb, m, dd[jb - 1] - lm));
+      }
+    }
+    int kb = 0;
+    double gb = 1e308;
+    {
+      double el = 0.0;   // e_{k−1} l_{k−1}
+#pragma unroll 4
+      for (int k = 0; k < n; ++k) {
+        const double em = k + 1 < n ? ee[k] * zd[(int64_t)(k + 1) * zs] : 0.0;
+        const double gm = fabs(dd[k] - lm - el - em);
+        if (gm <= gb) {
+          gb = gm;
+          kb = k;
+        }
+        if (k + 1 < n) el = ee[k] * dp[(int64_t)k * zs];
+      }
+    }
+    double nrm = 1.0;
+    {
+      double z = 1.0;
+#pragma unroll 8
+      for (int j = kb - 1; j >= 0; --j) {
+        z *= -dp[(int64_t)j * zs];
+        nrm = fma(z, z, nrm);
+      }
+      z = 1.0;
+#pragma unroll 8
+      for (int j = kb + 1; j < n; ++j) {
+        z *= -zd[(int64_t)j * zs];
+        nrm = fma(z, z, nrm);
+      }
+    }
+    const double inv = 1.0 / sqrt(nrm);
+    cf* zc = Z + tid;
+    double z = inv;
+    for (int j = kb + 1; j < n; j += 4) {   // (the slots that hold the multipliers first)
+      double mv[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) mv[q] = j + q < n ? zd[(int64_t)(j + q) * zs] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        z *= -mv[q];
+        if (j + q < n) zc[(int64_t)(j + q) * zs] = make_float2((float)z, 0.f);
+      }
+    }
+    zc[(int64_t)kb * zs] = make_float2((float)inv, 0.f);
+    z = inv;
+    for (int j = kb - 1; j >= 0; j -= 4) {
+      double lv[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) lv[q] = j - q >= 0 ? dp[(int64_t)(j - q) * zs] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        z *= -lv[q];
+        if (j - q >= 0) zc[(int64_t)(j - q) * zs] = make_float2((float)z, 0.f);
+      }
+    }
+  }
+  __syncthreads();
+  // Eigenvalues equal to working precision: Gram–Schmidt inside the cluster,
+  // cooperatively (every thread walks the same clusters).
+  {
+    const double ctol = 1e-12 * fmax(tnorm, 1e-300);
+    int s0 = 0, rb = 0;
+    while (s0 < r) {
+      int t = s0 + 1;
+      while (t < r && lam[t - 1] - lam[t] <= ctol) ++t;
+      for (int qv = s0 + 1; qv < t; ++qv) {
+        for (int attempt = 0; attempt < 4; ++attempt) {
+          for (int pv = s0; pv < qv; ++pv) {
+            double dot = 0.0;
+            for (int j = tid; j < n; j += kThr) dot += (double)Z[j * zs + pv].x * Z[j * zs + qv].x;
+            dot = block_sum_d(dot, redd + 32 * (rb++ & 1));
+            for (int j = tid; j < n; j += kThr) Z[j * zs + qv].x -= (float)dot * Z[j * zs + pv].x;
+            __syncthreads();
+          }
+          double nr = 0.0;
+          for (int j = tid; j < n; j += kThr) nr += (double)Z[j * zs + qv].x * Z[j * zs + qv].x;
+          nr = sqrt(block_sum_d(nr, redd + 32 * (rb++ & 1)));
+          if (nr > 0.1) {
+            for (int j = tid; j < n; j += kThr) Z[j * zs + qv].x /= (float)nr;
+            __syncthreads();
+            break;
+          }
+          // collapsed onto earlier vectors: restart from a unit vector
+          for (int j = tid; j < n; j += kThr)
+            Z[j * zs + qv].x = (j == (qv + attempt * 7919) % n) ? 1.f : 0.f;
+          __syncthreads();
+        }
+      }
+      s0 = t;
+    }
+  }
+  float* sh = reinterpret_cast<float*>(side + 4 * (int64_t)n);
+  for (int q = tid; q < r; q += kThr) {
+    side[3 * n + q] = lam[q];
+    sh[q] = hv[q];
+    if (full) S.lam_out[ip * n + q] = lam[q];
+  }
+}
+
+size_t pairs_smem(int n) { return (size_t)n * (2 + 3) * sizeof(double) + 64 * sizeof(double) + n * sizeof(float) + 16; }
+
 // ---- split stage, third launch: Ṽ = conj(Q Z) diag(√h) -------------------------
 // One CTA per (32 eigenvectors, patch); warp w holds rows w, w + 16, … of its
 // 32 vectors in registers (lane = vector) through all WY blocks, taken from
@@ -2004,11 +2272,12 @@ __global__ void __launch_bounds__(kWyThreads, 1) k_wy_apply(EigArgs g) {
     cpa_wait_all();
     __syncthreads();
   }
-  const float sh = (c < r) ? sqrtf(hw[c]) : 0.f;
+  // Ṽ, or V itself when every eigenpair is wanted
+  const float sh = S.lam_out ? 1.f : (c < r) ? sqrtf(hw[c]) : 0.f, sc = S.lam_out ? 1.f : -sh;
 #pragma unroll
   for (int q = 0; q < RPW; ++q) {
     const int row = w + 16 * q;
-    if (row < n && c < n) Z[(int64_t)row * n + c] = make_float2(zr[q] * sh, -zi[q] * sh);
+    if (row < n && c < n) Z[(int64_t)row * n + c] = make_float2(zr[q] * sh, zi[q] * sc);
   }
 }
 
@@ -2022,8 +2291,6 @@ int eig2_prepare(int nmax) {
   MSLR_CUDA_TRY(cudaFuncSetAttribute(k_eig<kT, 1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   MSLR_CUDA_TRY(cudaFuncSetAttribute(k_eig<kSmallT, 2, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, small));
   MSLR_CUDA_TRY(cudaFuncSetAttribute(k_eig<kT, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_eig<kSmallT, kPairsMinB, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(228 * 1024 / kPairsMinB - 1024)));
   MSLR_CUDA_TRY(cudaFuncSetAttribute(k_tri_reg<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TriSmem<3>)));
   MSLR_CUDA_TRY(cudaFuncSetAttribute(k_tri_reg<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TriSmem<4>)));
   MSLR_CUDA_TRY(cudaFuncSetAttribute(k_tri_big<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BigSmem)));
@@ -2041,8 +2308,7 @@ int eig2_prepare(int nmax) {
 
 namespace {
 
-// The split stage applies to thresholded SVSTs (not the values-only or
-// all-eigenpairs modes) with a side buffer and 33 <= n <= 384 (the
+// The split stage applies to stages with a side buffer and 33 <= n <= 384 (the
 // back-transform's register tile) whose T factors fit the upper triangle.
 // MSLR_EIG_SPLIT=0 keeps the one-launch stage everywhere (for comparisons).
 bool split_ok(const EigSegment& e) {
@@ -2050,7 +2316,7 @@ bool split_ok(const EigSegment& e) {
     const char* v = std::getenv("MSLR_EIG_SPLIT");
     return v && v[0] == '0';
   }();
-  if (off || !e.side || e.nuc || e.lam_out || e.n <= 32 || e.n > kSmallT) return false;
+  if (off || !e.side || e.n <= 32 || e.n > kSmallT) return false;
   const int64_t nblk = (e.n - 1 + kNb - 1) / kNb;
   return nblk * kNb * kNb <= (int64_t)e.n * (e.n - 1) / 2;
 }
@@ -2132,10 +2398,13 @@ int eig_launch_group(const std::vector<const EigSegment*>& segs, const double* t
       tri_launch(one, threads == kT, st);
       if (launches) *launches += 1;
     }
-    k_eig<kSmallT, kPairsMinB, 2><<<(unsigned)total, kSmallT, vec_bytes(nmax) + 128, st>>>(a);
-    wy_apply_launch(a, nmax, total, st);
+    // (486 patches of 300 are resident at once with 320 threads, and fewer threads have more registers)
+    if (nmax <= 320) k_pairs<320><<<(unsigned)total, 320, pairs_smem(nmax), st>>>(a);
+    else k_pairs<kSmallT><<<(unsigned)total, kSmallT, pairs_smem(nmax), st>>>(a);
+    const bool values = segs[0]->nuc != nullptr;   // (such calls have one segment)
+    if (!values) wy_apply_launch(a, nmax, total, st);
     MSLR_CUDA_TRY(cudaGetLastError());
-    if (launches) *launches += 2;
+    if (launches) *launches += values ? 1 : 2;
     return MSLR_OK;
   }
   a.rz = stage_cols(nmax, threads);

@@ -592,8 +592,8 @@ int patch_nucnorms(Ctx* c, int k, const cf* X, std::vector<double>& h, cudaStrea
   seg.rank = w.rank;
   seg.lam = 0.0;
   seg.nuc = c->d_nuc;
-  if ((rc = eig_launch_multi(1, &seg, c->d_zero, 0, st))) return rc;
-  c->launches += 1;
+  seg.side = w.vecs;
+  if ((rc = eig_launch_multi(1, &seg, c->d_zero, 0, st, &c->launches))) return rc;
   h.resize((size_t)g.Np);
   MSLR_CUDA_TRY(cudaMemcpyAsync(h.data(), c->d_nuc, (size_t)g.Np * sizeof(double), cudaMemcpyDeviceToHost, st));
   MSLR_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1017,7 +1017,9 @@ int svst_vjp_scale(Ctx* c, int s, const cf* z, const cf* xbar, double beta, cf* 
   seg.rank = v.rank;
   seg.lam = 0.0;
   seg.lam_out = v.lam;
-  if ((rc = eig_launch_multi(1, &seg, c->d_thr, 0, st))) return rc;
+  // 6n doubles per patch of the stage's scratch, in a product's buffer not yet in use
+  if (n >= 6) seg.side = reinterpret_cast<double*>(v.t1);
+  if ((rc = eig_launch_multi(1, &seg, c->d_thr, 0, st, &c->launches))) return rc;
   if ((rc = xgram_launch(ob, z, m, np, v.wbar, v.part, xsplit_of(np, n, g.L), st))) return rc;
   if ((rc = bgemm_launch(0, 0, v.wbar, v.V, v.t1, n, np, st))) return rc;         // W̄ V
   if ((rc = bgemm_launch(1, 0, v.V, v.t1, v.d, n, np, st))) return rc;            // D = Vᴴ W̄ V
@@ -1031,7 +1033,7 @@ int svst_vjp_scale(Ctx* c, int s, const cf* z, const cf* xbar, double beta, cf* 
     if ((rc = vjp_rebuild_launch(ob, z, v.wbar, v.d, m, np, c->d_pbuf, 0, st))) return rc;
     if ((rc = patch_sum_launch(c->d_pbuf, m, g.d_cover, zbar, st))) return rc;
   }
-  c->launches += 11;
+  c->launches += 10;
   std::vector<double> hb((size_t)np);
   MSLR_CUDA_TRY(cudaMemcpyAsync(hb.data(), v.bbar, np * sizeof(double), cudaMemcpyDeviceToHost, st));
   MSLR_CUDA_TRY(cudaStreamSynchronize(st));
