@@ -189,24 +189,6 @@ int stage_cols(int n, int threads) {
   return rz;
 }
 
-__device__ __forceinline__ unsigned long long pk2(float a, float b) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float2 upk2(unsigned long long u) {
-  float2 v;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(u));
-  return v;
-}
-// (a.x·b.x + c.x, a.y·b.y + c.y), each lane one correctly rounded FMA
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
-                                                   unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-
 // Eight columns of a tile row: the pending rank-2 update of element
 // (row, jb + b), its contribution to the row sum y_row and to the column
 // partials (cr, ci), written back.
@@ -1108,9 +1090,9 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
 }
 
 // ---- tridiagonalisation with the matrix in registers (n <= 128) -------------------
-// Phase 1 for Gram sides up to 32·NT: NT × NT warps hold the whole Hermitian
-// matrix, one 32 × 32 tile per warp, lane (rg, cg) rows rg + 8t and columns
-// cg + 4u of it (32 values).  A step is what k_eig's is — the previous
+// Phase 1 for Gram sides up to 32·NT: the warps hold the whole Hermitian
+// matrix, one tile of 32 rows × 4·CU columns per warp, lane (rg, cg) rows rg +
+// 8t and columns cg + 4u of it.  A step is what k_eig's is — the previous
 // rank-2 update applied on the fly while y = A v is formed — but nothing but
 // vectors moves: the tile pass is six packed FMAs per value on registers with
 // the column's (v, w) from shared memory, and both triangles are stored, so a
@@ -1121,38 +1103,59 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
 // uᴴ A u after it (so no third one reduces vᴴ y).
 // With the matrix in L2 a step cost 5.6 µs whatever n was (n = 64, one
 // patch: 351 µs), the latency of its round trips and four barriers.
-// Tile of warp w: row w / NT, column (w + w / NT) mod NT, so that the tiles
-// left in play when the leading ones are done stay spread over the SM's four
-// schedulers.
+// A warp's tile column is rotated by its tile row, so that the tiles left in
+// play when the leading ones are done stay spread over the SM's schedulers.
+// CU columns per lane: tiles of 32 rows × 4·CU columns, one per warp.  Eight is
+// what 16 warps' registers hold at NT = 4; with four the smaller sides have
+// twice the warps, so the latencies of a tile pass overlap.
+constexpr int tri_cu(int nt) { return nt == 4 ? 8 : 4; }
 template <int NT>
 struct TriVec {
-  static constexpr int NP = 32 * NT, LD = NP + 1;
+  static constexpr int NP = 32 * NT, LD = NP + 1, CU = tri_cu(NT), TC = 4 * CU, NTC = NP / TC;
+  static constexpr int kThreads = NT * NTC * 32;
   float4 dw[NP], dv[NP];  // the pending update of column j: (wp.x, wp.x, wp.y, wp.y), (vp.x, vp.x, vp.y, vp.y)
   float4 sx[NP];          // this step's column x below the subdiagonal: (x.x, x.y, x.y, x.x)
   cf scol[NP];            // next column, before the pending update
-  cf part[NT][NP];        // per tile column: partial sums of A u
-  float red0[4], redt[16];
+  cf part[NTC][NP];       // per tile column: partial sums of A u
+  float red0[4], redt[NT * NTC];
   cf x1;
 };
 
+// zlarfg with α = (ar, ai) and ‖x‖² = xn: β, τ, u₁ = α − β and 1 / u₁.  The root
+// and its reciprocal from one approximation, each refined to the last bit by
+// a Newton step (shorter than a root followed by a division by it).
+__device__ __forceinline__ void reflector(float ar, float ai, float xn, float* bt, cf* tau, cf* u1, cf* scal) {
+  const float s = ar * ar + ai * ai + xn;
+  float r = rsqrtf(s);
+  r = fmaf(0.5f * r, fmaf(-s * r, r, 1.f), r);
+  float q = s * r;
+  q = fmaf(0.5f * r, fmaf(-q, q, s), q);
+  const float b = -copysignf(q, ar), ib = -copysignf(r, ar);
+  *bt = b;
+  *tau = make_float2((b - ar) * ib, -ai * ib);
+  *u1 = make_float2(ar - b, ai);
+  const float id = __frcp_rn(u1->x * u1->x + ai * ai);
+  *scal = make_float2(u1->x * id, -ai * id);
+}
+
 // The n steps of the n × n Hermitian matrix at A (column stride ld, n <= 32·NT,
 // lower triangle read): d, e and τ; reflectors below A's subdiagonal and, when
-// given, in Y (unit entry and zeros included).  NT·NT warps.
+// given, in Y (unit entry and zeros included).  TriVec<NT>::kThreads threads.
 template <int NT>
 __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, double* dd, double* ee, cf* taus,
                                           cf* Y) {
-  constexpr int NP = 32 * NT, LD = TriVec<NT>::LD;
+  constexpr int NP = 32 * NT, LD = TriVec<NT>::LD, CU = TriVec<NT>::CU, TC = TriVec<NT>::TC, NTC = TriVec<NT>::NTC;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int I = warp / NT, J = (warp + I) % NT;
+  const int I = warp / NTC, J = (warp + I) % NTC;
   const int rg = lane >> 2, cg = lane & 3;
 
   // the tile, from the lower triangle
-  cf a[4][8];
+  cf a[4][CU];
 #pragma unroll
   for (int t = 0; t < 4; ++t)
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int r = I * 32 + rg + 8 * t, c = J * 32 + cg + 4 * u;
+    for (int u = 0; u < CU; ++u) {
+      const int r = I * 32 + rg + 8 * t, c = J * TC + cg + 4 * u;
       cf v = make_float2(0.f, 0.f);
       if (r < n && c < n) {
         v = r >= c ? __ldcg(A + (int64_t)c * ld + r) : __ldcg(A + (int64_t)r * ld + c);
@@ -1191,17 +1194,12 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
     cf tau = make_float2(0.f, 0.f), scal = make_float2(1.f, 0.f), u1 = scal;
     const bool refl = !(xn == 0.f && ai == 0.f);
     if (refl) {
-      bt = -copysignf(sqrtf(ar * ar + ai * ai + xn), ar);
-      const float ib = 1.f / bt;
-      tau = make_float2((bt - ar) * ib, -ai * ib);
-      u1 = make_float2(ar - bt, ai);
-      const float id = 1.f / (u1.x * u1.x + ai * ai);
-      scal = make_float2(u1.x * id, -ai * id);
+      reflector(ar, ai, xn, &bt, &tau, &u1, &scal);
     }
     // A ← A − (vp wpᴴ + wp vpᴴ), A u on the tiles still in play
     float tq = 0.f;
-    if (I * 32 + 31 > k && J * 32 + 31 > k) {
-      const int c0 = J * 32 + cg;
+    if (I * 32 + 31 > k && J * TC + TC - 1 > k) {
+      const int c0 = J * TC + cg;
       {
         cf r1[4], r2[4], r3[4], r4[4];   // −(vp), −(vp rotated), −(wp), −(wp rotated) of the rows
 #pragma unroll
@@ -1213,7 +1211,7 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
           r4[t] = make_float2(-w.z, w.x);
         }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {   // a −= vp conj(wp_j) + wp conj(vp_j)
+        for (int u = 0; u < CU; ++u) {   // a −= vp conj(wp_j) + wp conj(vp_j)
           const float4 w = m.dw[c0 + 4 * u], v = m.dv[c0 + 4 * u];
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
@@ -1231,7 +1229,7 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
 #pragma unroll
         for (int t = 0; t < 4; ++t) P[t] = Q[t] = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = 0; u < CU; ++u) {
           const float4 v = m.sx[c0 + 4 * u];
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
@@ -1242,13 +1240,13 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
 #pragma unroll
         for (int t = 0; t < 4; ++t) y[t] = make_float2(P[t].x - P[t].y, Q[t].x + Q[t].y);
       }
-      if (J == (k + 1) >> 5) {   // column k + 1: entry u1 of u, and the next step's column
-        const int us = ((k + 1) & 31) >> 2;
+      if (J == (k + 1) / TC) {   // column k + 1: entry u1 of u, and the next step's column
+        const int us = ((k + 1) % TC) >> 2;
         cf nx[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) nx[t] = a[t][0];
 #pragma unroll
-        for (int u = 1; u < 8; ++u)
+        for (int u = 1; u < CU; ++u)
           if (u == us) {
 #pragma unroll
             for (int t = 0; t < 4; ++t) nx[t] = a[t][u];
@@ -1283,16 +1281,16 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
     if (own) {
       // y = A v of this row and of row k + 1 (the next pivot row), in tile order
       cf y = make_float2(0.f, 0.f), y1 = y;
-      const int q0 = (k + 1) >> 5;
+      const int q0 = (k + 1) / TC;
 #pragma unroll
-      for (int q = 0; q < NT; ++q)
+      for (int q = 0; q < NTC; ++q)
         if (q >= q0) {
           y = cadd(y, m.part[q][i]);
           y1 = cadd(y1, m.part[q][k + 1]);
         }
       float t = 0.f;
 #pragma unroll
-      for (int q = 0; q < NT * NT; ++q) t += m.redt[q];
+      for (int q = 0; q < NT * NTC; ++q) t += m.redt[q];
       const float c = 0.5f * (tau.x * tau.x + tau.y * tau.y) * (scal.x * scal.x + scal.y * scal.y) * t;
       const cf vi = i == k + 1 ? make_float2(1.f, 0.f) : cmul(x, scal);   // 0 for i <= k and i >= n
       if (i == k + 1) {
@@ -1364,7 +1362,7 @@ struct TriSmem {
 };
 
 template <int NT>
-__global__ void __launch_bounds__(NT * NT * 32, NT == 4 ? 1 : NT == 3 ? 2 : NT == 2 ? 4 : 8) k_tri_reg(EigArgs g) {
+__global__ void __launch_bounds__(TriVec<NT>::kThreads, NT == 2 ? 2 : 1) k_tri_reg(EigArgs g) {
   extern __shared__ __align__(16) unsigned char smraw[];
   TriSmem<NT>& m = *reinterpret_cast<TriSmem<NT>*>(smraw);
   int s = 0;
@@ -1372,7 +1370,7 @@ __global__ void __launch_bounds__(NT * NT * 32, NT == 4 ? 1 : NT == 3 ? 2 : NT =
   const Seg& S = g.seg[s];
   const int n = S.n;
   const int64_t ip = (int64_t)blockIdx.x - S.first;
-  constexpr int kThreads = NT * NT * 32, LD = TriVec<NT>::LD;
+  constexpr int kThreads = TriVec<NT>::kThreads, LD = TriVec<NT>::LD;
   const int tid = threadIdx.x, warp = tid >> 5;
   cf* A = S.gram + ip * (int64_t)n * n;
   tri_steps<NT>(A, n, n, m.v, m.dd, m.ee, m.tau, m.Y);
@@ -1548,12 +1546,7 @@ __global__ void __launch_bounds__(kBigT, 1) k_tri_big(EigArgs g) {
       cf tau = make_float2(0.f, 0.f), scal = make_float2(1.f, 0.f), u1 = scal;
       const bool refl = !(xn == 0.f && ai == 0.f);
       if (refl) {
-        bt = -copysignf(sqrtf(ar * ar + ai * ai + xn), ar);
-        const float ib = 1.f / bt;
-        tau = make_float2((bt - ar) * ib, -ai * ib);
-        u1 = make_float2(ar - bt, ai);
-        const float id = 1.f / (u1.x * u1.x + ai * ai);
-        scal = make_float2(u1.x * id, -ai * id);
+        reflector(ar, ai, xn, &bt, &tau, &u1, &scal);
       }
       const int o = k + 1;
       if (i == o) m.p.sx[o] = make_float4(u1.x, u1.y, u1.y, u1.x);
@@ -1799,7 +1792,7 @@ __global__ void __launch_bounds__(kBigT, 1) k_tri_big(EigArgs g) {
 
 template <int NT>
 void tri_reg_launch(const EigArgs& a, unsigned grid, cudaStream_t st) {
-  k_tri_reg<NT><<<grid, NT * NT * 32, sizeof(TriSmem<NT>), st>>>(a);
+  k_tri_reg<NT><<<grid, TriVec<NT>::kThreads, sizeof(TriSmem<NT>), st>>>(a);
 }
 
 // ---- split stage, second launch: eigenpairs of T --------------------------------------
@@ -2096,22 +2089,28 @@ __global__ void __launch_bounds__(TH, kPairsMinB) k_pairs(EigArgs g) {
 size_t pairs_smem(int n) { return (size_t)n * (2 + 3) * sizeof(double) + 64 * sizeof(double) + n * sizeof(float) + 16; }
 
 // ---- split stage, third launch: Ṽ = conj(Q Z) diag(√h) -------------------------
-// One CTA per (32 eigenvectors, patch); warp w holds rows w, w + 16, … of its
-// 32 vectors in registers (lane = vector) through all WY blocks, taken from
-// the last reflector down.  Each block's Y (rows k0+1 … n−1, kYS-strided so a
-// row's 16 reflector entries load as warp-wide broadcasts) and T arrive by
-// cp.async into one of two buffers while the previous block is applied:
-// S = Yᴴ Z by per-warp partial sums added in warp order, S ← T S, then
-// Z −= Y S.  The complex products run as packed FP32x2 FMAs on lane-wise
-// products, (y.re·z.re, y.im·z.im) and (y.re·z.im, y.im·z.re), combined once
-// per row or per reflector.  Columns at or beyond the patch's rank are
-// written as zeros.
+// One CTA per 64 eigenvectors of a patch (32 when no more are left, or above
+// side 320); warp w holds rows w, w + 16, … of its vectors in registers (lane
+// = vectors lane and lane + 32) through all WY blocks, taken from the last
+// reflector down.  Each block's Y (rows k0+1 … n−1, kYS-strided so a row's 16
+// reflector entries load as warp-wide broadcasts) and T arrive by cp.async
+// into one of two buffers while the previous block is applied: S = Yᴴ Z by
+// per-warp partial sums added in warp order, eight reflectors at a time, S ← T
+// S, then Z −= Y S.  The complex products run as packed FP32x2 FMAs on
+// lane-wise products, (y.re·z.re, y.im·z.im) and (y.re·z.im, y.im·z.re),
+// combined once per row or per reflector.  A 16-byte broadcast of Y takes the
+// shared-memory pipe four cycles whatever it feeds: with one vector per lane
+// (four FMAs) the kernel waited for it at twice the FMAs' time, two vectors
+// balance the two (486 full-rank patches of side 300: 5.3 → 4.5 ms).
+// Columns at or beyond the patch's rank are written as zeros.
 constexpr int kYS = 18;        // row stride of the staged Y (16-byte aligned rows)
 constexpr int kWyThreads = 512;
-constexpr int kWyCols = 32;
+constexpr int kWyCols = 64;
+constexpr int kWyWarps = kWyThreads / 32;
 
 size_t wy_apply_smem(int nmax) {
-  return ((size_t)2 * nmax * kYS + 16 * kNb * kWyCols + 2 * kNb * kWyCols + 2 * kNb * kNb) * sizeof(cf);
+  const int rows = (nmax + 63) / 64 * 64;   // 16 · rows per warp
+  return ((size_t)2 * rows * kYS + kWyWarps * 8 * kWyCols + 2 * kNb * kWyCols + 2 * kNb * kNb) * sizeof(cf);
 }
 
 __device__ __forceinline__ void cpa8(void* dst, const void* src) {
@@ -2143,42 +2142,32 @@ __device__ __forceinline__ void wy_stage(const cf* A, int n, int kend, cf* ys, c
   cpa_commit();
 }
 
-template <int RPW>
-__global__ void __launch_bounds__(kWyThreads, 1) k_wy_apply(EigArgs g) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  int s = 0;
-  while (s + 1 < g.nseg && (int64_t)blockIdx.y >= g.seg[s + 1].first) ++s;
-  const Seg& S = g.seg[s];
-  const int n = S.n;
-  const int64_t ip = (int64_t)blockIdx.y - S.first;
-  const int cb = blockIdx.x * kWyCols;
-  if (cb >= n) return;   // the grid covers the launch's largest n
+// NV vectors per lane: columns cb + lane + 32 v of the patch's n × n matrix Z
+template <int RPW, int NV>
+__device__ __forceinline__ void wy_apply_body(const Seg& S, const cf* A, cf* Z, const float* hw, int n, int r, int cb,
+                                              cf* smem) {
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-  const cf* A = S.gram + ip * (int64_t)n * n;
-  cf* Z = S.zv + ip * (int64_t)n * n;
-  const int r = S.rank[ip];
-  const int c = cb + lane;
-  if (cb >= r) {
-    if (c < n)
-      for (int row = w; row < n; row += kWyThreads / 32) Z[(int64_t)row * n + c] = make_float2(0.f, 0.f);
-    return;
-  }
-  const double* side = S.side + ip * 6 * (int64_t)n;
-  const float* hw = reinterpret_cast<const float*>(side + 4 * (int64_t)n);
-  cf* Ybuf = reinterpret_cast<cf*>(smraw);    // two buffers of n × kYS
-  const int ystride = n * kYS;
-  cf* part = Ybuf + 2 * ystride;              // 16 warps × kNb × 32
-  cf* Ss = part + 16 * kNb * kWyCols;         // kNb × 32
-  cf* S2 = Ss + kNb * kWyCols;                // kNb × 32
-  cf* Tbuf = S2 + kNb * kWyCols;              // two buffers of kNb × kNb
-  float zr[RPW], zi[RPW];
+  // two buffers of Y, zero in the rows no block has reached yet (they are taken
+  // from the last reflector down) and beyond n, so that rows go untested in fours
+  cf* Ybuf = smem;
+  constexpr int ystride = 16 * RPW * kYS;
+  cf* part = Ybuf + 2 * ystride;                 // 16 warps × 8 × 64
+  cf* Ss = part + kWyWarps * 8 * kWyCols;        // kNb × 64
+  cf* S2 = Ss + kNb * kWyCols;                   // kNb × 64
+  cf* Tbuf = S2 + kNb * kWyCols;                 // two buffers of kNb × kNb
+  cf z[RPW][NV];
 #pragma unroll
   for (int q = 0; q < RPW; ++q) {
     const int row = w + 16 * q;
-    zr[q] = (c < r && row < n) ? __ldcg(&Z[(int64_t)row * n + c].x) : 0.f;
-    zi[q] = 0.f;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const int c = cb + lane + 32 * v;
+      z[q][v] = make_float2((c < r && row < n) ? __ldcg(&Z[(int64_t)row * n + c].x) : 0.f, 0.f);
+    }
   }
   const int nref = n - 1;
+  for (int q = tid; q < ystride; q += kWyThreads) reinterpret_cast<float4*>(Ybuf)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncthreads();
   if (nref > 0) wy_stage(A, n, nref, Ybuf, Tbuf, tid);
   cpa_wait_all();
   __syncthreads();
@@ -2189,83 +2178,102 @@ __global__ void __launch_bounds__(kWyThreads, 1) k_wy_apply(EigArgs g) {
     const cf* Ts = Tbuf + buf * kNb * kNb;
     if (kend - kNb > 0)   // the next block, into the other buffers
       wy_stage(A, n, kend - kNb, Ybuf + (buf ^ 1) * ystride, Tbuf + (buf ^ 1) * kNb * kNb, tid);
-    // partial S = Yᴴ Z over this warp's rows, eight reflectors per pass
-#pragma unroll
+#pragma unroll 1
     for (int h = 0; h < 2; ++h) {
-      unsigned long long P[8], Q[8];
+      // partial S = Yᴴ Z over this warp's rows, reflectors 8h … 8h + 7 in passes of four
 #pragma unroll
-      for (int a = 0; a < 8; ++a) P[a] = Q[a] = 0ull;
+      for (int a4 = 0; a4 < 2; ++a4) {
+        cf P[4][NV], Q[4][NV];
 #pragma unroll
-      for (int q = 0; q < RPW; ++q) {
-        const int row = w + 16 * q;
-        if (row > k0 && row < n) {
-          const unsigned long long z1 = pk2(zr[q], zi[q]), z2 = pk2(zi[q], zr[q]);
-          const float4* yr = reinterpret_cast<const float4*>(Ys + row * kYS) + 4 * h;
+        for (int a = 0; a < 4; ++a)
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            const float4 y = yr[t];
-            const unsigned long long y0 = pk2(y.x, y.y), y1 = pk2(y.z, y.w);
-            P[2 * t] = fma2(y0, z1, P[2 * t]);
-            Q[2 * t] = fma2(y0, z2, Q[2 * t]);
-            P[2 * t + 1] = fma2(y1, z1, P[2 * t + 1]);
-            Q[2 * t + 1] = fma2(y1, z2, Q[2 * t + 1]);
+          for (int v = 0; v < NV; ++v) P[a][v] = Q[a][v] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int q4 = 0; q4 < RPW; q4 += 4) {
+          if (w + 16 * (q4 + 3) <= k0) continue;
+#pragma unroll
+          for (int q = q4; q < q4 + 4; ++q) {
+            const int row = w + 16 * q;
+            const float4* yr = reinterpret_cast<const float4*>(Ys + row * kYS) + 4 * h + 2 * a4;
+            const float4 y01 = yr[0], y23 = yr[1];
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+              const cf z1 = z[q][v], z2 = make_float2(z1.y, z1.x);
+              P[0][v] = __ffma2_rn(make_float2(y01.x, y01.y), z1, P[0][v]);
+              Q[0][v] = __ffma2_rn(make_float2(y01.x, y01.y), z2, Q[0][v]);
+              P[1][v] = __ffma2_rn(make_float2(y01.z, y01.w), z1, P[1][v]);
+              Q[1][v] = __ffma2_rn(make_float2(y01.z, y01.w), z2, Q[1][v]);
+              P[2][v] = __ffma2_rn(make_float2(y23.x, y23.y), z1, P[2][v]);
+              Q[2][v] = __ffma2_rn(make_float2(y23.x, y23.y), z2, Q[2][v]);
+              P[3][v] = __ffma2_rn(make_float2(y23.z, y23.w), z1, P[3][v]);
+              Q[3][v] = __ffma2_rn(make_float2(y23.z, y23.w), z2, Q[3][v]);
+            }
           }
         }
-      }
+        // conj(y)·z = (Σ y.re z.re + y.im z.im, Σ y.re z.im − y.im z.re)
 #pragma unroll
-      for (int a = 0; a < 8; ++a) {   // conj(y)·z = (Σ y.re z.re + y.im z.im, Σ y.re z.im − y.im z.re)
-        const float2 p = upk2(P[a]), qq = upk2(Q[a]);
-        part[(w * kNb + 8 * h + a) * kWyCols + lane] = make_float2(p.x + p.y, qq.x - qq.y);
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int v = 0; v < NV; ++v)
+            part[(w * 8 + 4 * a4 + a) * kWyCols + 32 * v + lane] =
+                make_float2(P[a][v].x + P[a][v].y, Q[a][v].x - Q[a][v].y);
       }
+      __syncthreads();
+      if (NV == 2 || w < 8) {   // one sum per thread: reflector 8h + a, vector c
+        const int a = NV == 2 ? w >> 1 : w, c = NV == 2 ? 32 * (w & 1) + lane : lane;
+        cf sum = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int w2 = 0; w2 < kWyWarps; ++w2) sum = cadd(sum, part[(w2 * 8 + a) * kWyCols + c]);
+        Ss[(8 * h + a) * kWyCols + c] = sum;
+      }
+      __syncthreads();
     }
-    __syncthreads();
     {
-      const int a = tid >> 5;   // kWyThreads / 32 = kNb rows of S
-      float sr = 0.f, si = 0.f;
+      const int a = w;
+      cf acc[NV];
 #pragma unroll
-      for (int w2 = 0; w2 < kWyThreads / 32; ++w2) {
-        const cf v = part[(w2 * kNb + a) * kWyCols + lane];
-        sr += v.x;
-        si += v.y;
-      }
-      Ss[a * kWyCols + lane] = make_float2(sr, si);
-    }
-    __syncthreads();
-    {
-      const int a = tid >> 5;
-      cf acc = make_float2(0.f, 0.f);
-      for (int b = a; b < kNb; ++b) acc = cadd(acc, cmul(Ts[a * kNb + b], Ss[b * kWyCols + lane]));
-      S2[a * kWyCols + lane] = acc;
-    }
-    __syncthreads();
-    // Z −= Y (T S) on this warp's rows, eight reflectors per pass
+      for (int v = 0; v < NV; ++v) acc[v] = make_float2(0.f, 0.f);
+      for (int b = a; b < kNb; ++b) {
+        const cf t = Ts[a * kNb + b];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      unsigned long long sa[8], sb[8];
-#pragma unroll
-      for (int a = 0; a < 8; ++a) {
-        const cf v = S2[(8 * h + a) * kWyCols + lane];
-        sa[a] = pk2(v.x, v.y);
-        sb[a] = pk2(v.y, v.x);
+        for (int v = 0; v < NV; ++v) acc[v] = cadd(acc[v], cmul(t, Ss[b * kWyCols + 32 * v + lane]));
       }
 #pragma unroll
-      for (int q = 0; q < RPW; ++q) {
-        const int row = w + 16 * q;
-        if (row > k0 && row < n) {
-          const float4* yr = reinterpret_cast<const float4*>(Ys + row * kYS) + 4 * h;
-          unsigned long long U = 0ull, V = 0ull;
+      for (int v = 0; v < NV; ++v) S2[a * kWyCols + 32 * v + lane] = acc[v];
+    }
+    __syncthreads();
+    // Z −= Y (T S) on this warp's rows, four reflectors per pass
+#pragma unroll 1
+    for (int a4 = 0; a4 < 4; ++a4) {
+      cf sa[4][NV], sb[4][NV];
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            const float4 y = yr[t];
-            const unsigned long long y0 = pk2(y.x, y.y), y1 = pk2(y.z, y.w);
-            U = fma2(y0, sa[2 * t], U);
-            V = fma2(y0, sb[2 * t], V);
-            U = fma2(y1, sa[2 * t + 1], U);
-            V = fma2(y1, sb[2 * t + 1], V);
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          sa[a][v] = S2[(4 * a4 + a) * kWyCols + 32 * v + lane];
+          sb[a][v] = make_float2(sa[a][v].y, sa[a][v].x);
+        }
+#pragma unroll
+      for (int q4 = 0; q4 < RPW; q4 += 4) {
+        if (w + 16 * (q4 + 3) <= k0) continue;
+#pragma unroll
+        for (int q = q4; q < q4 + 4; ++q) {
+          const int row = w + 16 * q;
+          const float4* yr = reinterpret_cast<const float4*>(Ys + row * kYS) + 2 * a4;
+          const float4 y01 = yr[0], y23 = yr[1];
+#pragma unroll
+          for (int v = 0; v < NV; ++v) {
+            cf U = __fmul2_rn(make_float2(y01.x, y01.y), sa[0][v]), V = __fmul2_rn(make_float2(y01.x, y01.y), sb[0][v]);
+            U = __ffma2_rn(make_float2(y01.z, y01.w), sa[1][v], U);
+            V = __ffma2_rn(make_float2(y01.z, y01.w), sb[1][v], V);
+            U = __ffma2_rn(make_float2(y23.x, y23.y), sa[2][v], U);
+            V = __ffma2_rn(make_float2(y23.x, y23.y), sb[2][v], V);
+            U = __ffma2_rn(make_float2(y23.z, y23.w), sa[3][v], U);
+            V = __ffma2_rn(make_float2(y23.z, y23.w), sb[3][v], V);
+            // y·s = (Σ y.re s.re − y.im s.im, Σ y.re s.im + y.im s.re)
+            z[q][v].x -= U.x - U.y;
+            z[q][v].y -= V.x + V.y;
           }
-          const float2 u = upk2(U), v = upk2(V);   // y·s = (Σ y.re s.re − y.im s.im, Σ y.re s.im + y.im s.re)
-          zr[q] -= u.x - u.y;
-          zi[q] -= v.x + v.y;
         }
       }
     }
@@ -2273,12 +2281,51 @@ __global__ void __launch_bounds__(kWyThreads, 1) k_wy_apply(EigArgs g) {
     __syncthreads();
   }
   // Ṽ, or V itself when every eigenpair is wanted
-  const float sh = S.lam_out ? 1.f : (c < r) ? sqrtf(hw[c]) : 0.f, sc = S.lam_out ? 1.f : -sh;
 #pragma unroll
-  for (int q = 0; q < RPW; ++q) {
-    const int row = w + 16 * q;
-    if (row < n && c < n) Z[(int64_t)row * n + c] = make_float2(zr[q] * sh, zi[q] * sc);
+  for (int v = 0; v < NV; ++v) {
+    const int c = cb + lane + 32 * v;
+    const float sh = S.lam_out ? 1.f : (c < r) ? sqrtf(hw[c]) : 0.f, sc = S.lam_out ? 1.f : -sh;
+#pragma unroll
+    for (int q = 0; q < RPW; ++q) {
+      const int row = w + 16 * q;
+      if (row < n && c < n) Z[(int64_t)row * n + c] = make_float2(z[q][v].x * sh, z[q][v].y * sc);
+    }
   }
+}
+
+// blockIdx.x: group of 32·NV columns
+template <int RPW, int NV>
+__global__ void __launch_bounds__(kWyThreads, 1) k_wy_apply(EigArgs g) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  int s = 0;
+  while (s + 1 < g.nseg && (int64_t)blockIdx.y >= g.seg[s + 1].first) ++s;
+  const Seg& S = g.seg[s];
+  const int n = S.n;
+  const int64_t ip = (int64_t)blockIdx.y - S.first;
+  const int cb = blockIdx.x * 32 * NV;
+  if (cb >= n) return;   // the grid covers the launch's largest n
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const cf* A = S.gram + ip * (int64_t)n * n;
+  cf* Z = S.zv + ip * (int64_t)n * n;
+  const int r = S.rank[ip];
+  const float* hw = reinterpret_cast<const float*>(S.side + ip * 6 * (int64_t)n + 4 * (int64_t)n);
+  cf* smem = reinterpret_cast<cf*>(smraw);
+  // columns from the next group of 32 on that have no vector
+  const int z0 = max(cb, (r + 31) / 32 * 32);
+  for (int c = z0 + lane; c < min(n, cb + 32 * NV); c += 32)
+    for (int row = w; row < n; row += kWyWarps) Z[(int64_t)row * n + c] = make_float2(0.f, 0.f);
+  if (cb >= r) return;
+  if (NV == 2 && r - cb > 32) wy_apply_body<RPW, NV>(S, A, Z, hw, n, r, cb, smem);
+  else wy_apply_body<RPW, 1>(S, A, Z, hw, n, r, cb, smem);
+}
+
+const void* wy_kernel(int rows_per_warp) {
+  return rows_per_warp <= 4    ? reinterpret_cast<const void*>(&k_wy_apply<4, 2>)
+         : rows_per_warp <= 8  ? reinterpret_cast<const void*>(&k_wy_apply<8, 2>)
+         : rows_per_warp <= 12 ? reinterpret_cast<const void*>(&k_wy_apply<12, 2>)
+         : rows_per_warp <= 16 ? reinterpret_cast<const void*>(&k_wy_apply<16, 2>)
+         : rows_per_warp <= 20 ? reinterpret_cast<const void*>(&k_wy_apply<20, 2>)
+                               : reinterpret_cast<const void*>(&k_wy_apply<24, 1>);
 }
 
 }  // namespace
@@ -2297,12 +2344,8 @@ int eig2_prepare(int nmax) {
   MSLR_CUDA_TRY(cudaFuncSetAttribute(k_tri_big<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BigSmem)));
   static_assert(sizeof(BigSmem) <= 227 * 1024, "shared memory of the blocked tridiagonalisation");
   const int wy = (int)wy_apply_smem(kSmallT);
-  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_wy_apply<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, wy));
-  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_wy_apply<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, wy));
-  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_wy_apply<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, wy));
-  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_wy_apply<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, wy));
-  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_wy_apply<20>, cudaFuncAttributeMaxDynamicSharedMemorySize, wy));
-  MSLR_CUDA_TRY(cudaFuncSetAttribute(k_wy_apply<24>, cudaFuncAttributeMaxDynamicSharedMemorySize, wy));
+  for (const void* k : {wy_kernel(4), wy_kernel(8), wy_kernel(12), wy_kernel(16), wy_kernel(20), wy_kernel(24)})
+    MSLR_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, wy));
   return MSLR_OK;
 }
 
@@ -2322,15 +2365,11 @@ bool split_ok(const EigSegment& e) {
 }
 
 int wy_apply_launch(const EigArgs& a, int nmax, int64_t total, cudaStream_t st) {
-  const dim3 grid((unsigned)((nmax + kWyCols - 1) / kWyCols), (unsigned)total);
-  const size_t sm = wy_apply_smem(nmax);
-  const int rpw = (nmax + 15) / 16;
-  if (rpw <= 4) k_wy_apply<4><<<grid, kWyThreads, sm, st>>>(a);
-  else if (rpw <= 8) k_wy_apply<8><<<grid, kWyThreads, sm, st>>>(a);
-  else if (rpw <= 12) k_wy_apply<12><<<grid, kWyThreads, sm, st>>>(a);
-  else if (rpw <= 16) k_wy_apply<16><<<grid, kWyThreads, sm, st>>>(a);
-  else if (rpw <= 20) k_wy_apply<20><<<grid, kWyThreads, sm, st>>>(a);
-  else k_wy_apply<24><<<grid, kWyThreads, sm, st>>>(a);
+  const int rpw = (nmax + 15) / 16, cols = rpw <= 20 ? 64 : 32;   // columns per CTA
+  const dim3 grid((unsigned)((nmax + cols - 1) / cols), (unsigned)total);
+  EigArgs arg = a;
+  void* args[] = {&arg};
+  MSLR_CUDA_TRY(cudaLaunchKernel(wy_kernel(rpw), grid, dim3(kWyThreads), args, wy_apply_smem(nmax), st));
   return MSLR_OK;
 }
 
@@ -2402,7 +2441,8 @@ int eig_launch_group(const std::vector<const EigSegment*>& segs, const double* t
     if (nmax <= 320) k_pairs<320><<<(unsigned)total, 320, pairs_smem(nmax), st>>>(a);
     else k_pairs<kSmallT><<<(unsigned)total, kSmallT, pairs_smem(nmax), st>>>(a);
     const bool values = segs[0]->nuc != nullptr;   // (such calls have one segment)
-    if (!values) wy_apply_launch(a, nmax, total, st);
+    if (!values)
+      if (int rc = wy_apply_launch(a, nmax, total, st)) return rc;
     MSLR_CUDA_TRY(cudaGetLastError());
     if (launches) *launches += values ? 1 : 2;
     return MSLR_OK;
