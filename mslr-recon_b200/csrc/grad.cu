@@ -30,26 +30,24 @@
 
 #include "internal.h"
 #include "patchmap.cuh"
+#include "simt_tile.cuh"
 
 namespace mslr {
 
 namespace {
 
-constexpr int kTile = 64;
-constexpr int kKc = 16;
+constexpr int kTile = simt::kTile;
+constexpr int kKc = simt::kKc;
 constexpr int kRedBlocks = 592;
-
-__device__ __forceinline__ cf cmul_(cf a, cf b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
 
 // W̄[ip][a][b] = Σ_l Ō[a][l] conj(M[b][l]) over l in this split's chunk, Ō
 // and M read through the patch map from two images.  Row-major n × n blocks,
 // one per (split, patch) when split.  grid (T·T, Np, nsplit).
-__global__ void __launch_bounds__(256) k_xgram(const cf* __restrict__ imgO, const cf* __restrict__ imgM,
-                                               PatchMap m, cf* __restrict__ out, int nsplit, int lchunk) {
-  __shared__ cf As[kKc][kTile + 1];
-  __shared__ cf Bs[kKc][kTile + 1];
+template <bool TALL>
+__global__ void __launch_bounds__(simt::kThreads, 2) k_xgram(const cf* __restrict__ imgO,
+                                                             const cf* __restrict__ imgM, const PatchMap m,
+                                                             cf* __restrict__ out, int nsplit, int lchunk) {
+  __shared__ __align__(16) simt::Smem sm;
   const int T = (m.n + kTile - 1) / kTile;
   const int ta = blockIdx.x / T, tb = blockIdx.x - ta * T;
   const int64_t ip = blockIdx.y, np = gridDim.y;
@@ -58,57 +56,18 @@ __global__ void __launch_bounds__(256) k_xgram(const cf* __restrict__ imgO, cons
   const int a0 = ta * kTile, b0 = tb * kTile;
   const int l_begin = split * lchunk;
   const int l_end = min(m.L, l_begin + lchunk);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  cf acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
-  for (int l0 = l_begin; l0 < l_end; l0 += kKc) {
-    for (int q = threadIdx.x; q < kKc * kTile; q += blockDim.x) {
-      int kk, r;
-      if (m.tall) {
-        kk = q % kKc;
-        r = q / kKc;
-      } else {
-        r = q % kTile;
-        kk = q / kTile;
-      }
-      const int l = l0 + kk;
-      cf va = make_float2(0.f, 0.f), vb = make_float2(0.f, 0.f);
-      if (l < l_end) {
-        if (a0 + r < m.n) va = m_elem(m, imgO, org, a0 + r, l);
-        if (b0 + r < m.n) vb = m_elem(m, imgM, org, b0 + r, l);
-      }
-      As[kk][r] = va;
-      Bs[kk][r] = vb;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < kKc; ++kk) {
-      cf av[4], bv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[i][j].x += av[i].x * bv[j].x + av[i].y * bv[j].y;
-          acc[i][j].y += av[i].y * bv[j].x - av[i].x * bv[j].y;
-        }
-    }
-    __syncthreads();
-  }
+  simt::Acc acc;
+  acc.zero();
+  simt::accumulate(sm, simt::rows_of<TALL>(m, imgO, org, a0), simt::rows_of<TALL>(m, imgM, org, b0), l_begin, l_end,
+                   false, acc);
   const int n = m.n;
   cf* Wb = out + ((int64_t)split * np + ip) * n * n;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int a = a0 + ty * 4 + i, b = b0 + tx * 4 + j;
-      if (a < n && b < n) Wb[(int64_t)a * n + b] = acc[i][j];
+    for (int j = 0; j < 8; ++j) {
+      const int a = a0 + simt::row(i), b = b0 + simt::col(j);
+      if (a < n && b < n) Wb[(int64_t)a * n + b] = TALL ? acc.cab(i, j) : acc.acb(i, j);
     }
 }
 
@@ -123,80 +82,29 @@ __global__ void k_split_sum(const cf* __restrict__ part, cf* __restrict__ out, i
 }
 
 // C[ip] = op_a(A[ip]) · op_b(B[ip]) for row-major n × n blocks; op 0 = as is,
-// 1 = conjugate transpose.  grid (T·T, Np), 256 threads, 4 × 4 per thread.
+// 1 = conjugate transpose, at most one of the two.  grid (T·T, Np).
 template <int OPA, int OPB>
-__global__ void __launch_bounds__(256) k_bgemm(const cf* __restrict__ A, const cf* __restrict__ B,
-                                               cf* __restrict__ C, int n) {
-  __shared__ cf As[kKc][kTile + 1];   // As[k][i] = op_a(A)(i, k)
-  __shared__ cf Bs[kKc][kTile + 1];   // Bs[k][j] = op_b(B)(k, j)
+__global__ void __launch_bounds__(simt::kThreads, 2) k_bgemm(const cf* __restrict__ A, const cf* __restrict__ B,
+                                                             cf* __restrict__ C, int n) {
+  static_assert(OPA + OPB < 2, "conj(a) conj(b) is not a form of the tile's epilogue");
+  __shared__ __align__(16) simt::Smem sm;
   const int T = (n + kTile - 1) / kTile;
   const int ti = blockIdx.x / T, tj = blockIdx.x - ti * T;
   const int64_t nn = (int64_t)n * n;
-  const cf* Ap = A + blockIdx.y * nn;
-  const cf* Bp = B + blockIdx.y * nn;
   const int i0 = ti * kTile, j0 = tj * kTile;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  cf acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
-  for (int k0 = 0; k0 < n; k0 += kKc) {
-    for (int q = threadIdx.x; q < kKc * kTile; q += blockDim.x) {
-      {   // A: contiguous index fastest across threads
-        int kk, r;
-        if (OPA == 0) {   // A[i][k]: k contiguous
-          kk = q % kKc;
-          r = q / kKc;
-        } else {          // conj(A[k][i]): i contiguous
-          r = q % kTile;
-          kk = q / kTile;
-        }
-        const int i = i0 + r, k = k0 + kk;
-        cf v = make_float2(0.f, 0.f);
-        if (i < n && k < n) v = (OPA == 0) ? Ap[(int64_t)i * n + k] : cconj(Ap[(int64_t)k * n + i]);
-        As[kk][r] = v;
-      }
-      {
-        int kk, r;
-        if (OPB == 0) {   // B[k][j]: j contiguous
-          r = q % kTile;
-          kk = q / kTile;
-        } else {          // conj(B[j][k]): k contiguous
-          kk = q % kKc;
-          r = q / kKc;
-        }
-        const int j = j0 + r, k = k0 + kk;
-        cf v = make_float2(0.f, 0.f);
-        if (j < n && k < n) v = (OPB == 0) ? Bp[(int64_t)k * n + j] : cconj(Bp[(int64_t)j * n + k]);
-        Bs[kk][r] = v;
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < kKc; ++kk) {
-      cf av[4], bv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[i][j].x += av[i].x * bv[j].x - av[i].y * bv[j].y;
-          acc[i][j].y += av[i].x * bv[j].y + av[i].y * bv[j].x;
-        }
-    }
-    __syncthreads();
-  }
+  simt::Acc acc;
+  acc.zero();
+  // A[i][k] has k contiguous, A[k][i] has i; B[k][j] has j, B[j][k] has k
+  const simt::Operand<OPA == 0, simt::Linear> a(A + blockIdx.y * nn, n, i0, n, simt::Linear{});
+  const simt::Operand<OPB == 1, simt::Linear> b(B + blockIdx.y * nn, n, j0, n, simt::Linear{});
+  simt::accumulate(sm, a, b, 0, n, false, acc);
   cf* Cp = C + blockIdx.y * nn;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int a = i0 + ty * 4 + i, b = j0 + tx * 4 + j;
-      if (a < n && b < n) Cp[(int64_t)a * n + b] = acc[i][j];
+    for (int j = 0; j < 8; ++j) {
+      const int r = i0 + simt::row(i), q = j0 + simt::col(j);
+      if (r < n && q < n) Cp[(int64_t)r * n + q] = OPA ? acc.cab(i, j) : OPB ? acc.acb(i, j) : acc.ab(i, j);
     }
 }
 
@@ -248,85 +156,25 @@ __global__ void __launch_bounds__(256) k_divdiff(const cf* __restrict__ D, const
 //   tall: out[t=a][vox_l] = Σ_b conj(W[a][b]) x̄[b][vox_l] + conj(K[a][b]) z[b][vox_l]
 //   wide: out[t=l][vox_a] = Σ_b W[a][b] x̄[l][vox_b] + K[a][b] z[l][vox_b]
 // W, K row-major n × n per patch.  grid (ceil(n/64), ceil(L/64), Np).
-__global__ void __launch_bounds__(256) k_vjp_rebuild(const cf* __restrict__ xb, const cf* __restrict__ z,
-                                                     const cf* __restrict__ W, const cf* __restrict__ K,
-                                                     PatchMap m, cf* __restrict__ out, int direct) {
-  __shared__ cf As[kKc][kTile + 1];
-  __shared__ cf Bs[kKc][kTile + 1];
+template <bool TALL>
+__global__ void __launch_bounds__(simt::kThreads, 2) k_vjp_rebuild(const cf* __restrict__ xb,
+                                                                   const cf* __restrict__ z,
+                                                                   const cf* __restrict__ W,
+                                                                   const cf* __restrict__ K, const PatchMap m,
+                                                                   cf* __restrict__ out, int direct) {
+  __shared__ __align__(16) simt::Smem sm;
   const int a0 = blockIdx.x * kTile, l0 = blockIdx.y * kTile;
   const int64_t ip = blockIdx.z;
   const int n = m.n;
   const int64_t org = patch_origin(m, ip);
-  const int64_t ts = tstride(m);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  cf acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
+  simt::Acc acc;
+  acc.zero();
+#pragma unroll 1
   for (int src = 0; src < 2; ++src) {
-    const cf* Mp = (src ? K : W) + ip * (int64_t)n * n;
-    const cf* img = src ? z : xb;
-    for (int b0 = 0; b0 < n; b0 += kKc) {
-      for (int q = threadIdx.x; q < kKc * kTile; q += blockDim.x) {
-        {   // matrix tile As[b][a] = W[a][b] (row-major: b contiguous)
-          const int kk = q % kKc, r = q / kKc;
-          const int a = a0 + r, b = b0 + kk;
-          cf w = make_float2(0.f, 0.f);
-          if (a < n && b < n) {
-            w = Mp[(int64_t)a * n + b];
-            if (m.tall) w = cconj(w);
-          }
-          As[kk][r] = w;
-        }
-        {
-          int kk, r;
-          if (m.tall) {
-            r = q % kTile;
-            kk = q / kTile;
-          } else {
-            kk = q % kKc;
-            r = q / kKc;
-          }
-          const int b = b0 + kk, l = l0 + r;
-          cf v = make_float2(0.f, 0.f);
-          if (b < n && l < m.L) {
-            v = m.tall ? img[org + patch_off(m, l) + (int64_t)b * ts]
-                       : img[org + patch_off(m, b) + (int64_t)l * ts];
-          }
-          Bs[kk][r] = v;
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int kk = 0; kk < kKc; ++kk) {
-        cf av[4], bv[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) av[i] = As[kk][ty * 4 + i];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            acc[i][j].x += av[i].x * bv[j].x - av[i].y * bv[j].y;
-            acc[i][j].y += av[i].x * bv[j].y + av[i].y * bv[j].x;
-          }
-      }
-      __syncthreads();
-    }
+    const simt::Operand<true, simt::Linear> w((src ? K : W) + ip * (int64_t)n * n, n, a0, n, simt::Linear{});
+    simt::accumulate(sm, w, simt::cols_of<TALL>(m, src ? z : xb, org, l0), 0, n, false, acc);
   }
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int a = a0 + ty * 4 + i, l = l0 + tx * 4 + j;
-      if (a >= n || l >= m.L) continue;
-      const int pv = m.tall ? l : a;
-      const int tt = m.tall ? a : l;
-      if (direct) out[org + patch_off(m, pv) + (int64_t)tt * ts] = acc[i][j];
-      else out[(ip * m.Nt + tt) * (int64_t)m.p + pv] = acc[i][j];
-    }
+  simt::put_tile<TALL>(m, acc, org, ip, a0, l0, out, direct);
 }
 
 // Coverage count of voxel (x, y, z) from the per-dimension covering ranges.
@@ -436,8 +284,10 @@ int xgram_launch(const cf* imgO, const cf* imgM, const PatchMap& m, int64_t np, 
                  int nsplit, cudaStream_t st) {
   const int T = (m.n + kTile - 1) / kTile;
   const int lchunk = (nsplit > 1) ? ((m.L + nsplit - 1) / nsplit + kKc - 1) / kKc * kKc : m.L;
-  k_xgram<<<dim3(T * T, (unsigned)np, nsplit), 256, 0, st>>>(imgO, imgM, m, nsplit > 1 ? part : out,
-                                                             nsplit, lchunk);
+  const dim3 grid(T * T, (unsigned)np, nsplit);
+  cf* dst = nsplit > 1 ? part : out;
+  if (m.tall) k_xgram<true><<<grid, simt::kThreads, 0, st>>>(imgO, imgM, m, dst, nsplit, lchunk);
+  else k_xgram<false><<<grid, simt::kThreads, 0, st>>>(imgO, imgM, m, dst, nsplit, lchunk);
   if (nsplit > 1) k_split_sum<<<kRedBlocks, 256, 0, st>>>(part, out, nsplit, np * m.n * (int64_t)m.n);
   MSLR_CUDA_TRY(cudaGetLastError());
   return MSLR_OK;
@@ -446,10 +296,10 @@ int xgram_launch(const cf* imgO, const cf* imgM, const PatchMap& m, int64_t np, 
 int bgemm_launch(int opa, int opb, const cf* A, const cf* B, cf* C, int n, int64_t np, cudaStream_t st) {
   const int T = (n + kTile - 1) / kTile;
   const dim3 grid(T * T, (unsigned)np);
-  if (opa == 0 && opb == 0) k_bgemm<0, 0><<<grid, 256, 0, st>>>(A, B, C, n);
-  else if (opa == 1 && opb == 0) k_bgemm<1, 0><<<grid, 256, 0, st>>>(A, B, C, n);
-  else if (opa == 0 && opb == 1) k_bgemm<0, 1><<<grid, 256, 0, st>>>(A, B, C, n);
-  else k_bgemm<1, 1><<<grid, 256, 0, st>>>(A, B, C, n);
+  if (opa && opb) return fail(MSLR_ERR_ARG, "batched product: one conjugate transpose at most");
+  if (opa) k_bgemm<1, 0><<<grid, simt::kThreads, 0, st>>>(A, B, C, n);
+  else if (opb) k_bgemm<0, 1><<<grid, simt::kThreads, 0, st>>>(A, B, C, n);
+  else k_bgemm<0, 0><<<grid, simt::kThreads, 0, st>>>(A, B, C, n);
   MSLR_CUDA_TRY(cudaGetLastError());
   return MSLR_OK;
 }
@@ -463,8 +313,9 @@ int divdiff_launch(const cf* D, const double* lam, const cf* V, double beta, int
 
 int vjp_rebuild_launch(const cf* xb, const cf* z, const cf* W, const cf* K, const PatchMap& m,
                        int64_t np, cf* out, int direct, cudaStream_t st) {
-  k_vjp_rebuild<<<dim3((m.n + kTile - 1) / kTile, (m.L + kTile - 1) / kTile, (unsigned)np), 256, 0,
-                  st>>>(xb, z, W, K, m, out, direct);
+  const dim3 grid((m.n + kTile - 1) / kTile, (m.L + kTile - 1) / kTile, (unsigned)np);
+  if (m.tall) k_vjp_rebuild<true><<<grid, simt::kThreads, 0, st>>>(xb, z, W, K, m, out, direct);
+  else k_vjp_rebuild<false><<<grid, simt::kThreads, 0, st>>>(xb, z, W, K, m, out, direct);
   MSLR_CUDA_TRY(cudaGetLastError());
   return MSLR_OK;
 }

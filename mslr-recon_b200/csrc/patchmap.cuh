@@ -42,17 +42,6 @@ __device__ __forceinline__ int64_t patch_off(const PatchMap& m, int l) {
 
 __device__ __forceinline__ int64_t tstride(const PatchMap& m) { return m.batch ? (int64_t)m.p : m.nvox; }
 
-// M[a][l] of patch with origin `org`
-__device__ __forceinline__ cf m_elem(const PatchMap& m, const cf* __restrict__ img, int64_t org,
-                                     int a, int l) {
-  if (m.tall) {
-    const cf v = img[org + patch_off(m, l) + (int64_t)a * tstride(m)];
-    return cconj(v);
-  }
-  return img[org + patch_off(m, a) + (int64_t)l * tstride(m)];
-}
-
-
 // gram_umma.cu: split-precision BF16 (or TF32) patch Grams and rebuilds on
 // tcgen05 for the tuned and TF32 forms.
 // umma_supported: the 32-bit offset tables of those kernels cover this map.

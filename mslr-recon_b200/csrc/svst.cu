@@ -29,6 +29,7 @@
 
 #include "internal.h"
 #include "patchmap.cuh"
+#include "simt_tile.cuh"
 
 namespace mslr {
 
@@ -40,17 +41,16 @@ void set_context_free_polls(int polls) { g_free_polls.store(polls); }
 
 namespace {
 
-constexpr int kTile = 64;
-constexpr int kKc = 16;
+constexpr int kTile = simt::kTile;
 
 // ---------------------------------------------------------------------------
 // Gram: G[a][b] = Σ_l M[a][l] conj(M[b][l]) on lower-triangle 64×64 tiles.
 // grid (ntri, Np, nsplit).  Output column-major: G[b*n + a].
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_gram(const cf* __restrict__ img, PatchMap m,
-                                              cf* __restrict__ out, int nsplit, int lchunk) {
-  __shared__ cf As[kKc][kTile + 1];
-  __shared__ cf Bs[kKc][kTile + 1];
+template <bool TALL>
+__global__ void __launch_bounds__(simt::kThreads, 2) k_gram(const cf* __restrict__ img, const PatchMap m,
+                                                            cf* __restrict__ out, int nsplit, int lchunk) {
+  __shared__ __align__(16) simt::Smem sm;
   // tile pair from the linear lower-triangle index
   int t = blockIdx.x, ta = 0;
   while (t > ta) {
@@ -64,61 +64,21 @@ __global__ void __launch_bounds__(256) k_gram(const cf* __restrict__ img, PatchM
   const int a0 = ta * kTile, b0 = tb * kTile;
   const int l_begin = split * lchunk;
   const int l_end = min(m.L, l_begin + lchunk);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  cf acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
-  for (int l0 = l_begin; l0 < l_end; l0 += kKc) {
-    // load: 1024 elements each for A and B; kk fastest for tall (voxel-contiguous)
-    for (int q = threadIdx.x; q < kKc * kTile; q += blockDim.x) {
-      int kk, r;
-      if (m.tall) {
-        kk = q % kKc;
-        r = q / kKc;
-      } else {
-        r = q % kTile;
-        kk = q / kTile;
-      }
-      const int l = l0 + kk;
-      cf va = make_float2(0.f, 0.f), vb = make_float2(0.f, 0.f);
-      if (l < l_end) {
-        if (a0 + r < m.n) va = m_elem(m, img, org, a0 + r, l);
-        if (b0 + r < m.n) vb = m_elem(m, img, org, b0 + r, l);
-      }
-      As[kk][r] = va;
-      Bs[kk][r] = vb;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < kKc; ++kk) {
-      cf av[4], bv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          // av * conj(bv)
-          acc[i][j].x += av[i].x * bv[j].x + av[i].y * bv[j].y;
-          acc[i][j].y += av[i].y * bv[j].x - av[i].x * bv[j].y;
-        }
-    }
-    __syncthreads();
-  }
+  simt::Acc acc;
+  acc.zero();
+  simt::accumulate(sm, simt::rows_of<TALL>(m, img, org, a0), simt::rows_of<TALL>(m, img, org, b0), l_begin, l_end,
+                   ta == tb, acc);
   const int n = m.n;
   cf* G = out + ((nsplit > 1) ? (int64_t)split * n * n : ip * (int64_t)n * n);
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int a = a0 + ty * 4 + i, b = b0 + tx * 4 + j;
+    for (int j = 0; j < 8; ++j) {
+      const int a = a0 + simt::row(i), b = b0 + simt::col(j);
       if (a < n && b < n) {
-        G[(int64_t)b * n + a] = acc[i][j];
-        if (ta != tb) G[(int64_t)a * n + b] = cconj(acc[i][j]);
+        const cf g = TALL ? acc.cab(i, j) : acc.acb(i, j);
+        G[(int64_t)b * n + a] = g;
+        if (ta != tb) G[(int64_t)a * n + b] = cconj(g);
       }
     }
 }
@@ -139,84 +99,20 @@ __global__ void k_gram_reduce(const cf* __restrict__ part, cf* __restrict__ G, i
 // grid (ceil(n/64), ceil(L/64), Np).  Writes the image directly when the
 // patch grid is an exact partition, else the per-patch buffer (p, Nt, Np).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_rebuild(const cf* __restrict__ img, const cf* __restrict__ W,
-                                                 PatchMap m, cf* __restrict__ out, int direct) {
-  __shared__ cf As[kKc][kTile + 1];   // W[a][b]
-  __shared__ cf Bs[kKc][kTile + 1];   // input values for (b, l)
+template <bool TALL>
+__global__ void __launch_bounds__(simt::kThreads, 2) k_rebuild(const cf* __restrict__ img, const cf* __restrict__ W,
+                                                               const PatchMap m, cf* __restrict__ out, int direct) {
+  __shared__ __align__(16) simt::Smem sm;
   const int a0 = blockIdx.x * kTile, l0 = blockIdx.y * kTile;
   const int64_t ip = blockIdx.z;
   const int n = m.n;
-  const cf* Wp = W + ip * (int64_t)n * n;
   const int64_t org = patch_origin(m, ip);
-  const int64_t ts = tstride(m);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  cf acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
-  for (int b0 = 0; b0 < n; b0 += kKc) {
-    for (int q = threadIdx.x; q < kKc * kTile; q += blockDim.x) {
-      // W tile: a fastest (column-major W[b*n + a])
-      {
-        const int r = q % kTile, kk = q / kTile;
-        const int a = a0 + r, b = b0 + kk;
-        cf w = make_float2(0.f, 0.f);
-        if (a < n && b < n) {
-          w = Wp[(int64_t)b * n + a];
-          if (m.tall) w = cconj(w);
-        }
-        As[kk][r] = w;
-      }
-      // input tile
-      {
-        int kk, r;
-        if (m.tall) {   // img[b][vox_l]: l contiguous
-          r = q % kTile;
-          kk = q / kTile;
-        } else {        // img[l][vox_b]: b contiguous
-          kk = q % kKc;
-          r = q / kKc;
-        }
-        const int b = b0 + kk, l = l0 + r;
-        cf v = make_float2(0.f, 0.f);
-        if (b < n && l < m.L) {
-          v = m.tall ? img[org + patch_off(m, l) + (int64_t)b * ts]
-                     : img[org + patch_off(m, b) + (int64_t)l * ts];
-        }
-        Bs[kk][r] = v;
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < kKc; ++kk) {
-      cf av[4], bv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[i][j].x += av[i].x * bv[j].x - av[i].y * bv[j].y;
-          acc[i][j].y += av[i].x * bv[j].y + av[i].y * bv[j].x;
-        }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int a = a0 + ty * 4 + i, l = l0 + tx * 4 + j;
-      if (a >= n || l >= m.L) continue;
-      // element (voxel, frame) of the patch
-      const int pv = m.tall ? l : a;
-      const int tt = m.tall ? a : l;
-      if (direct) out[org + patch_off(m, pv) + (int64_t)tt * ts] = acc[i][j];
-      else out[(ip * m.Nt + tt) * (int64_t)m.p + pv] = acc[i][j];
-    }
+  simt::Acc acc;
+  acc.zero();
+  // W column-major: W[b*n + a]
+  const simt::Operand<false, simt::Linear> w(W + ip * (int64_t)n * n, n, a0, n, simt::Linear{});
+  simt::accumulate(sm, w, simt::cols_of<TALL>(m, img, org, l0), 0, n, false, acc);
+  simt::put_tile<TALL>(m, acc, org, ip, a0, l0, out, direct);
 }
 
 // img2patches: P[(ip*Nt + t)*p + l] = img[t][vox(ip, l)]
@@ -324,7 +220,9 @@ int svst_gram(const cf* in, const PatchMap& m, int64_t np, const WorkPtrs& w, in
   if (tc && umma_supported(m)) {
     if (int rc = gram_umma_launch(in, m, np, dst, nsplit, lchunk, dw, st, tc == 2, kcols)) return rc;
   } else {
-    k_gram<<<dim3(ntri, (unsigned)np, nsplit), 256, 0, st>>>(in, m, dst, nsplit, lchunk);
+    const dim3 grid(ntri, (unsigned)np, nsplit);
+    if (m.tall) k_gram<true><<<grid, simt::kThreads, 0, st>>>(in, m, dst, nsplit, lchunk);
+    else k_gram<false><<<grid, simt::kThreads, 0, st>>>(in, m, dst, nsplit, lchunk);
   }
   if (nsplit > 1) k_gram_reduce<<<592, 256, 0, st>>>(w.part, w.gram, nsplit, (int64_t)n * n);
   MSLR_CUDA_TRY(cudaGetLastError());
@@ -338,8 +236,9 @@ int svst_rebuild(const cf* in, const PatchMap& m, int64_t np, const WorkPtrs& w,
   if (tc && umma_supported(m))
     return rebuild_umma_launch(in, w.gram, m, np, out, direct, dw, st, tc == 2);
   const int n = m.n;
-  k_rebuild<<<dim3((n + kTile - 1) / kTile, (m.L + kTile - 1) / kTile, (unsigned)np), 256, 0, st>>>(
-      in, w.gram, m, out, direct);
+  const dim3 grid((n + kTile - 1) / kTile, (m.L + kTile - 1) / kTile, (unsigned)np);
+  if (m.tall) k_rebuild<true><<<grid, simt::kThreads, 0, st>>>(in, w.gram, m, out, direct);
+  else k_rebuild<false><<<grid, simt::kThreads, 0, st>>>(in, w.gram, m, out, direct);
   MSLR_CUDA_TRY(cudaGetLastError());
   return MSLR_OK;
 }
