@@ -68,7 +68,6 @@ static void free_ctx(mslr_ctx* c) {
     if (p) cudaFree(p);
   for (auto& w : c->svw)
     if (w.gram) cudaFree(w.gram);
-  for (auto& g : c->scales) geom_free(&g);
   for (cudaEvent_t e : c->prof_ev) cudaEventDestroy(e);
   if (c->gexec) cudaGraphExecDestroy(c->gexec);
   if (c->gev_in) cudaEventDestroy(c->gev_in);
@@ -245,7 +244,6 @@ int mslr_create(const int32_t N[3], int32_t Nc, int32_t Nt, int64_t K, int32_t n
     rc = geom_build(c->N, Nt, p3, s3, &c->scales[k]);
     if (!rc && c->scales[k].n > 1024)
       rc = fail(MSLR_ERR_UNSUPPORTED, "min(patch voxels, Nt) must be <= 1024");
-    if (!rc) rc = geom_upload(&c->scales[k], c->N);
     // Ong–Lustig λ with the unclamped patch size (scripts/reconstruct.jl:163-169)
     const double pk = (double)p3[0] * p3[1] * p3[2];
     c->lambdas.push_back(std::sqrt(pk) + std::sqrt((double)Nt) +

@@ -58,13 +58,9 @@ struct ScaleGeom {
   bool tall;        // p >= Nt: Gram = P^H P (time x time); else P P^H (voxel x voxel)
   bool partition;   // patches tile the volume exactly (no overlap, no gaps)
   bool global;      // one patch covering the whole volume
-  int* d_starts;    // device: x-starts, y-starts, z-starts (nsteps+1 each)
-  // coverage ranges per dim for the gather recombine: for coordinate c in dim d,
-  // covering patch indices along d are [lo, hi] (inclusive); -1 if none
-  int* d_cover;     // device: per dim, 2*N[d] ints
   int nsplit_tuned = 0;   // split-K count of the Gram chosen by the autotuner (0: heuristic)
   int eig_big = 0;        // eigen stage in the 1024-thread CTA variant (autotuner; n > 384 always is)
-  std::vector<int> h_starts;
+  std::vector<int> h_starts;   // x-starts, y-starts, z-starts (nsteps+1 each)
 };
 
 // Status helpers -------------------------------------------------------------

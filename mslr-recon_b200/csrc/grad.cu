@@ -177,62 +177,6 @@ __global__ void __launch_bounds__(simt::kThreads, 2) k_vjp_rebuild(const cf* __r
   simt::put_tile<TALL>(m, acc, org, ip, a0, l0, out, direct);
 }
 
-// Coverage count of voxel (x, y, z) from the per-dimension covering ranges.
-__device__ __forceinline__ float cover_count(const int* cover, const PatchMap& m, int64_t v) {
-  const int x = (int)(v % m.Nx);
-  const int y = (int)((v / m.Nx) % m.Ny);
-  const int z = (int)(v / ((int64_t)m.Nx * m.Ny));
-  const int* cx = cover;
-  const int* cy = cover + 2 * m.Nx;
-  const int* cz = cy + 2 * m.Ny;
-  if (cx[2 * x] < 0 || cy[2 * y] < 0 || cz[2 * z] < 0) return 0.f;
-  return (float)((cx[2 * x + 1] - cx[2 * x] + 1) * (cy[2 * y + 1] - cy[2 * y] + 1) *
-                 (cz[2 * z + 1] - cz[2 * z] + 1));
-}
-
-// out = img / max(count, 1): the adjoint of patches2img's averaging, before the gather
-__global__ void k_div_count(const cf* __restrict__ img, PatchMap m, const int* __restrict__ cover,
-                            cf* __restrict__ out) {
-  const int64_t total = (int64_t)m.Nt * m.nvox;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
-       q += (int64_t)gridDim.x * blockDim.x) {
-    const float c = fmaxf(cover_count(cover, m, q % m.nvox), 1.f);
-    out[q] = make_float2(img[q].x / c, img[q].y / c);
-  }
-}
-
-// Scatter-add of per-patch values (the adjoint of img2patches) as a gather
-// over covering patches in ascending ip; uncovered voxels get 0.
-__global__ void k_patch_sum(const cf* __restrict__ P, PatchMap m, const int* __restrict__ cover,
-                            cf* __restrict__ img) {
-  const int64_t total = (int64_t)m.Nt * m.nvox;
-  const int* cx = cover;
-  const int* cy = cover + 2 * m.Nx;
-  const int* cz = cy + 2 * m.Ny;
-  const int* sxs = m.starts;
-  const int* sys = m.starts + m.nx;
-  const int* szs = m.starts + m.nx + m.ny;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
-       q += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t v = q % m.nvox;
-    const int t = (int)(q / m.nvox);
-    const int x = (int)(v % m.Nx);
-    const int y = (int)((v / m.Nx) % m.Ny);
-    const int z = (int)(v / ((int64_t)m.Nx * m.Ny));
-    cf acc = make_float2(0.f, 0.f);
-    if (cx[2 * x] >= 0 && cy[2 * y] >= 0 && cz[2 * z] >= 0) {
-      for (int iz = cz[2 * z]; iz <= cz[2 * z + 1]; ++iz)
-        for (int iy = cy[2 * y]; iy <= cy[2 * y + 1]; ++iy)
-          for (int ix = cx[2 * x]; ix <= cx[2 * x + 1]; ++ix) {
-            const int64_t ip = ix + (int64_t)m.nx * (iy + (int64_t)m.ny * iz);
-            const int l = (x - sxs[ix]) + m.psx * ((y - sys[iy]) + m.psy * (z - szs[iz]));
-            acc = cadd(acc, P[(ip * m.Nt + t) * (int64_t)m.p + l]);
-          }
-    }
-    img[q] = acc;
-  }
-}
-
 // r = Σ_k X_k − X_true;  xbar_k = r for every scale;  part[b] = Σ |r|² (FP64)
 __global__ void __launch_bounds__(256) k_loss_seed(const cf* __restrict__ X, const cf* __restrict__ Xt,
                                                    int ns, int64_t E, cf* __restrict__ xbar,
@@ -316,18 +260,6 @@ int vjp_rebuild_launch(const cf* xb, const cf* z, const cf* W, const cf* K, cons
   const dim3 grid((m.n + kTile - 1) / kTile, (m.L + kTile - 1) / kTile, (unsigned)np);
   if (m.tall) k_vjp_rebuild<true><<<grid, simt::kThreads, 0, st>>>(xb, z, W, K, m, out, direct);
   else k_vjp_rebuild<false><<<grid, simt::kThreads, 0, st>>>(xb, z, W, K, m, out, direct);
-  MSLR_CUDA_TRY(cudaGetLastError());
-  return MSLR_OK;
-}
-
-int div_count_launch(const cf* img, const PatchMap& m, const int* cover, cf* out, cudaStream_t st) {
-  k_div_count<<<1184, 256, 0, st>>>(img, m, cover, out);
-  MSLR_CUDA_TRY(cudaGetLastError());
-  return MSLR_OK;
-}
-
-int patch_sum_launch(const cf* P, const PatchMap& m, const int* cover, cf* img, cudaStream_t st) {
-  k_patch_sum<<<1184, 256, 0, st>>>(P, m, cover, img);
   MSLR_CUDA_TRY(cudaGetLastError());
   return MSLR_OK;
 }

@@ -219,8 +219,6 @@ int patch_svst_lambdas(Ctx* c, int s, const double* lambdas_host, const cf* img_
 // nuclear norms of every patch of scale s of img, in patch order (synchronises st)
 int patch_nucnorms(Ctx* c, int s, const cf* img, std::vector<double>& out, cudaStream_t st);
 int geom_build(const int N[3], int Nt, const int ps_in[3], const int ss_in[3], ScaleGeom* g);
-int geom_upload(ScaleGeom* g, const int N[3]);
-void geom_free(ScaleGeom* g);
 
 // ---- eig.cu --------------------------------------------------------------------
 // One group of patches that share a Gram side n and a threshold multiplier.
@@ -318,7 +316,9 @@ int divdiff_launch(const cf* D, const double* lam, const cf* V, double beta, int
                    cf* T3, double* bbar, cudaStream_t st);
 int vjp_rebuild_launch(const cf* xb, const cf* z, const cf* W, const cf* K, const PatchMap& m,
                        int64_t np, cf* out, int direct, cudaStream_t st);
-int div_count_launch(const cf* img, const PatchMap& m, const int* cover, cf* out, cudaStream_t st);
-int patch_sum_launch(const cf* P, const PatchMap& m, const int* cover, cf* img, cudaStream_t st);
+int div_count_launch(const cf* img, const PatchMap& m, cf* out, cudaStream_t st);
+int patch_sum_launch(const cf* P, const PatchMap& m, cf* img, cudaStream_t st);
+int img2patches_launch(const cf* img, const PatchMap& m, int64_t np, cf* P, cudaStream_t st);
+int patches2img_launch(const cf* P, const PatchMap& m, cf* img, cudaStream_t st);
 
 }  // namespace mslr

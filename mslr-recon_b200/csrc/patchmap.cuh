@@ -15,20 +15,24 @@ struct PatchMap {
   int Nt;
   int psx, psy, psz;
   int nx, ny, nz;     // patches per dim
-  const int* starts;  // nx x-starts, ny y-starts, nz z-starts
+  int ssx, ssy, ssz;  // strides
   int p, n, L;
   int tall;
   int batch;
   int64_t mstride;
 };
 
+// Start of the i-th of an axis's patches: the last one ends with the axis.
+__device__ __forceinline__ int patch_start(int i, int ss, int n, int ps) { return min(i * ss, n - ps); }
+
 __device__ __forceinline__ int64_t patch_origin(const PatchMap& m, int64_t ip) {
   if (m.batch) return ip * m.mstride;
   const int ix = (int)(ip % m.nx);
   const int iy = (int)((ip / m.nx) % m.ny);
   const int iz = (int)(ip / ((int64_t)m.nx * m.ny));
-  const int sx = m.starts[ix], sy = m.starts[m.nx + iy], sz = m.starts[m.nx + m.ny + iz];
-  return sx + (int64_t)m.Nx * (sy + (int64_t)m.Ny * sz);
+  return patch_start(ix, m.ssx, m.Nx, m.psx) +
+         (int64_t)m.Nx * (patch_start(iy, m.ssy, m.Ny, m.psy) +
+                          (int64_t)m.Ny * patch_start(iz, m.ssz, m.Nz, m.psz));
 }
 
 __device__ __forceinline__ int64_t patch_off(const PatchMap& m, int l) {

@@ -115,64 +115,6 @@ __global__ void __launch_bounds__(simt::kThreads, 2) k_rebuild(const cf* __restr
   simt::put_tile<TALL>(m, acc, org, ip, a0, l0, out, direct);
 }
 
-// img2patches: P[(ip*Nt + t)*p + l] = img[t][vox(ip, l)]
-__global__ void k_img2patches(const cf* __restrict__ img, PatchMap m, cf* __restrict__ P,
-                              int64_t total) {
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
-       q += (int64_t)gridDim.x * blockDim.x) {
-    const int l = (int)(q % m.p);
-    const int64_t r = q / m.p;
-    const int t = (int)(r % m.Nt);
-    const int64_t ip = r / m.Nt;
-    P[q] = img[patch_origin(m, ip) + patch_off(m, l) + (int64_t)t * m.nvox];
-  }
-}
-
-// Gather recombine (patches2img): for voxel v and frame t, Σ over covering
-// patches in ascending ip of P[(ip*Nt + t)*p + l(v, ip)], divided by
-// max(count, 1).  cover: per dim 2*N[d] ints (lo, hi) of covering indices.
-__global__ void k_recombine(const cf* __restrict__ P, PatchMap m, const int* __restrict__ cover,
-                            cf* __restrict__ img) {
-  const int64_t total = (int64_t)m.Nt * m.nvox;
-  const int* cx = cover;
-  const int* cy = cover + 2 * m.Nx;
-  const int* cz = cy + 2 * m.Ny;
-  const int* sxs = m.starts;
-  const int* sys = m.starts + m.nx;
-  const int* szs = m.starts + m.nx + m.ny;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
-       q += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t v = q % m.nvox;
-    const int t = (int)(q / m.nvox);
-    const int x = (int)(v % m.Nx);
-    const int y = (int)((v / m.Nx) % m.Ny);
-    const int z = (int)(v / ((int64_t)m.Nx * m.Ny));
-    const int xl = cx[2 * x], xh = cx[2 * x + 1];
-    const int yl = cy[2 * y], yh = cy[2 * y + 1];
-    const int zl = cz[2 * z], zh = cz[2 * z + 1];
-    cf acc = make_float2(0.f, 0.f);
-    float cnt = 0.f;
-    if (xl >= 0 && yl >= 0 && zl >= 0) {
-      for (int iz = zl; iz <= zh; ++iz)
-        for (int iy = yl; iy <= yh; ++iy)
-          for (int ix = xl; ix <= xh; ++ix) {
-            const int64_t ip = ix + (int64_t)m.nx * (iy + (int64_t)m.ny * iz);
-            const int l = (x - sxs[ix]) + m.psx * ((y - sys[iy]) + m.psy * (z - szs[iz]));
-            acc = cadd(acc, P[(ip * m.Nt + t) * (int64_t)m.p + l]);
-            cnt += 1.f;
-          }
-    }
-    cnt = fmaxf(cnt, 1.f);
-    img[q] = make_float2(acc.x / cnt, acc.y / cnt);
-  }
-}
-
-__global__ void k_zero(cf* p, int64_t n) {
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n;
-       q += (int64_t)gridDim.x * blockDim.x)
-    p[q] = make_float2(0.f, 0.f);
-}
-
 PatchMap map_of(const ScaleGeom& g, const int N[3], int Nt, int64_t nvox) {
   PatchMap m;
   m.Nx = N[0];
@@ -186,7 +128,9 @@ PatchMap map_of(const ScaleGeom& g, const int N[3], int Nt, int64_t nvox) {
   m.nx = g.nsteps[0] + 1;
   m.ny = g.nsteps[1] + 1;
   m.nz = g.nsteps[2] + 1;
-  m.starts = g.d_starts;
+  m.ssx = g.ss[0];
+  m.ssy = g.ss[1];
+  m.ssz = g.ss[2];
   m.p = g.p;
   m.n = g.n;
   m.L = g.L;
@@ -291,78 +235,6 @@ int split_of(const ScaleGeom& g) {
 
 }  // namespace
 
-// ---------------------------------------------------------------------------
-// geometry (host)
-// ---------------------------------------------------------------------------
-int geom_build(const int N[3], int Nt, const int ps_in[3], const int ss_in[3], ScaleGeom* g) {
-  int64_t Np = 1;
-  g->h_starts.clear();
-  bool partition = true;
-  for (int d = 0; d < 3; ++d) {
-    if (ps_in[d] <= 0 || ss_in[d] <= 0)
-      return fail(MSLR_ERR_ARG, "patch sizes and strides must be positive");
-    g->ps[d] = std::min(ps_in[d], N[d]);
-    g->ss[d] = ss_in[d];
-    const int num = N[d] - g->ps[d];
-    g->nsteps[d] = (num + g->ss[d] - 1) / g->ss[d];   // cld for num >= 0
-    Np *= (g->nsteps[d] + 1);
-    int prev = -1;
-    for (int i = 0; i <= g->nsteps[d]; ++i) {
-      const int s = std::min(i * g->ss[d], N[d] - g->ps[d]);
-      g->h_starts.push_back(s);
-      if (i == 0 && s != 0) partition = false;
-      if (i > 0 && s - prev != g->ps[d]) partition = false;
-      prev = s;
-    }
-    if (prev + g->ps[d] != N[d]) partition = false;
-  }
-  g->Np = Np;
-  g->p = g->ps[0] * g->ps[1] * g->ps[2];
-  g->n = std::min(g->p, Nt);
-  g->L = std::max(g->p, Nt);
-  g->tall = g->p >= Nt;
-  g->partition = partition;
-  g->global = (Np == 1 && g->ps[0] == N[0] && g->ps[1] == N[1] && g->ps[2] == N[2]);
-  g->d_starts = nullptr;
-  g->d_cover = nullptr;
-  return MSLR_OK;
-}
-
-int geom_upload(ScaleGeom* g, const int N[3]) {
-  std::vector<int> cover;
-  size_t off = 0;
-  for (int d = 0; d < 3; ++d) {
-    const int cnt = g->nsteps[d] + 1;
-    for (int c = 0; c < N[d]; ++c) {
-      int lo = -1, hi = -1;
-      for (int i = 0; i < cnt; ++i) {
-        const int s = g->h_starts[off + i];
-        if (s <= c && c < s + g->ps[d]) {
-          if (lo < 0) lo = i;
-          hi = i;
-        }
-      }
-      cover.push_back(lo);
-      cover.push_back(hi);
-    }
-    off += cnt;
-  }
-  MSLR_CUDA_TRY(cudaMalloc((void**)&g->d_starts, g->h_starts.size() * sizeof(int)));
-  MSLR_CUDA_TRY(cudaMemcpy(g->d_starts, g->h_starts.data(), g->h_starts.size() * sizeof(int),
-                           cudaMemcpyHostToDevice));
-  MSLR_CUDA_TRY(cudaMalloc((void**)&g->d_cover, cover.size() * sizeof(int)));
-  MSLR_CUDA_TRY(cudaMemcpy(g->d_cover, cover.data(), cover.size() * sizeof(int),
-                           cudaMemcpyHostToDevice));
-  return MSLR_OK;
-}
-
-void geom_free(ScaleGeom* g) {
-  if (g->d_starts) cudaFree(g->d_starts);
-  if (g->d_cover) cudaFree(g->d_cover);
-  g->d_starts = nullptr;
-  g->d_cover = nullptr;
-}
-
 static size_t eig_work_bytes(int64_t np, int n, int nsplit) {
   const size_t nn = (size_t)n * n;
   return np * nn * sizeof(cf) * 2 + np * nn * sizeof(double) + np * 6 * (size_t)n * sizeof(double) +
@@ -445,8 +317,7 @@ int patch_svst(Ctx* c, int s, const double* thr_dev, double lam, const cf* img_i
     if ((rc = svst_core(img_in, m, g.Np, w, nsplit, thr_dev, thr_per_patch, lam, c->d_pbuf, 0, tc,
                         ctx_wait(c), st, &c->launches, g.eig_big)))
       return rc;
-    k_recombine<<<1184, 256, 0, st>>>(c->d_pbuf, m, g.d_cover, img_out);
-    MSLR_CUDA_TRY(cudaGetLastError());
+    if ((rc = patches2img_launch(c->d_pbuf, m, img_out, st))) return rc;
     c->launches += 1;
   }
   return MSLR_OK;
@@ -538,8 +409,7 @@ int patch_svst_from_gram(Ctx* c, int s, double beta, const cf* gram, const cf* i
   if ((rc = svst_rebuild(img_in, m, 1, w, dst, g.partition ? 1 : 0, tc, ctx_wait(c), st, &c->launches)))
     return rc;
   if (!g.partition) {
-    k_recombine<<<1184, 256, 0, st>>>(c->d_pbuf, m, g.d_cover, img_out);
-    MSLR_CUDA_TRY(cudaGetLastError());
+    if ((rc = patches2img_launch(c->d_pbuf, m, img_out, st))) return rc;
     c->launches += 1;
   } else if (dst != img_out) {
     MSLR_CUDA_TRY(cudaMemcpyAsync(img_out, dst, (size_t)c->Nt * c->nvox * sizeof(cf), cudaMemcpyDeviceToDevice,
@@ -643,8 +513,7 @@ int patch_svst_all(Ctx* c, const double* thr_dev, const cf* Zin, cf* Xout, cudaS
       if ((rc = svst_rebuild(Zin + k * E, m, g.Np, ws[k], c->d_pbuf, 0, c->tc_mode(), ctx_wait(c), st,
                              &c->launches)))
         return rc;
-      k_recombine<<<1184, 256, 0, st>>>(c->d_pbuf, m, g.d_cover, Xout + k * E);
-      MSLR_CUDA_TRY(cudaGetLastError());
+      if ((rc = patches2img_launch(c->d_pbuf, m, Xout + k * E, st))) return rc;
       c->launches += 1;
     }
   }
@@ -659,22 +528,10 @@ int patches_op(const int N[3], int Nt, const int ps[3], const int ss[3], const c
   ScaleGeom g;
   int rc = geom_build(N, Nt, ps, ss, &g);
   if (rc) return rc;
-  if ((rc = geom_upload(&g, N))) {
-    geom_free(&g);
-    return rc;
-  }
-  const int64_t nvox = (int64_t)N[0] * N[1] * N[2];
-  const PatchMap m = map_of(g, N, Nt, nvox);
-  if (to_patches) {
-    const int64_t total = g.Np * Nt * (int64_t)g.p;
-    k_img2patches<<<1184, 256, 0, st>>>(src, m, dst, total);
-  } else {
-    k_recombine<<<1184, 256, 0, st>>>(src, m, g.d_cover, dst);
-  }
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  geom_free(&g);
-  if (e != cudaSuccess) return fail(MSLR_ERR_CUDA, cudaGetErrorString(e));
+  const PatchMap m = map_of(g, N, Nt, (int64_t)N[0] * N[1] * N[2]);
+  rc = to_patches ? img2patches_launch(src, m, g.Np, dst, st) : patches2img_launch(src, m, dst, st);
+  if (rc) return rc;
+  MSLR_CUDA_TRY(cudaStreamSynchronize(st));
   return MSLR_OK;
 }
 
@@ -714,7 +571,8 @@ int svst_batch(int mrows, int ncols, int batch, const double* betas, const cf* i
   m.psy = 1;
   m.psz = 1;
   m.nx = m.ny = m.nz = 1;
-  m.starts = nullptr;
+  m.ssx = mrows;
+  m.ssy = m.ssz = 1;
   m.p = mrows;
   m.n = n;
   m.L = std::max(mrows, ncols);
@@ -897,7 +755,7 @@ int svst_vjp_scale(Ctx* c, int s, const cf* z, const cf* xbar, double beta, cf* 
   int rc;
   const cf* ob = xbar;
   if (!g.partition) {
-    if ((rc = div_count_launch(xbar, m, g.d_cover, tmp, st))) return rc;
+    if ((rc = div_count_launch(xbar, m, tmp, st))) return rc;
     ob = tmp;
   }
   WorkPtrs w{};
@@ -930,7 +788,7 @@ int svst_vjp_scale(Ctx* c, int s, const cf* z, const cf* xbar, double beta, cf* 
     if ((rc = vjp_rebuild_launch(ob, z, v.wbar, v.d, m, np, zbar, 1, st))) return rc;
   } else {
     if ((rc = vjp_rebuild_launch(ob, z, v.wbar, v.d, m, np, c->d_pbuf, 0, st))) return rc;
-    if ((rc = patch_sum_launch(c->d_pbuf, m, g.d_cover, zbar, st))) return rc;
+    if ((rc = patch_sum_launch(c->d_pbuf, m, zbar, st))) return rc;
   }
   c->launches += 10;
   std::vector<double> hb((size_t)np);
