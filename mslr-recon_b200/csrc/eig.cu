@@ -1105,6 +1105,12 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
 // patch: 351 µs), the latency of its round trips and four barriers.
 // A warp's tile column is rotated by its tile row, so that the tiles left in
 // play when the leading ones are done stay spread over the SM's schedulers.
+// The tile pass is as much shared-memory loads as FMAs: a 16-byte load takes
+// the pipe four cycles, so (v, w) of a row or column come in one, without the
+// doubled components that a packed FMA would take directly (those are moves,
+// for which the FMAs leave issue slots), and the reflector's scalars that only
+// the vector phases need are worked out by their warps alone: 148 matrices of
+// side 128 252 -> 227 us, 216 of side 64 99 -> 94.
 // CU columns per lane: tiles of 32 rows × 4·CU columns, one per warp.  Eight is
 // what 16 warps' registers hold at NT = 4; with four the smaller sides have
 // twice the warps, so the latencies of a tile pass overlap.
@@ -1113,29 +1119,36 @@ template <int NT>
 struct TriVec {
   static constexpr int NP = 32 * NT, LD = NP + 1, CU = tri_cu(NT), TC = 4 * CU, NTC = NP / TC;
   static constexpr int kThreads = NT * NTC * 32;
-  float4 dw[NP], dv[NP];  // the pending update of column j: (wp.x, wp.x, wp.y, wp.y), (vp.x, vp.x, vp.y, vp.y)
-  float4 sx[NP];          // this step's column x below the subdiagonal: (x.x, x.y, x.y, x.x)
+  float4 vw[NP];          // the pending update, by row: (vp, wp)
+  cf sx[NP];              // this step's column x below the subdiagonal
   cf scol[NP];            // next column, before the pending update
   cf part[NTC][NP];       // per tile column: partial sums of A u
   float red0[4], redt[NT * NTC];
   cf x1;
 };
 
-// zlarfg with α = (ar, ai) and ‖x‖² = xn: β, τ, u₁ = α − β and 1 / u₁.  The root
-// and its reciprocal from one approximation, each refined to the last bit by
-// a Newton step (shorter than a root followed by a division by it).
-__device__ __forceinline__ void reflector(float ar, float ai, float xn, float* bt, cf* tau, cf* u1, cf* scal) {
-  const float s = ar * ar + ai * ai + xn;
-  float r = rsqrtf(s);
-  r = fmaf(0.5f * r, fmaf(-s * r, r, 1.f), r);
-  float q = s * r;
-  q = fmaf(0.5f * r, fmaf(-q, q, s), q);
-  const float b = -copysignf(q, ar), ib = -copysignf(r, ar);
-  *bt = b;
-  *tau = make_float2((b - ar) * ib, -ai * ib);
-  *u1 = make_float2(ar - b, ai);
-  const float id = __frcp_rn(u1->x * u1->x + ai * ai);
-  *scal = make_float2(u1->x * id, -ai * id);
+// zlarfg with α = (ar, ai) and ‖x‖² = xn: Hᴴ (α, x) = (β, 0), H = I − τ v vᴴ, β
+// real, v = (1, x / u₁), u₁ = α − β.  The root and its reciprocal come from one
+// approximation, each refined to the last bit by a Newton step (shorter than a
+// root followed by a division by it).
+struct Reflector {
+  float b, ib;   // β, 1/β
+  __device__ __forceinline__ Reflector(float ar, float ai, float xn) {
+    const float s = ar * ar + ai * ai + xn;
+    float r = rsqrtf(s);
+    r = fmaf(0.5f * r, fmaf(-s * r, r, 1.f), r);
+    float q = s * r;
+    q = fmaf(0.5f * r, fmaf(-q, q, s), q);
+    b = -copysignf(q, ar);
+    ib = -copysignf(r, ar);
+  }
+  __device__ __forceinline__ cf u1(float ar, float ai) const { return make_float2(ar - b, ai); }
+  __device__ __forceinline__ cf tau(float ar, float ai) const { return make_float2((b - ar) * ib, -ai * ib); }
+};
+// 1 / u₁
+__device__ __forceinline__ cf inverse(cf u) {
+  const float id = __frcp_rn(u.x * u.x + u.y * u.y);
+  return make_float2(u.x * id, -u.y * id);
 }
 
 // The n steps of the n × n Hermitian matrix at A (column stride ld, n <= 32·NT,
@@ -1167,7 +1180,7 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
   const int i = tid;                 // row of the vector phases
   const bool own = tid < NP;         // (the first NT warps)
   if (own) {
-    m.dw[i] = m.dv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    m.vw[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     m.scol[i] = (i < n) ? __ldcg(A + i) : make_float2(0.f, 0.f);
   }
   const int row = I * 32 + rg + 8 * cg;   // row whose sum this lane ends with
@@ -1180,7 +1193,7 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
       if (i == k) dd[k] = (double)x.x;
       if (i == k + 1) m.x1 = x;
       if (i <= k + 1) x = make_float2(0.f, 0.f);
-      m.sx[i] = make_float4(x.x, x.y, x.y, x.x);
+      m.sx[i] = x;
       const float q = warp_sum(cabs2(x));
       if (lane == 0) m.red0[warp] = q;
     }
@@ -1188,13 +1201,21 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
     float xn = 0.f;
 #pragma unroll
     for (int q = 0; q < NT; ++q) xn += m.red0[q];
-    // zlarfg, by every thread on the same values: Hᴴ (α, x) = (β, 0), H = I − τ v vᴴ, β real
+    // the reflector, by every thread on the same values: all need u1, those
+    // of the vector phases the rest, worked out here, under the tiles' work
     const float ar = m.x1.x, ai = m.x1.y;
     float bt = ar;
     cf tau = make_float2(0.f, 0.f), scal = make_float2(1.f, 0.f), u1 = scal;
     const bool refl = !(xn == 0.f && ai == 0.f);
     if (refl) {
-      reflector(ar, ai, xn, &bt, &tau, &u1, &scal);
+      const Reflector h(ar, ai, xn);
+      u1 = h.u1(ar, ai);
+      if (own) {
+        bt = h.b;
+        tau = h.tau(ar, ai);
+        scal = inverse(u1);
+        asm volatile("" : "+f"(scal.x), "+f"(scal.y), "+f"(tau.x), "+f"(tau.y));
+      }
     }
     // A ← A − (vp wpᴴ + wp vpᴴ), A u on the tiles still in play
     float tq = 0.f;
@@ -1204,22 +1225,22 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
         cf r1[4], r2[4], r3[4], r4[4];   // −(vp), −(vp rotated), −(wp), −(wp rotated) of the rows
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-          const float4 w = m.dw[I * 32 + rg + 8 * t], v = m.dv[I * 32 + rg + 8 * t];
-          r1[t] = make_float2(-v.x, -v.z);
-          r2[t] = make_float2(-v.z, v.x);
-          r3[t] = make_float2(-w.x, -w.z);
-          r4[t] = make_float2(-w.z, w.x);
+          const float4 q = m.vw[I * 32 + rg + 8 * t];
+          r1[t] = make_float2(-q.x, -q.y);
+          r2[t] = make_float2(-q.y, q.x);
+          r3[t] = make_float2(-q.z, -q.w);
+          r4[t] = make_float2(-q.w, q.z);
         }
 #pragma unroll
         for (int u = 0; u < CU; ++u) {   // a −= vp conj(wp_j) + wp conj(vp_j)
-          const float4 w = m.dw[c0 + 4 * u], v = m.dv[c0 + 4 * u];
+          const float4 q = m.vw[c0 + 4 * u];
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
             cf e = a[t][u];
-            e = __ffma2_rn(r1[t], make_float2(w.x, w.y), e);
-            e = __ffma2_rn(r2[t], make_float2(w.z, w.w), e);
-            e = __ffma2_rn(r3[t], make_float2(v.x, v.y), e);
-            a[t][u] = __ffma2_rn(r4[t], make_float2(v.z, v.w), e);
+            e = __ffma2_rn(r1[t], make_float2(q.z, q.z), e);
+            e = __ffma2_rn(r2[t], make_float2(q.w, q.w), e);
+            e = __ffma2_rn(r3[t], make_float2(q.x, q.x), e);
+            a[t][u] = __ffma2_rn(r4[t], make_float2(q.y, q.y), e);
           }
         }
       }
@@ -1230,11 +1251,11 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
         for (int t = 0; t < 4; ++t) P[t] = Q[t] = make_float2(0.f, 0.f);
 #pragma unroll
         for (int u = 0; u < CU; ++u) {
-          const float4 v = m.sx[c0 + 4 * u];
+          const cf v = m.sx[c0 + 4 * u];
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
-            P[t] = __ffma2_rn(a[t][u], make_float2(v.x, v.y), P[t]);
-            Q[t] = __ffma2_rn(a[t][u], make_float2(v.z, v.w), Q[t]);
+            P[t] = __ffma2_rn(a[t][u], v, P[t]);
+            Q[t] = __ffma2_rn(a[t][u], make_float2(v.y, v.x), Q[t]);
           }
         }
 #pragma unroll
@@ -1272,8 +1293,7 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
       z.x += __shfl_xor_sync(0xffffffffu, o.x, 1);
       z.y += __shfl_xor_sync(0xffffffffu, o.y, 1);
       m.part[J][row] = z;
-      const float4 xr = m.sx[row];
-      const cf ur = row == k + 1 ? u1 : make_float2(xr.x, xr.y);
+      const cf ur = row == k + 1 ? u1 : m.sx[row];
       tq = warp_sum(ur.x * z.x + ur.y * z.y);   // uᴴ A u is real
     }
     if (lane == 0) m.redt[warp] = tq;
@@ -1310,8 +1330,7 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
           wpi = make_float2(ty.x - c * vi.x, ty.y - c * vi.y);
         }
       }
-      m.dv[i] = make_float4(vpi.x, vpi.x, vpi.y, vpi.y);
-      m.dw[i] = make_float4(wpi.x, wpi.x, wpi.y, wpi.y);
+      m.vw[i] = make_float4(vpi.x, vpi.y, wpi.x, wpi.y);
     }
     // what the next step's first phase reads was written before the last
     // barrier or is this thread's own
@@ -1546,7 +1565,11 @@ __global__ void __launch_bounds__(kBigT, 1) k_tri_big(EigArgs g) {
       cf tau = make_float2(0.f, 0.f), scal = make_float2(1.f, 0.f), u1 = scal;
       const bool refl = !(xn == 0.f && ai == 0.f);
       if (refl) {
-        reflector(ar, ai, xn, &bt, &tau, &u1, &scal);
+        const Reflector h(ar, ai, xn);
+        bt = h.b;
+        tau = h.tau(ar, ai);
+        u1 = h.u1(ar, ai);
+        scal = inverse(u1);
       }
       const int o = k + 1;
       if (i == o) m.p.sx[o] = make_float4(u1.x, u1.y, u1.y, u1.x);
