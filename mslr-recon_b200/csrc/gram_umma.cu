@@ -20,15 +20,27 @@
 // 8-element K step: Gram Re += Ar·Brᵀ + Ai·Biᵀ, Im += Ai·Brᵀ − Ar·Biᵀ (the
 // rebuild's signs as above).
 //
-// One CTA of 8 warps per 128 × 128 output tile.  K advances 32 elements per
-// chunk: every thread loads its share of the next chunk from global memory
-// into registers (patch element addresses from per-row / per-K offset
-// tables) while the tensor core works on the current chunk, then converts it
-// into the K-major, unswizzled core-matrix layout of a free stage (two stages,
-// 8 tiles of 8 KB each).  A stage is reused only after the tcgen05.commit of
+// One CTA of 8 warps per 128 × 128 output tile, two CTAs per SM (all of its
+// tensor memory).  K advances 16 elements per chunk: every thread loads its
+// share of the next chunk from global memory into registers (patch element
+// addresses from per-row / per-K offset tables; a diagonal Gram tile, which
+// has one operand, the next two chunks) while the tensor core works on the
+// current chunk, then converts it into the K-major, unswizzled core-matrix
+// layout of a free stage (two stages, 8 tiles of 4 KB each).  What bounds the
+// kernels is the chain load → convert → barrier → MMA of a tile and its
+// epilogue, not a pipe (LSU 47 %, issue 21 %, tensor cores below that): the
+// two CTAs run one tile's chain under the other's.  With chunks of 32 and one
+// CTA per SM, and tall rebuilds stored a row per lane (32 lines a store), 486
+// patches of 1000 × 300 took 3.34 ms to rebuild, 1.78 for their Grams and 0.60
+// for W; now 1.93, 1.42 and 0.44.  A Gram of at most 64 rows takes half of each
+// operand and half the columns of an MMA; with few patches its longer chain of
+// chunks then costs what it did (one 216 × 64: 17.4 -> 17.7 us, its rebuild
+// 12.8 -> 10.7; 240 of 343 × 50: 48 -> 31 and 65 -> 42).
+// A stage is reused only after the tcgen05.commit of
 // the MMAs that read it has arrived on the stage's mbarrier.  The epilogue
 // reads the accumulators with tcgen05.ld (warp w: TMEM lanes 32·(w mod 4),
-// columns 64·(w / 4)).  Every wait is bounded (DevWait::polls polls).  On a
+// columns 64·(w / 4)); stores along a row's columns go through shared memory so
+// that 16 lanes share a line.  Every wait is bounded (DevWait::polls polls).  On a
 // time-out the kernel stops issuing work, thread 0 waits (with the default
 // poll count) for the MMAs it has already committed, the output tile is
 // written as zeros, the tensor memory is freed and kErrMmaWait is raised in
@@ -37,6 +49,7 @@
 #include <cuda_fp16.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "internal.h"
 #include "patchmap.cuh"
@@ -47,16 +60,16 @@ namespace {
 
 constexpr int kTM = 128;          // output rows per CTA (TMEM lanes)
 constexpr int kTN = 128;          // output columns per CTA
-constexpr int kKc = 32;           // K elements per chunk
+constexpr int kKc = 16;           // K elements per chunk
 constexpr int kThr = 256;
 constexpr int kTile = kTM * kKc;  // bf16 per planar tile
-constexpr int kPairs = kTile / 2 / kThr;   // (k, k+1) pairs per thread per operand: 8
+constexpr int kPairs = kTile / 2 / kThr;   // (k, k+1) pairs per thread per operand: 4
 constexpr int kTmemCols = 256;
 
 enum { AR_H, AR_L, AI_H, AI_L, BR_H, BR_L, BI_H, BI_L, NOPS };
 
 struct USmem {
-  uint32_t op[2][NOPS][kTile / 2];   // two stages × 8 tiles of 128 × 32 bf16 (as bf16 pairs)
+  uint32_t op[2][NOPS][kTile / 2];   // two stages × 8 tiles of 128 × 16 bf16 (as bf16 pairs)
   int rowA[kTM], rowB[kTN];
   int kof[2][kKc];
   uint64_t bar[2];
@@ -69,16 +82,16 @@ __device__ __forceinline__ unsigned su32(const void* p) {
 
 // word index of the bf16 pair (r, k..k+1), k even, in a K-major unswizzled tile:
 // 8-row × 8-element core matrices of 128 bytes, k-adjacent cores 128 B apart
-// (LBO), 8-row groups 512 B apart (SBO)
+// (LBO), 8-row groups 256 B apart (SBO)
 __device__ __forceinline__ int pair_word(int r, int k) {
-  return ((r >> 3) * 4 + (k >> 3)) * 32 + (r & 7) * 4 + ((k & 7) >> 1);
+  return ((r >> 3) * 2 + (k >> 3)) * 32 + (r & 7) * 4 + ((k & 7) >> 1);
 }
 
-// shared-memory matrix descriptor (sm_100 layout): start, LBO = 128 B, SBO = 512 B,
+// shared-memory matrix descriptor (sm_100 layout): start, LBO = 128 B, SBO = 256 B,
 // version 1, no swizzle
 __device__ __forceinline__ uint64_t sdesc(const void* p) {
   const uint64_t a = su32(p);
-  return ((a >> 4) & 0x3FFFull) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(512 >> 4) << 32) |
+  return ((a >> 4) & 0x3FFFull) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(256 >> 4) << 32) |
          (1ull << 46);
 }
 
@@ -90,11 +103,12 @@ __device__ __forceinline__ uint64_t sdesc(const void* p) {
 enum Mode { kBf16 = 0, kTf32 = 1, kF16 = 2 };
 constexpr float kF16Scale = 1024.f;
 
-// instruction descriptor: BF16 × BF16 (F16 × F16) → F32, both K-major, M = 128, N = 128
+// instruction descriptor: BF16 × BF16 (F16 × F16) → F32, both K-major, M = 128; N is added by with_n
 __host__ __device__ constexpr uint32_t idesc(bool negA, bool f16 = false) {
-  return (1u << 4) | (f16 ? 0u : (1u << 7) | (1u << 10)) | ((negA ? 1u : 0u) << 13) | ((uint32_t)(kTN >> 3) << 17) |
-         ((uint32_t)(kTM >> 4) << 24);
+  return (1u << 4) | (f16 ? 0u : (1u << 7) | (1u << 10)) | ((negA ? 1u : 0u) << 13) | ((uint32_t)(kTM >> 4) << 24);
 }
+// N columns, rounded up to the 16 that M = 128 takes
+__device__ __forceinline__ uint32_t with_n(uint32_t id, int N) { return id | (uint32_t)((N + 15) >> 4 << 1) << 17; }
 
 __device__ __forceinline__ void umma(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t id, bool acc) {
   asm volatile(
@@ -170,9 +184,9 @@ __device__ __forceinline__ void split_pair_f16(float x0, float x1, uint32_t& hi,
 // TF32 operands (the TF32 form): one FP32 plane per real / imaginary part,
 // each value rounded to TF32 (to nearest, ties away), in K-major unswizzled
 // core matrices of 8 rows × 4 values (128 bytes): k-adjacent cores 128 B apart
-// (LBO), 8-row groups 1024 B apart (SBO).  A chunk of 32 K values is four
-// 8-value MMA steps.  Planes per stage: Ar, Ai, Br, Bi of 4096 words each.
-constexpr int kTfPlane = kTile;   // words per TF32 plane (128 rows × 32 values)
+// (LBO), 8-row groups 512 B apart (SBO).  A chunk of 16 K values is two
+// 8-value MMA steps.  Planes per stage: Ar, Ai, Br, Bi of 2048 words each.
+constexpr int kTfPlane = kTile;   // words per TF32 plane (128 rows × 16 values)
 
 __device__ __forceinline__ uint32_t to_tf32(float x) {
   uint32_t r;
@@ -180,17 +194,16 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
   return r;
 }
 __device__ __forceinline__ int tf_word(int r, int k) {
-  return ((r >> 3) * 8 + (k >> 2)) * 32 + (r & 7) * 4 + (k & 3);
+  return ((r >> 3) * 4 + (k >> 2)) * 32 + (r & 7) * 4 + (k & 3);
 }
 __device__ __forceinline__ uint64_t sdesc_tf(const void* p) {
   const uint64_t a = su32(p);
-  return ((a >> 4) & 0x3FFFull) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+  return ((a >> 4) & 0x3FFFull) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(512 >> 4) << 32) |
          (1ull << 46);
 }
-// instruction descriptor: TF32 × TF32 → F32, both K-major, M = 128, N = 128
+// instruction descriptor: TF32 × TF32 → F32, both K-major, M = 128; N is added by with_n
 __host__ __device__ constexpr uint32_t idesc_tf(bool negA) {
-  return (1u << 4) | (2u << 7) | (2u << 10) | ((negA ? 1u : 0u) << 13) | ((uint32_t)(kTN >> 3) << 17) |
-         ((uint32_t)(kTM >> 4) << 24);
+  return (1u << 4) | (2u << 7) | (2u << 10) | ((negA ? 1u : 0u) << 13) | ((uint32_t)(kTM >> 4) << 24);
 }
 __device__ __forceinline__ void umma_tf(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t id, bool acc) {
   asm volatile(
@@ -199,8 +212,10 @@ __device__ __forceinline__ void umma_tf(uint32_t dtmem, uint64_t a, uint64_t b, 
       "l"(a), "l"(b), "r"(id), "r"(acc ? 1u : 0u));
 }
 
-// Registers of one operand chunk: thread t holds pairs q = t + 256 i, i < 8, of
-// the 128 × 32 tile; pair q is (row r, k..k+1) of core c = q / 32.
+// Registers of one operand chunk: thread t holds pairs q = t + 256 i, i < 4, of
+// the 128 × 16 tile; pair q is (row r, k..k+1) of core c = q / 32, so pair i
+// lies in rows 32 i … 32 i + 31.  A Gram's tile of at most 64 rows takes the
+// first half only (NI = 2): what the stage holds beyond reaches no output.
 struct Chunk {
   cf v[kPairs][2];
 };
@@ -208,14 +223,15 @@ struct Chunk {
 __device__ __forceinline__ void pair_rk(int i, int& r, int& k) {
   const int q = threadIdx.x + kThr * i;
   const int c = q >> 5, w = q & 31;
-  r = (c >> 2) * 8 + (w >> 2);
-  k = (c & 3) * 8 + (w & 3) * 2;
+  r = (c >> 1) * 8 + (w >> 2);
+  k = (c & 1) * 8 + (w & 3) * 2;
 }
 
+template <int NI>
 __device__ __forceinline__ void load_chunk(Chunk& ch, const cf* __restrict__ base, const int* row,
                                            const int* kof) {
 #pragma unroll
-  for (int i = 0; i < kPairs; ++i) {
+  for (int i = 0; i < NI; ++i) {
     int r, k;
     pair_rk(i, r, k);
     const int ro = row[r];
@@ -228,11 +244,11 @@ __device__ __forceinline__ void load_chunk(Chunk& ch, const cf* __restrict__ bas
 }
 
 // chunk → planar hi / lo tiles (re_h, re_l, im_h, im_l), conjugated when conj
-template <bool F16>
+template <bool F16, int NI>
 __device__ __forceinline__ void store_chunk(const Chunk& ch, uint32_t* rh, uint32_t* rl,
                                             uint32_t* ih, uint32_t* il, bool conj) {
 #pragma unroll
-  for (int i = 0; i < kPairs; ++i) {
+  for (int i = 0; i < NI; ++i) {
     int r, k;
     pair_rk(i, r, k);
     const int w = pair_word(r, k);
@@ -251,13 +267,13 @@ __device__ __forceinline__ void store_chunk(const Chunk& ch, uint32_t* rh, uint3
 }
 
 // One operand chunk into stage `stage` (B operand when isB), conjugated when conj.
-template <int MODE>
+template <int MODE, int NI>
 __device__ __forceinline__ void store_operand(const Chunk& ch, uint32_t* stage, bool isB, bool conj) {
   if constexpr (MODE == kTf32) {
     uint32_t* re = stage + (isB ? 2 : 0) * kTfPlane;
     uint32_t* im = stage + (isB ? 3 : 1) * kTfPlane;
 #pragma unroll
-    for (int i = 0; i < kPairs; ++i) {
+    for (int i = 0; i < NI; ++i) {
       int r, k;
       pair_rk(i, r, k);
       const int w = tf_word(r, k);
@@ -267,20 +283,20 @@ __device__ __forceinline__ void store_operand(const Chunk& ch, uint32_t* stage, 
     }
   } else {
     const int o = isB ? BR_H : AR_H;
-    store_chunk<MODE == kF16>(ch, stage + (o + 0) * (kTile / 2), stage + (o + 1) * (kTile / 2),
+    store_chunk<MODE == kF16, NI>(ch, stage + (o + 0) * (kTile / 2), stage + (o + 1) * (kTile / 2),
                 stage + (o + 2) * (kTile / 2), stage + (o + 3) * (kTile / 2), conj);
   }
 }
 
-// The 12 MMAs of one 16-element K step t of stage s.
+// The 12 MMAs of stage st, one 16-element K step.
 template <bool GRAM, bool F16>
-__device__ __forceinline__ void issue_step(const USmem& s, int st, int t, uint32_t dre, uint32_t dim,
-                                           bool acc, bool bSameAsA) {
+__device__ __forceinline__ void issue_step(const USmem& s, int st, uint32_t dre, uint32_t dim, bool acc,
+                                           bool bSameAsA, int cols) {
   const uint32_t* o = &s.op[st][0][0];
-  auto A = [&](int k) { return sdesc(o + k * (kTile / 2) + t * 64); };   // +2 cores = 256 B = 64 words
+  auto A = [&](int k) { return sdesc(o + k * (kTile / 2)); };
   const int bro = bSameAsA ? AR_H : BR_H;   // B operands: same tiles as A on diagonal Gram tiles
-  auto B = [&](int k) { return sdesc(o + (bro + (k - BR_H)) * (kTile / 2) + t * 64); };
-  constexpr uint32_t P = idesc(false, F16), N = idesc(true, F16);
+  auto B = [&](int k) { return sdesc(o + (bro + (k - BR_H)) * (kTile / 2)); };
+  const uint32_t P = with_n(idesc(false, F16), cols), N = with_n(idesc(true, F16), cols);
   // real part
   umma(dre, A(AR_H), B(BR_H), P, acc);
   umma(dre, A(AR_H), B(BR_L), P, true);
@@ -309,11 +325,11 @@ __device__ __forceinline__ void issue_step(const USmem& s, int st, int t, uint32
 // All MMAs of the chunk in stage st (first: the accumulators start from zero).
 template <bool GRAM, int MODE>
 __device__ __forceinline__ void issue_chunk(const USmem& s, int st, uint32_t dre, uint32_t dim,
-                                            bool first, bool bSameAsA) {
+                                            bool first, bool bSameAsA, int cols) {
   if constexpr (MODE == kTf32) {
     const uint32_t* o = &s.op[st][0][0];
     const int br = bSameAsA ? 0 : 2, bi = bSameAsA ? 1 : 3;
-    constexpr uint32_t P = idesc_tf(false), N = idesc_tf(true);
+    const uint32_t P = with_n(idesc_tf(false), cols), N = with_n(idesc_tf(true), cols);
 #pragma unroll
     for (int t = 0; t < kKc / 8; ++t) {
       auto D = [&](int pl) { return sdesc_tf(o + pl * kTfPlane + t * 64); };   // +2 cores = 256 B
@@ -331,8 +347,7 @@ __device__ __forceinline__ void issue_chunk(const USmem& s, int st, uint32_t dre
       }
     }
   } else {
-    issue_step<GRAM, MODE == kF16>(s, st, 0, dre, dim, !first, bSameAsA);
-    issue_step<GRAM, MODE == kF16>(s, st, 1, dre, dim, true, bSameAsA);
+    issue_step<GRAM, MODE == kF16>(s, st, dre, dim, !first, bSameAsA, cols);
   }
 }
 
@@ -359,48 +374,93 @@ struct Pending {
 };
 
 // Main loop shared by both kernels: nch chunks; kofs(c, buf) fills s.kof[buf]
-// for chunk c (threads < 32); load(c, buf) loads chunk c's operands into
-// registers (A, and B unless bSameAsA); returns false when a wait timed out.
-template <bool GRAM, int MODE, class KOfs, class Load>
-__device__ __forceinline__ bool mainloop(USmem& s, int nch, Chunk& ca, Chunk& cb, bool conjA,
-                                         bool conjB, bool bSameAsA, const KOfs& kofs,
-                                         const Load& load, int polls) {
-  const int tid = threadIdx.x;
-  bool ok = true;
-  Pending pend;
-  if (nch > 0) load(0, 0);
-  for (int c = 0; c < nch; ++c) {
-    const int st = c & 1;
-    if (c + 1 < nch) kofs(c + 1, (c + 1) & 1);
-    if (c >= 2 && ok) {
-      if (mbar_wait(&s.bar[st], (unsigned)(((c - 2) >> 1) & 1), polls)) pend.observed(c - 2);
-      else ok = false;
-    }
-    if (ok) {
-      store_operand<MODE>(ca, &s.op[st][0][0], false, conjA);
-      if (!bSameAsA) store_operand<MODE>(cb, &s.op[st][0][0], true, conjB);
-    }
-    fence_async_smem();
-    __syncthreads();
-    if (c + 1 < nch) load(c + 1, (c + 1) & 1);
-    if (tid == 0 && ok) {
-      tc_fence_after();
-      issue_chunk<GRAM, MODE>(s, st, s.tmem, s.tmem + kTN, c == 0, bSameAsA);
-      umma_commit(&s.bar[st]);
-      pend.committed(c);
-    }
-    ok = __syncthreads_and(ok);
+// for chunk c (threads < kKc; chunks 0 and 1 are in place).  Returns false when
+// a wait timed out.
+//
+// One chunk of the main loop: its operands, already in registers, into stage
+// c mod 2; the loads that `next` issues run under its MMAs.
+template <bool GRAM, int MODE, class Store, class Next>
+__device__ __forceinline__ void chunk_step(USmem& s, int c, bool& ok, Pending& pend, bool bSameAsA, int cols, int polls,
+                                           const Store& store, const Next& next) {
+  const int st = c & 1;
+  if (c >= 2 && ok) {
+    if (mbar_wait(&s.bar[st], (unsigned)(((c - 2) >> 1) & 1), polls)) pend.observed(c - 2);
+    else ok = false;
   }
+  if (ok) store(&s.op[st][0][0]);
+  fence_async_smem();
+  // the only barrier of a chunk: while thread 0 issues its MMAs the others fill
+  // the other stage; s.kof's slots are rewritten two barriers after being read
+  ok = __syncthreads_and(ok);
+  next();
+  if (threadIdx.x == 0 && ok) {
+    tc_fence_after();
+    issue_chunk<GRAM, MODE>(s, st, s.tmem, s.tmem + kTN, c == 0, bSameAsA, cols);
+    umma_commit(&s.bar[st]);
+    pend.committed(c);
+  }
+}
+
+__device__ __forceinline__ bool mainloop_end(USmem& s, int nch, bool ok, Pending& pend, int polls) {
   if (nch > 0 && ok) {
     const int l = nch - 1;
     if (mbar_wait(&s.bar[l & 1], (unsigned)((l >> 1) & 1), polls)) pend.observed(l);
     else ok = false;
   }
   ok = __syncthreads_and(ok);
-  if (!ok && tid == 0) pend.drain(s);
+  if (!ok && threadIdx.x == 0) pend.drain(s);
   tc_fence_after();
   __syncthreads();
   return ok;
+}
+
+// Two operands, cols rows of B; load(c, buf) brings chunk c of both to registers.
+template <bool GRAM, int MODE, class KOfs, class Load>
+__device__ __forceinline__ bool mainloop(USmem& s, int nch, Chunk& ca, Chunk& cb, bool conjA, bool conjB,
+                                         int cols, const KOfs& kofs, const Load& load, int polls) {
+  bool ok = true;
+  Pending pend;
+  if (nch > 0) load(0, 0);
+  __syncthreads();
+  for (int c = 0; c < nch; ++c) {
+    if (c > 0 && c + 1 < nch) kofs(c + 1, (c + 1) & 1);
+    chunk_step<GRAM, MODE>(
+        s, c, ok, pend, false, cols, polls,
+        [&](uint32_t* stage) {
+          store_operand<MODE, kPairs>(ca, stage, false, conjA);
+          store_operand<MODE, kPairs>(cb, stage, true, conjB);
+        },
+        [&] {
+          if (c + 1 < nch) load(c + 1, (c + 1) & 1);
+        });
+  }
+  return mainloop_end(s, nch, ok, pend, polls);
+}
+
+// One operand on both sides (a Gram's diagonal tiles): with the registers of
+// the second, two chunks of loads are under way.  load(x, c, buf): chunk c into x.
+template <int MODE, int NI, class KOfs, class Load>
+__device__ __forceinline__ bool mainloop_same(USmem& s, int nch, Chunk& c0, Chunk& c1, bool conj, int rows,
+                                              const KOfs& kofs, const Load& load, int polls) {
+  bool ok = true;
+  Pending pend;
+  if (nch > 0) load(c0, 0, 0);
+  if (nch > 1) load(c1, 1, 1);
+  __syncthreads();
+  auto step = [&](Chunk& x, int c) {
+    if (c + 2 < nch) kofs(c + 2, c & 1);
+    chunk_step<true, MODE>(
+        s, c, ok, pend, true, rows, polls,
+        [&](uint32_t* stage) { store_operand<MODE, NI>(x, stage, false, conj); },
+        [&] {
+          if (c + 2 < nch) load(x, c + 2, c & 1);
+        });
+  };
+  for (int c = 0; c < nch; c += 2) {
+    step(c0, c);
+    if (c + 1 < nch) step(c1, c + 1);
+  }
+  return mainloop_end(s, nch, ok, pend, polls);
 }
 
 __device__ __forceinline__ void tmem_alloc(USmem& s) {
@@ -427,11 +487,30 @@ __device__ __forceinline__ void tmem_free(USmem& s) {
                  : "memory");
 }
 
+// A warp's 32 rows × 16 columns of a tile, from lane = row to 16 lanes along a
+// row and two rows per access: 16 consecutive columns leave in one store where
+// lane = row would touch 32 lines.  Uses the operand stages, which no MMA reads
+// any more; put(row, column, value) for this lane's share.
+template <class Put>
+__device__ __forceinline__ void by_columns(USmem& s, const cf (&v)[16], const Put& put) {
+  cf* t = reinterpret_cast<cf*>(&s.op[0][0][0]) + (threadIdx.x >> 5) * (32 * 17);
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 16; ++j) t[lane * 17 + j] = v[j];
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int r = 2 * i + (lane >> 4), j = lane & 15;
+    put(r, j, t[r * 17 + j]);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // kcols (or null): the patch's contraction stops at kcols[ip] values (the
 // eigenvectors beyond the rank are zero).
 template <int MODE>
-__global__ void __launch_bounds__(kThr, 1)
+__global__ void __launch_bounds__(kThr, 2)
     k_gram_umma(const cf* __restrict__ img, PatchMap m, cf* __restrict__ out, int nsplit,
                 int lchunk, const int* __restrict__ kcols, DevWait dw) {
   extern __shared__ __align__(1024) unsigned char smraw[];
@@ -465,17 +544,29 @@ __global__ void __launch_bounds__(kThr, 1)
     }
   };
   kofs(0, 0);
+  kofs(1, 1);
   __syncthreads();
   tc_fence_after();
   const cf* base = img + org;
   const bool cj = m.tall != 0;
   Chunk ca, cb;
-  auto load = [&](int c, int buf) {
-    (void)c;
-    load_chunk(ca, base, s.rowA, s.kof[buf]);
-    if (!diag) load_chunk(cb, base, s.rowB, s.kof[buf]);
-  };
-  const bool ok = mainloop<true, MODE>(s, nch, ca, cb, cj, cj, diag, kofs, load, dw.polls);
+  const int ra = min(kTM, n - a0);
+  bool ok;
+  if (diag) {
+    auto one = [&](auto ni) {
+      constexpr int NI = decltype(ni)::value;
+      return mainloop_same<MODE, NI>(
+          s, nch, ca, cb, cj, ra, kofs, [&](Chunk& x, int, int buf) { load_chunk<NI>(x, base, s.rowA, s.kof[buf]); },
+          dw.polls);
+    };
+    ok = ra <= kTM / 2 ? one(std::integral_constant<int, kPairs / 2>{}) : one(std::integral_constant<int, kPairs>{});
+  } else {
+    auto load = [&](int, int buf) {
+      load_chunk<kPairs>(ca, base, s.rowA, s.kof[buf]);
+      load_chunk<kPairs>(cb, base, s.rowB, s.kof[buf]);
+    };
+    ok = mainloop<true, MODE>(s, nch, ca, cb, cj, cj, kTN, kofs, load, dw.polls);
+  }
   cf* G = out + ((nsplit > 1) ? (int64_t)split * n * n : ip * (int64_t)n * n);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int a = a0 + (warp & 3) * 32 + lane;
@@ -494,18 +585,19 @@ __global__ void __launch_bounds__(kThr, 1)
 #pragma unroll
         for (int j = 0; j < 16; ++j) re[j] = im[j] = 0.f;
       }
-      if (a < n) {
+      constexpr float sc = MODE == kF16 ? 1.f / (kF16Scale * kF16Scale) : 1.f;
+      cf v[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int b = b0 + col + j;
-          if (b < n) {
-            constexpr float sc = MODE == kF16 ? 1.f / (kF16Scale * kF16Scale) : 1.f;
-            const cf v = make_float2(re[j] * sc, im[j] * sc);
-            G[(int64_t)b * n + a] = v;
-            if (!diag) G[(int64_t)a * n + b] = cconj(v);
-          }
-        }
+      for (int j = 0; j < 16; ++j) {
+        const int b = b0 + col + j;
+        v[j] = make_float2(re[j] * sc, im[j] * sc);
+        if (a < n && b < n) G[(int64_t)b * n + a] = v[j];
       }
+      if (!diag)
+        by_columns(s, v, [&](int r, int j, cf x) {
+          const int ar = a0 + (warp & 3) * 32 + r, b = b0 + col + j;
+          if (ar < n && b < n) G[(int64_t)ar * n + b] = cconj(x);
+        });
     }
   }
   tmem_free(s);
@@ -513,7 +605,7 @@ __global__ void __launch_bounds__(kThr, 1)
 
 // ---------------------------------------------------------------------------
 template <int MODE>
-__global__ void __launch_bounds__(kThr, 1)
+__global__ void __launch_bounds__(kThr, 2)
     k_rebuild_umma(const cf* __restrict__ img, const cf* __restrict__ W, PatchMap m,
                    cf* __restrict__ out, int direct, DevWait dw) {
   extern __shared__ __align__(1024) unsigned char smraw[];
@@ -541,6 +633,7 @@ __global__ void __launch_bounds__(kThr, 1)
     }
   };
   kofs(0, 0);
+  kofs(1, 1);
   __syncthreads();
   tc_fence_after();
   // A's element (a, b) is at Wp[a·n + b] (rows a·n in rowA, K offset b itself);
@@ -558,9 +651,9 @@ __global__ void __launch_bounds__(kThr, 1)
         ca.v[i][d] = (ro >= 0 && b < n) ? __ldg(Wp + ro + b) : make_float2(0.f, 0.f);
       }
     }
-    load_chunk(cb, img + org, s.rowB, s.kof[buf]);
+    load_chunk<kPairs>(cb, img + org, s.rowB, s.kof[buf]);
   };
-  const bool ok = mainloop<false, MODE>(s, nch, ca, cb, true, m.tall != 0, false, kofs, load, dw.polls);
+  const bool ok = mainloop<false, MODE>(s, nch, ca, cb, true, m.tall != 0, min(kTN, m.L - l0), kofs, load, dw.polls);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int a = a0 + (warp & 3) * 32 + lane;
   // on a time-out the output tile is written as zeros and the error raised
@@ -578,20 +671,26 @@ __global__ void __launch_bounds__(kThr, 1)
 #pragma unroll
         for (int j = 0; j < 16; ++j) re[j] = im[j] = 0.f;
       }
-      if (a < n) {
+      if (m.tall) {   // frame a, voxel l: conj(M_out[a][l])
+        cf v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = make_float2(re[j], -im[j]);
+        const int l = l0 + col + (lane & 15);
+        const int64_t rs = direct ? ts : (int64_t)m.p;
+        cf* o = direct ? out + org + (l < m.L ? s.rowB[col + (lane & 15)] : 0)
+                       : out + ip * m.Nt * (int64_t)m.p + l;
+        by_columns(s, v, [&](int r, int, cf x) {
+          const int f = a0 + (warp & 3) * 32 + r;
+          if (f < n && l < m.L) o[f * rs] = x;
+        });
+      } else if (a < n) {   // frame l, voxel a
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const int l = l0 + col + j;
           if (l >= m.L) continue;
-          if (m.tall) {   // frame a, voxel l: conj(M_out[a][l])
-            const cf v = make_float2(re[j], -im[j]);
-            if (direct) out[org + s.rowB[col + j] + (int64_t)a * ts] = v;
-            else out[(ip * m.Nt + a) * (int64_t)m.p + l] = v;
-          } else {        // frame l, voxel a
-            const cf v = make_float2(re[j], im[j]);
-            if (direct) out[org + offa + (int64_t)l * ts] = v;
-            else out[(ip * m.Nt + l) * (int64_t)m.p + a] = v;
-          }
+          const cf v = make_float2(re[j], im[j]);
+          if (direct) out[org + offa + (int64_t)l * ts] = v;
+          else out[(ip * m.Nt + l) * (int64_t)m.p + a] = v;
         }
       }
     }
