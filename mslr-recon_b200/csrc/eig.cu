@@ -57,7 +57,6 @@ constexpr int kT = 1024;   // most threads per CTA (one row / eigenvalue per thr
 constexpr int kSmallT = 384;   // CTA size for n <= 384: two patches share an SM
 constexpr int kNb = 16;    // reflectors per WY block
 constexpr int kCW = 16;    // eigenvectors per back-transform pass
-constexpr int kPairsMinB = 4;   // CTAs per SM of the split stage's eigenpair launch
 
 __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -1834,7 +1833,7 @@ void tri_reg_launch(const EigArgs& a, unsigned grid, cudaStream_t st) {
 // row instead of four); γ_k = d_k − λ − e_{k−1} l_{k−1} − e_k m_{k+1}, z_k = 1 at
 // the smallest |γ_k|, z_j = −l_j z_{j+1} above it and −m_j z_{j−1} below.
 // Against the quotient form with FP32 first rounds: 486 full-rank sides of 300
-// 3.60 → 1.78 ms, one of 64 87 → 32 µs, 40 of 128 493 → 170 µs.
+// 3.60 → 1.68 ms, one of 64 87 → 24 µs, 40 of 128 493 → 119 µs.
 
 // the reciprocal by two Newton steps from the hardware's approximation (|q| >= 1e-290)
 __device__ __forceinline__ double recip(double q) {
@@ -1868,9 +1867,9 @@ __device__ __forceinline__ int sturm_count(const double2* de, int n, double x) {
   return cnt;
 }
 
-// TH threads, n <= TH
-template <int TH>
-__global__ void __launch_bounds__(TH, kPairsMinB) k_pairs(EigArgs g) {
+// TH threads, n <= TH, MINB CTAs per SM
+template <int TH, int MINB>
+__global__ void __launch_bounds__(TH, MINB) k_pairs(EigArgs g) {
   extern __shared__ __align__(16) unsigned char smraw[];
   int s = 0;
   while (s + 1 < g.nseg && (int64_t)blockIdx.x >= g.seg[s + 1].first) ++s;
@@ -2110,6 +2109,23 @@ __global__ void __launch_bounds__(TH, kPairsMinB) k_pairs(EigArgs g) {
 }
 
 size_t pairs_smem(int n) { return (size_t)n * (2 + 3) * sizeof(double) + 64 * sizeof(double) + n * sizeof(float) + 16; }
+
+// A patch's chain of Sturm rounds and divisions wants no spills and threads for
+// several points per eigenvalue while patches are few; with more patches than
+// SMs, CTAs of about n threads keep more of them resident.  320 threads, two
+// CTAs per SM (96 registers, none spilled): 40 patches of 128 168 -> 119 us
+// against four CTAs (48 registers), 486 of 300 1.76 -> 1.68 ms; 160 threads, four
+// CTAs: 240 patches of 50 36 -> 30 us against that; 128 threads, eight CTAs:
+// 2250 patches of 128 0.30 -> 0.26 ms against the four (0.52 against the two).
+void pairs_launch(const EigArgs& a, int nmax, int64_t total, cudaStream_t st) {
+  constexpr int kSms = 148;
+  const size_t sm = pairs_smem(nmax);
+  const unsigned grid = (unsigned)total;
+  if (nmax <= 128 && total > 4 * kSms) k_pairs<128, 8><<<grid, 128, sm, st>>>(a);
+  else if (nmax <= 160 && total > kSms) k_pairs<160, 4><<<grid, 160, sm, st>>>(a);
+  else if (nmax <= 320) k_pairs<320, 2><<<grid, 320, sm, st>>>(a);
+  else k_pairs<kSmallT, 2><<<grid, kSmallT, sm, st>>>(a);
+}
 
 // ---- split stage, third launch: Ṽ = conj(Q Z) diag(√h) -------------------------
 // One CTA per 64 eigenvectors of a patch (32 when no more are left, or above
@@ -2460,9 +2476,7 @@ int eig_launch_group(const std::vector<const EigSegment*>& segs, const double* t
       tri_launch(one, threads == kT, st);
       if (launches) *launches += 1;
     }
-    // (486 patches of 300 are resident at once with 320 threads, and fewer threads have more registers)
-    if (nmax <= 320) k_pairs<320><<<(unsigned)total, 320, pairs_smem(nmax), st>>>(a);
-    else k_pairs<kSmallT><<<(unsigned)total, kSmallT, pairs_smem(nmax), st>>>(a);
+    pairs_launch(a, nmax, total, st);
     const bool values = segs[0]->nuc != nullptr;   // (such calls have one segment)
     if (!values)
       if (int rc = wy_apply_launch(a, nmax, total, st)) return rc;
