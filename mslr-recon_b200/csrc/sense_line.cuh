@@ -31,10 +31,13 @@ namespace line {
 // ---- launch shapes ------------------------------------------------------------
 constexpr int kColThreads = 128;
 // resident CTAs of a 128-thread column kernel: a line of N values needs 2·N
-// registers and about 8 more, of the 512 that each of an SM sub-partition's
-// 32 lanes has for its warps (one per CTA)
+// registers and about 20 more, of the 512 that each of an SM sub-partition's
+// 32 lanes has for its warps (one per CTA).  With 8 more, one CTA more was
+// resident and some of the line spilled: normal operator at 75 × 64 × 45 × 12 ×
+// 40 1.55 -> 1.43 ms, at 90 × 90 × 60 × 18 × 300 30.5 -> 30.0; with 32 or 48
+// more it is no faster or slower (1.43 / 1.50 and 30.1 / 30.1 ms).
 constexpr int col_ctas(int n) {
-  const int c = 512 / (2 * n + 8);
+  const int c = 512 / (2 * n + 20);
   return c < 1 ? 1 : c > 8 ? 8 : c;
 }
 // rows per CTA of the x pass: a shared tile of at most about 50 KB
