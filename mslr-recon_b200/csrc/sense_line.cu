@@ -202,7 +202,7 @@ PlaneOps plane_ops_of() {
 const PlaneOps* plane_ops(int nx, int ny, int nz) {
   static const PlaneOps table[] = {plane_ops_of<Plane<90, 90, 60, 1, 3>>(),
                                    plane_ops_of<Plane<48, 48, 32, 2, 5>>(),
-                                   plane_ops_of<Plane<32, 32, 24, 4, 4>>()};
+                                   plane_ops_of<Plane<32, 32, 24, 2, 8>>()};
   for (const PlaneOps& o : table)
     if (o.nx == nx && o.ny == ny && o.nz == nz) return &o;
   return nullptr;
