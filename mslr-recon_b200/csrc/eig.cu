@@ -34,7 +34,7 @@
 // Zero patches give no eigenvalue above β² and Ṽ = 0, hence W = 0 (the
 // reference's zero-norm skip, src/recon.jl:185).
 //
-// Split stage (33 <= n <= 384): three launches (two for the values alone) instead
+// Split stage (9 <= n <= 384): three launches (two for the values alone) instead
 // of one, so that each phase has the shape it needs — phase 1 and the WY
 // blocks' T factors (k_tri_reg: the matrix in registers, n <= 128; k_tri_big:
 // panels), phases 2–3 (four CTAs per SM, all patches resident at once), and
@@ -368,9 +368,16 @@ __device__ __forceinline__ int64_t upper_slot(int n, int q) {
   return (int64_t)c * n + (q - c * (c - 1) / 2);
 }
 
+// Entry (a, b), a <= b, of block blk's T factor: the blocks' upper triangles
+// packed by columns.  Only the last block may have fewer than kNb columns, so
+// all of them take n (n − 1) / 2 slots at most, what the upper triangle has.
+__device__ __forceinline__ int64_t t_slot(int n, int blk, int a, int b) {
+  return upper_slot(n, blk * (kNb * (kNb + 1) / 2) + b * (b + 1) / 2 + a);
+}
+
 // T factors (zlarft, forward columnwise) of the WY blocks of kNb reflectors,
 // taken from the last reflector down as the back-transform applies them;
-// block blk = (n − 1 − kend) / kNb goes to upper slots [256·blk, 256·blk + 256).
+// block blk = (n − 1 − kend) / kNb goes to its slots of the upper triangle.
 // sYb: n × kNb complex scratch followed by two kNb × kNb blocks.
 __device__ void wy_factors(cf* A, int n, const float* taur, const float* taui, cf* sYb, int tid, int kT) {
   cf* sT = sYb + (int64_t)n * kNb;
@@ -419,7 +426,10 @@ __device__ void wy_factors(cf* A, int n, const float* taur, const float* taui, c
       }
     }
     __syncthreads();
-    for (int t = tid; t < kNb * kNb; t += kT) A[upper_slot(n, blk * kNb * kNb + t)] = sT[t];
+    for (int t = tid; t < kNb * kNb; t += kT) {
+      const int a = t / kNb, b = t - a * kNb;
+      if (a <= b && b < nb) A[t_slot(n, blk, a, b)] = sT[t];
+    }
     __syncthreads();
   }
 }
@@ -1359,7 +1369,8 @@ __device__ __forceinline__ void wy_tfactor(cf* A, int n, int blk, const cf* tau,
   }
   if (lane < kNb) {
 #pragma unroll
-    for (int jj = 0; jj < kNb; ++jj) A[upper_slot(n, blk * kNb * kNb + lane * kNb + jj)] = t[jj];
+    for (int jj = 0; jj < kNb; ++jj)
+      if (lane <= jj && jj < nb) A[t_slot(n, blk, lane, jj)] = t[jj];
   }
 }
 // entry e of a block's G: column jj, row b < jj
@@ -1380,7 +1391,7 @@ struct TriSmem {
 };
 
 template <int NT>
-__global__ void __launch_bounds__(TriVec<NT>::kThreads, NT == 2 ? 2 : 1) k_tri_reg(EigArgs g) {
+__global__ void __launch_bounds__(TriVec<NT>::kThreads, NT == 1 ? 8 : NT == 2 ? 2 : 1) k_tri_reg(EigArgs g) {
   extern __shared__ __align__(16) unsigned char smraw[];
   TriSmem<NT>& m = *reinterpret_cast<TriSmem<NT>*>(smraw);
   int s = 0;
@@ -2177,7 +2188,11 @@ __device__ __forceinline__ void wy_stage(const cf* A, int n, int kend, cf* ys, c
       else dst[jj] = make_float2((jj < nb && row == k + 1) ? 1.f : 0.f, 0.f);
     }
   }
-  if (tid < kNb * kNb) cpa8(ts + tid, A + upper_slot(n, blk * kNb * kNb + tid));
+  if (tid < kNb * kNb) {
+    const int a = tid / kNb, b = tid - a * kNb;
+    if (a <= b && b < nb) cpa8(ts + tid, A + t_slot(n, blk, a, b));
+    else ts[tid] = make_float2(0.f, 0.f);
+  }
   cpa_commit();
 }
 
@@ -2390,17 +2405,19 @@ int eig2_prepare(int nmax) {
 
 namespace {
 
-// The split stage applies to stages with a side buffer and 33 <= n <= 384 (the
-// back-transform's register tile) whose T factors fit the upper triangle.
+// The split stage applies to stages with a side buffer and 9 <= n <= 384 (the
+// back-transform's register tile); the autotuner's 1024 threads from 33 on.
+// Sides up to 32 in three launches instead of one: the SVST of 5 matrices 118 ×
+// 22 229 → 133 µs, patchSVST of 4³ patches at stride 3 of 35 × 35 × 26 × 21 (1296
+// of side 21) 1165 → 569.  Below 9 a matrix has no more than a few steps, and no
+// room for the side values of the all-pairs mode below 6: one launch.
 // MSLR_EIG_SPLIT=0 keeps the one-launch stage everywhere (for comparisons).
 bool split_ok(const EigSegment& e) {
   static const bool off = [] {
     const char* v = std::getenv("MSLR_EIG_SPLIT");
     return v && v[0] == '0';
   }();
-  if (off || !e.side || e.n <= 32 || e.n > kSmallT) return false;
-  const int64_t nblk = (e.n - 1 + kNb - 1) / kNb;
-  return nblk * kNb * kNb <= (int64_t)e.n * (e.n - 1) / 2;
+  return !off && e.side && e.n >= (e.big ? 33 : 9) && e.n <= kSmallT;
 }
 
 int wy_apply_launch(const EigArgs& a, int nmax, int64_t total, cudaStream_t st) {
@@ -2421,6 +2438,8 @@ void tri_launch(const EigArgs& a, bool big, cudaStream_t st) {
   const unsigned grid = (unsigned)S.np;
   if (big) {
     k_eig<kT, 1, 1><<<grid, kT, vec_bytes(n) + wy_bytes(n, kT) + 128, st>>>(a);
+  } else if (n <= 32) {
+    tri_reg_launch<1>(a, grid, st);
   } else if (n <= 64) {
     tri_reg_launch<2>(a, grid, st);
   } else if (n <= 96) {
