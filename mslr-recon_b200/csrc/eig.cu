@@ -1110,6 +1110,9 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
 // tile pass (which works on the unscaled reflector u = (α − β, x), v = u / (α
 // − β), so no second round publishes v), and the partial sums of A u and of
 // uᴴ A u after it (so no third one reduces vᴴ y).
+// That sum is of the third power of the matrix, so the matrix is scaled to
+// order one first (PowerOfTwo): unscaled, in FP32, it overflowed for entries
+// from 1e11 on (n = 300) and lost its bits below 2e-13.
 // With the matrix in L2 a step cost 5.6 µs whatever n was (n = 64, one
 // patch: 351 µs), the latency of its round trips and four barriers.
 // A warp's tile column is rotated by its tile row, so that the tiles left in
@@ -1135,6 +1138,27 @@ struct TriVec {
   float red0[4], redt[NT * NTC];
   cf x1;
 };
+
+// The power of two that takes a matrix's largest diagonal entry, which bounds a
+// Gram's entries, into [1, 2), and its inverse, with which d and e are scaled
+// back; reflectors and τ do not depend on it.  As it is when the entry is zero
+// or not finite.
+struct PowerOfTwo {
+  float up;
+  double down;
+  __device__ __forceinline__ explicit PowerOfTwo(float dmax) {
+    const int ex = __float_as_int(dmax) >> 23;   // (dmax >= 0)
+    const int k = dmax > 0.f && ex < 255 ? min(max(ex, 1), 253) : 127;
+    up = __int_as_float((254 - k) << 23);
+    down = __hiloint2double((k - 127 + 1023) << 20, 0);
+  }
+};
+
+// What is left of a column below its subdiagonal (and the subdiagonal's
+// imaginary part) is dropped, the column taken as it is, when its square is
+// at most this: 1e-16 of the scaled matrix, far below FP32's rounding of it.
+// Above, neither |u₁|² nor the sums with u lose bits to denormals.
+constexpr float kNoColumn = 1e-32f;
 
 // zlarfg with α = (ar, ai) and ‖x‖² = xn: Hᴴ (α, x) = (β, 0), H = I − τ v vᴴ, β
 // real, v = (1, x / u₁), u₁ = α − β.  The root and its reciprocal come from one
@@ -1163,9 +1187,11 @@ __device__ __forceinline__ cf inverse(cf u) {
 // The n steps of the n × n Hermitian matrix at A (column stride ld, n <= 32·NT,
 // lower triangle read): d, e and τ; reflectors below A's subdiagonal and, when
 // given, in Y (unit entry and zeros included).  TriVec<NT>::kThreads threads.
-template <int NT>
+// SCALE: the matrix is scaled here (PowerOfTwo), else it has been; d and e are
+// scaled back by `down`, which SCALE sets.
+template <int NT, bool SCALE>
 __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, double* dd, double* ee, cf* taus,
-                                          cf* Y) {
+                                          cf* Y, double down) {
   constexpr int NP = 32 * NT, LD = TriVec<NT>::LD, CU = TriVec<NT>::CU, TC = TriVec<NT>::TC, NTC = TriVec<NT>::NTC;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int I = warp / NTC, J = (warp + I) % NTC;
@@ -1188,9 +1214,28 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
     }
   const int i = tid;                 // row of the vector phases
   const bool own = tid < NP;         // (the first NT warps)
+  float up = 1.f;
+  if constexpr (SCALE) {
+    if (own) {
+      float q = i < n ? fabsf(__ldcg(&A[(int64_t)i * ld + i].x)) : 0.f;
+      for (int o = 16; o > 0; o >>= 1) q = fmaxf(q, __shfl_xor_sync(0xffffffffu, q, o));
+      if (lane == 0) m.redt[warp] = q;   // (next written after the first step's barrier)
+    }
+    __syncthreads();
+    float dmax = 0.f;
+#pragma unroll
+    for (int q = 0; q < NT; ++q) dmax = fmaxf(dmax, m.redt[q]);
+    const PowerOfTwo p(dmax);
+    up = p.up;
+    down = p.down;
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int u = 0; u < CU; ++u) a[t][u] = cscale(a[t][u], up);
+  }
   if (own) {
     m.vw[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    m.scol[i] = (i < n) ? __ldcg(A + i) : make_float2(0.f, 0.f);
+    m.scol[i] = (i < n) ? cscale(__ldcg(A + i), up) : make_float2(0.f, 0.f);
   }
   const int row = I * 32 + rg + 8 * cg;   // row whose sum this lane ends with
   cf vpi = make_float2(0.f, 0.f), wpi = vpi, vpk = vpi, wpk = vpi;
@@ -1199,7 +1244,7 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
     cf x = make_float2(0.f, 0.f);
     if (own) {
       if (i >= k && i < n) x = csub(m.scol[i], cadd(cmul(vpi, cconj(wpk)), cmul(wpi, cconj(vpk))));
-      if (i == k) dd[k] = (double)x.x;
+      if (i == k) dd[k] = (double)x.x * down;
       if (i == k + 1) m.x1 = x;
       if (i <= k + 1) x = make_float2(0.f, 0.f);
       m.sx[i] = x;
@@ -1214,8 +1259,8 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
     // of the vector phases the rest, worked out here, under the tiles' work
     const float ar = m.x1.x, ai = m.x1.y;
     float bt = ar;
-    cf tau = make_float2(0.f, 0.f), scal = make_float2(1.f, 0.f), u1 = scal;
-    const bool refl = !(xn == 0.f && ai == 0.f);
+    cf tau = make_float2(0.f, 0.f), scal = tau, u1 = tau;
+    const bool refl = !(xn + ai * ai <= kNoColumn);   // (true for NaN)
     if (refl) {
       const Reflector h(ar, ai, xn);
       u1 = h.u1(ar, ai);
@@ -1323,7 +1368,7 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
       const float c = 0.5f * (tau.x * tau.x + tau.y * tau.y) * (scal.x * scal.x + scal.y * scal.y) * t;
       const cf vi = i == k + 1 ? make_float2(1.f, 0.f) : cmul(x, scal);   // 0 for i <= k and i >= n
       if (i == k + 1) {
-        ee[k] = (double)bt;
+        ee[k] = (double)bt * down;
         taus[k] = tau;
       }
       if (Y) Y[k * LD + i] = vi;
@@ -1346,7 +1391,7 @@ __device__ __forceinline__ void tri_steps(cf* A, int ld, int n, TriVec<NT>& m, d
   }
   if (own && i == n - 1) {
     const cf x = csub(m.scol[i], cadd(cmul(vpi, cconj(wpi)), cmul(wpi, cconj(vpi))));
-    dd[n - 1] = (double)x.x;
+    dd[n - 1] = (double)x.x * down;
     ee[n - 1] = 0.0;
   }
   __syncthreads();
@@ -1402,7 +1447,7 @@ __global__ void __launch_bounds__(TriVec<NT>::kThreads, NT == 1 ? 8 : NT == 2 ? 
   constexpr int kThreads = TriVec<NT>::kThreads, LD = TriVec<NT>::LD;
   const int tid = threadIdx.x, warp = tid >> 5;
   cf* A = S.gram + ip * (int64_t)n * n;
-  tri_steps<NT>(A, n, n, m.v, m.dd, m.ee, m.tau, m.Y);
+  tri_steps<NT, true>(A, n, n, m.v, m.dd, m.ee, m.tau, m.Y, 1.0);
   double* side = S.side + ip * 6 * (int64_t)n;
   for (int q = tid; q < n; q += kThreads) {
     side[q] = m.dd[q];
@@ -1449,7 +1494,8 @@ __global__ void __launch_bounds__(TriVec<NT>::kThreads, NT == 1 ? 8 : NT == 2 ? 
 // chunk) and its column (a shuffle transpose of the group's eight sums).
 // So that no value needs a test, the diagonal 64 × 64 blocks are kept with
 // zeros above the diagonal and half the diagonal (each half counts once in the
-// row's and once in the column's sum).
+// row's and once in the column's sum).  The matrix is scaled as tri_steps does
+// it: by the first panel as it reads, by its update for good.
 // Each warp takes an equal share of the groups, chunk by chunk, and every
 // partial sum has its own slot, added up in a fixed order.  One 512-thread CTA
 // per SM, so that the working set, 148 triangles, stays in L2.
@@ -1532,12 +1578,22 @@ __global__ void __launch_bounds__(kBigT, 1) k_tri_big(EigArgs g) {
   cf* A = S.gram + ip * (int64_t)n * n;
   const int i = tid;   // row of the vector phases
   const int nchunk = (n + 63) >> 6;
+  float dmax = 0.f;   // (lane 0)
   for (int c = warp; c < n; c += kBigW) {   // the diagonal blocks (see above)
     cf* col = A + (int64_t)c * n;
     for (int r = (c & ~63) + lane; r < c; r += 32) col[r] = make_float2(0.f, 0.f);
-    if (lane == 0) col[c] = make_float2(0.5f * __ldcg(&col[c].x), 0.f);
+    if (lane == 0) {
+      const float d = __ldcg(&col[c].x);
+      dmax = fmaxf(dmax, fabsf(d));
+      col[c] = make_float2(0.5f * d, 0.f);
+    }
   }
+  if (lane == 0) m.p.redt[warp] = dmax;   // (next written after the first column's barriers)
   __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kBigW; ++q) dmax = fmaxf(dmax, m.p.redt[q]);
+  const PowerOfTwo pw(dmax);
+  float up = pw.up;   // of the matrix in memory: 1 from the first update on
   int k = 0;
   while (n - k > kTail) {
     const int p0 = k, pe = min(p0 + kPb, n - kTail);   // this panel's columns
@@ -1547,7 +1603,7 @@ __global__ void __launch_bounds__(kBigT, 1) k_tri_big(EigArgs g) {
       // column k with the panel's updates so far
       cf x = make_float2(0.f, 0.f);
       if (i >= k && i < n) {
-        x = xraw;
+        x = cscale(xraw, up);
         if (i == k) x.x *= 2.f;
 #pragma unroll 4
         for (int p = 0; p < np; ++p) {
@@ -1557,7 +1613,7 @@ __global__ void __launch_bounds__(kBigT, 1) k_tri_big(EigArgs g) {
         }
       }
       if (k + 1 < pe && i > k && i < n) xraw = __ldcg(A + (int64_t)(k + 1) * n + i);   // the next column
-      if (i == k) m.dd[k] = (double)x.x;
+      if (i == k) m.dd[k] = (double)x.x * pw.down;
       if (i == k + 1) m.p.x1 = x;
       if (i <= k + 1) x = make_float2(0.f, 0.f);
       if (i < kSmallT) m.p.sx[i] = make_float4(x.x, x.y, x.y, x.x);
@@ -1572,8 +1628,8 @@ __global__ void __launch_bounds__(kBigT, 1) k_tri_big(EigArgs g) {
       // zlarfg as in tri_steps: u = (α − β, x), v = scal · u
       const float ar = m.p.x1.x, ai = m.p.x1.y;
       float bt = ar;
-      cf tau = make_float2(0.f, 0.f), scal = make_float2(1.f, 0.f), u1 = scal;
-      const bool refl = !(xn == 0.f && ai == 0.f);
+      cf tau = make_float2(0.f, 0.f), scal = tau, u1 = tau;
+      const bool refl = !(xn + ai * ai <= kNoColumn);   // (true for NaN)
       if (refl) {
         const Reflector h(ar, ai, xn);
         bt = h.b;
@@ -1621,7 +1677,8 @@ __global__ void __launch_bounds__(kBigT, 1) k_tri_big(EigArgs g) {
         }
         auto flush = [&]() {
           if (cur < 0) return;
-          const cf y0 = make_float2(P0.x - P0.y, Q0.x + Q0.y), y1 = make_float2(P1.x - P1.y, Q1.x + Q1.y);
+          const cf y0 = make_float2((P0.x - P0.y) * up, (Q0.x + Q0.y) * up);
+          const cf y1 = make_float2((P1.x - P1.y) * up, (Q1.x + Q1.y) * up);
           *reinterpret_cast<float4*>(&m.p.rowp[cur][warp][2 * lane]) = make_float4(y0.x, y0.y, y1.x, y1.y);
           tq += u0.x * y0.x + u0.y * y0.y + uu.x * y1.x + uu.y * y1.y;
         };
@@ -1662,9 +1719,10 @@ __global__ void __launch_bounds__(kBigT, 1) k_tri_big(EigArgs g) {
           col_sums(cr, ci, lane);
           if ((lane & 3) == 0) {
             const int c = c0 + (lane >> 2);
-            m.p.colp[q][c] = make_float2(cr[0], ci[0]);
+            const cf y = make_float2(cr[0] * up, ci[0] * up);
+            m.p.colp[q][c] = y;
             const float4 v = m.p.sx[c];
-            tq += v.x * cr[0] + v.y * ci[0];
+            tq += v.x * y.x + v.y * y.y;
           }
           q = nq;
           c0 = nc0;
@@ -1701,7 +1759,7 @@ __global__ void __launch_bounds__(kBigT, 1) k_tri_big(EigArgs g) {
           }
           vi = i == o ? make_float2(1.f, 0.f) : cmul(x, scal);
           if (i == o) {
-            m.ee[k] = (double)bt;
+            m.ee[k] = (double)bt * pw.down;
             m.tau[k] = tau;
           } else {
             A[(int64_t)k * n + i] = vi;   // reflector kept below the subdiagonal
@@ -1729,6 +1787,11 @@ __global__ void __launch_bounds__(kBigT, 1) k_tri_big(EigArgs g) {
         cf a0[8], a1[8];
 #pragma unroll
         for (int b = 0; b < 8; ++b) load2<EVEN>(&a0[b], &a1[b], A + (int64_t)min(c0 + b, n - 1) * n, r, n);
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+          a0[b] = cscale(a0[b], up);
+          a1[b] = cscale(a1[b], up);
+        }
         if (c0 + 8 > 64 * it.q) {   // the whole diagonal
 #pragma unroll
           for (int b = 0; b < 8; ++b) {
@@ -1773,9 +1836,10 @@ __global__ void __launch_bounds__(kBigT, 1) k_tri_big(EigArgs g) {
         }
       }
     }
+    up = 1.f;
     __syncthreads();
   }
-  tri_steps<4>(A + (int64_t)k * n + k, n, n - k, m.t, m.dd + k, m.ee + k, m.tau + k, nullptr);
+  tri_steps<4, false>(A + (int64_t)k * n + k, n, n - k, m.t, m.dd + k, m.ee + k, m.tau + k, nullptr, pw.down);
   double* side = S.side + ip * 6 * (int64_t)n;
   for (int q = tid; q < n; q += kBigT) {
     side[q] = m.dd[q];
