@@ -1971,10 +1971,12 @@ __global__ void __launch_bounds__(TH, MINB) k_pairs(EigArgs g) {
     ee[q] = side[n + q];
   }
   __syncthreads();
-  // Gershgorin's interval
+  // Gershgorin's interval; fmin and fmax pass a NaN by, so it is looked for by itself
   double gl = 1e300, gu = -1e300;
+  bool bad = false;
   for (int q = tid; q < n; q += kThr) {
     const double rr = (q > 0 ? fabs(ee[q - 1]) : 0.0) + (q < n - 1 ? fabs(ee[q]) : 0.0);
+    bad = bad || !(fabs(dd[q]) + rr < 1e300);
     gl = fmin(gl, dd[q] - rr);
     gu = fmax(gu, dd[q] + rr);
   }
@@ -1986,13 +1988,29 @@ __global__ void __launch_bounds__(TH, MINB) k_pairs(EigArgs g) {
     redd[warp] = gl;
     redd[32 + warp] = gu;
   }
-  __syncthreads();
+  if (__syncthreads_or(bad)) {
+    // a NaN or Inf among the patch's values: all eigenpairs, NaN, so that the
+    // patch comes out NaN and not as the zeros of an empty spectrum
+    const float nan = __int_as_float(0x7fc00000);
+    if (tid == 0) {
+      S.rank[ip] = n;
+      if (S.nuc) S.nuc[ip] = nan;
+    }
+    if (S.nuc) return;
+    for (int q = tid; q < n * n; q += kThr) Z[q] = make_float2(nan, nan);
+    for (int q = tid; q < n; q += kThr) {
+      side[3 * n + q] = nan;
+      reinterpret_cast<float*>(side + 4 * (int64_t)n)[q] = 1.f;
+      if (full) S.lam_out[ip * n + q] = nan;
+    }
+    return;
+  }
   for (int w = 0; w < kThr / 32; ++w) {
     gl = fmin(gl, redd[w]);
     gu = fmax(gu, redd[32 + w]);
   }
   const double tnorm = fmax(fabs(gl), fabs(gu));
-  // power of two with norm · sc in [1/2, 1) (1 for a zero or non-finite T)
+  // power of two with norm · sc in [1/2, 1) (1 for a zero T)
   const int tex = (__double2hiint(tnorm) >> 20) & 0x7ff;
   const bool sane = tex > 64 && tex < 1983;
   const double sc = sane ? __hiloint2double((2045 - tex) << 20, 0) : 1.0;
