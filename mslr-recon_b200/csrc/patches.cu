@@ -170,12 +170,13 @@ int geom_build(const int N[3], int Nt, const int ps_in[3], const int ss_in[3], S
       return fail(MSLR_ERR_ARG, "patch sizes and strides must be positive");
     g->ps[d] = std::min(ps_in[d], N[d]);
     g->ss[d] = ss_in[d];
-    const int num = N[d] - g->ps[d];
-    g->nsteps[d] = (num + g->ss[d] - 1) / g->ss[d];   // cld for num >= 0
+    // 64-bit: a stride may be anything up to 2^31 - 1
+    const int64_t num = N[d] - g->ps[d], ss = g->ss[d];
+    g->nsteps[d] = (int)((num + ss - 1) / ss);   // cld for num >= 0
     Np *= (g->nsteps[d] + 1);
     int prev = -1;
     for (int i = 0; i <= g->nsteps[d]; ++i) {
-      const int s = std::min(i * g->ss[d], N[d] - g->ps[d]);
+      const int s = (int)std::min(i * ss, num);
       g->h_starts.push_back(s);
       if (i == 0 && s != 0) partition = false;
       if (i > 0 && s - prev != g->ps[d]) partition = false;

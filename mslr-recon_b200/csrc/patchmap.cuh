@@ -23,7 +23,10 @@ struct PatchMap {
 };
 
 // Start of the i-th of an axis's patches: the last one ends with the axis.
-__device__ __forceinline__ int patch_start(int i, int ss, int n, int ps) { return min(i * ss, n - ps); }
+// Unsigned: the last one's i·ss is below (n − ps) + ss, which may pass 2^31.
+__device__ __forceinline__ int patch_start(int i, int ss, int n, int ps) {
+  return (int)min((unsigned)i * (unsigned)ss, (unsigned)(n - ps));
+}
 
 __device__ __forceinline__ int64_t patch_origin(const PatchMap& m, int64_t ip) {
   if (m.batch) return ip * m.mstride;
