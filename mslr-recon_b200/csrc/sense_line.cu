@@ -570,7 +570,15 @@ int sense_line_bind(Ctx* c, cudaStream_t st) {
 int normal_op_line(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool subtract, cudaStream_t st) {
   const float scale = (float)(1.0 / (double)c->nvox);
   const cf* xs = X;
-  if (ns > 1) {
+  // One image is read where it is, unless the result lies over it and a second
+  // coil group would read what the first has written (with one group, a chunk's
+  // frames are read before they are written, and by no other chunk).
+  int ch, fr;
+  bool lanes;
+  chunk_of(c, &ch, &fr, &lanes);
+  const int64_t series = (int64_t)c->Nt * c->nvox;
+  const bool over = X < g + series && g < X + series;
+  if (ns > 1 || (over && (ch < c->Nc || g != X))) {
     if (int rc = image_sum(c, X, ns, sstride, c->d_xsum, st)) return rc;
     xs = c->d_xsum;
   }
