@@ -2429,16 +2429,18 @@ __device__ __forceinline__ void wy_apply_body(const Seg& S, const cf* A, cf* Z, 
   }
 }
 
-// blockIdx.x: group of 32·NV columns
+// One block per patch and group of 32·NV columns, the groups of a patch in a
+// row; one grid dimension, since all scales' patches may pass 65 535
 template <int RPW, int NV>
-__global__ void __launch_bounds__(kWyThreads, 1) k_wy_apply(EigArgs g) {
+__global__ void __launch_bounds__(kWyThreads, 1) k_wy_apply(EigArgs g, int groups) {
   extern __shared__ __align__(16) unsigned char smraw[];
+  const int64_t patch = blockIdx.x / groups;
   int s = 0;
-  while (s + 1 < g.nseg && (int64_t)blockIdx.y >= g.seg[s + 1].first) ++s;
+  while (s + 1 < g.nseg && patch >= g.seg[s + 1].first) ++s;
   const Seg& S = g.seg[s];
   const int n = S.n;
-  const int64_t ip = (int64_t)blockIdx.y - S.first;
-  const int cb = blockIdx.x * 32 * NV;
+  const int64_t ip = patch - S.first;
+  const int cb = (int)(blockIdx.x - patch * groups) * 32 * NV;
   if (cb >= n) return;   // the grid covers the launch's largest n
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const cf* A = S.gram + ip * (int64_t)n * n;
@@ -2504,10 +2506,11 @@ bool split_ok(const EigSegment& e) {
 
 int wy_apply_launch(const EigArgs& a, int nmax, int64_t total, cudaStream_t st) {
   const int rpw = (nmax + 15) / 16, cols = rpw <= 20 ? 64 : 32;   // columns per CTA
-  const dim3 grid((unsigned)((nmax + cols - 1) / cols), (unsigned)total);
+  int groups = (nmax + cols - 1) / cols;
   EigArgs arg = a;
-  void* args[] = {&arg};
-  MSLR_CUDA_TRY(cudaLaunchKernel(wy_kernel(rpw), grid, dim3(kWyThreads), args, wy_apply_smem(nmax), st));
+  void* args[] = {&arg, &groups};
+  MSLR_CUDA_TRY(cudaLaunchKernel(wy_kernel(rpw), dim3((unsigned)(total * groups)), dim3(kWyThreads), args,
+                                 wy_apply_smem(nmax), st));
   return MSLR_OK;
 }
 
