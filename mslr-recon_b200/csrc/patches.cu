@@ -52,11 +52,11 @@ __device__ __forceinline__ Cover cover_of(const PatchMap& m, int64_t v) {
 }
 
 // img2patches: P[(ip*Nt + t)*p + l] = img[t][vox(ip, l)].
-// grid (Np · ceil(p / threads), groups of frames)
+// grid (Np · ceil(p / threads), groups of frames), from block `first` on
 __global__ void __launch_bounds__(256) k_img2patches(const cf* __restrict__ img, const PatchMap m,
-                                                     cf* __restrict__ P, int lblocks) {
-  const int64_t ip = blockIdx.x / lblocks;
-  const int l = (int)(blockIdx.x - ip * lblocks) * blockDim.x + threadIdx.x;
+                                                     cf* __restrict__ P, int lblocks, int64_t first) {
+  const int64_t b = first + blockIdx.x, ip = b / lblocks;
+  const int l = (int)(b - ip * lblocks) * blockDim.x + threadIdx.x;
   if (l >= m.p) return;
   const cf* src = img + patch_origin(m, ip) + patch_off(m, l);
   cf* dst = P + ip * m.Nt * (int64_t)m.p + l;
@@ -137,8 +137,12 @@ dim3 voxel_grid(const PatchMap& m) { return dim3((unsigned)((m.nvox + 255) / 256
 int img2patches_launch(const cf* img, const PatchMap& m, int64_t np, cf* P, cudaStream_t st) {
   const int thr = std::min(256, (m.p + 31) / 32 * 32);
   const int lblocks = (m.p + thr - 1) / thr;
-  k_img2patches<<<dim3((unsigned)(np * lblocks), frame_groups(m)), thr, 0, st>>>(img, m, P, lblocks);
-  MSLR_CUDA_TRY(cudaGetLastError());
+  const int64_t blocks = np * lblocks, most = 0x7fffffff;   // what the grid's first dimension holds
+  for (int64_t b = 0; b < blocks; b += most) {
+    const dim3 grid((unsigned)std::min(blocks - b, most), frame_groups(m));
+    k_img2patches<<<grid, thr, 0, st>>>(img, m, P, lblocks, b);
+    MSLR_CUDA_TRY(cudaGetLastError());
+  }
   return MSLR_OK;
 }
 

@@ -1,5 +1,6 @@
-"""More patches than a grid's second dimension holds: two overlapping scales
-whose patches run through one eigen stage, 115 520 in all."""
+"""More patches than a dimension of a grid holds: two overlapping scales whose
+patches run through one eigen stage, 115 520 in all, and more than 2^31 patches
+of one voxel."""
 import numpy as np
 import pytest
 
@@ -28,3 +29,15 @@ def test_two_overlapping_scales():
     want = torch.linalg.vector_norm(out["plain"])
     assert float(want) > 0.0
     assert float(torch.linalg.vector_norm(out["tuned"] - out["plain"])) <= 9.2e-5 * float(want)
+
+
+def test_more_than_2_31_patches():
+    import torch
+    from mslr_recon_b200 import recon as R
+    Nx, Ny, Nz = 2048, 1024, 1025
+    img = torch.empty((1, Nz, Ny, Nx), dtype=torch.complex64, device="cuda")
+    v = torch.view_as_real(img)
+    v[..., 0] = torch.arange(Nx, device="cuda") + 3.0 * torch.arange(Ny, device="cuda")[:, None]
+    v[..., 1] = torch.arange(Nz, device="cuda")[:, None, None]
+    P = R.img2patches(img, (1, 1, 1), (1, 1, 1))
+    assert torch.equal(P.view(-1), img.view(-1))
