@@ -373,8 +373,8 @@ int sense_bind(Ctx* c, const cf* smaps, const cf* y, const int32_t* idx, int bas
   k_modmaps<<<1184, 256, 0, st>>>(smaps, c->d_smaps_mod, c->d_mod[0], c->d_mod[1], c->d_mod[2], d);
   MSLR_CUDA_TRY(cudaGetLastError());
   c->bound = true;
-  if (c->line && (rc = sense_line_bind(c, st))) return rc;
-  rc = sense_adjoint(c, y, c->d_ahy, st);
+  rc = c->line ? sense_line_bind(c, st) : MSLR_OK;
+  if (!rc) rc = sense_adjoint(c, y, c->d_ahy, st);
   if (!rc) rc = data_norm2(c, y, &c->ynorm2, st);   // ‖y‖² for dc_cost (cost.cu)
   if (rc) {
     c->bound = false;

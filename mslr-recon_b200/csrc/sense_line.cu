@@ -298,18 +298,19 @@ const void* coil_sum_kernel(int ch, bool pairs) { return pairs ? coil_sum_of<2>(
 // mz[(t·NW + q)·PL + i]: bit z − 32q set when (z, i) is sampled in frame t, i the
 // position within a plane of T (turned: kx·Ny + ky, else ky·Nx + kx)
 __global__ void k_mask_z(const uint32_t* __restrict__ mask, int nwords, uint32_t* __restrict__ mz,
-                         int nx, int ny, int turned, int nz, int nw) {
-  const int t = blockIdx.z, q = blockIdx.y;
-  const int pl = nx * ny;
-  const uint32_t* m = mask + (int64_t)t * nwords;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < pl; i += gridDim.x * blockDim.x) {
-    uint32_t w = 0;
-    const int j = turned ? (i % nx) * ny + i / nx : i;
-    for (int z = 32 * q; z < min(nz, 32 * q + 32); ++z) {
-      const int64_t k = (int64_t)z * pl + i;
-      w |= ((__ldg(m + (k >> 5)) >> (k & 31)) & 1u) << (z - 32 * q);
+                         int nx, int ny, int turned, int nz, int nw, int nt) {
+  const int q = blockIdx.y, pl = nx * ny;
+  for (int t = blockIdx.z; t < nt; t += gridDim.z) {
+    const uint32_t* m = mask + (int64_t)t * nwords;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < pl; i += gridDim.x * blockDim.x) {
+      uint32_t w = 0;
+      const int j = turned ? (i % nx) * ny + i / nx : i;
+      for (int z = 32 * q; z < min(nz, 32 * q + 32); ++z) {
+        const int64_t k = (int64_t)z * pl + i;
+        w |= ((__ldg(m + (k >> 5)) >> (k & 31)) & 1u) << (z - 32 * q);
+      }
+      mz[((int64_t)t * nw + q) * pl + j] = w;
     }
-    mz[((int64_t)t * nw + q) * pl + j] = w;
   }
 }
 
@@ -561,8 +562,9 @@ bool sense_line_setup(Ctx* c) {
 
 int sense_line_bind(Ctx* c, cudaStream_t st) {
   const int pl = c->N[0] * c->N[1], nw = (c->N[2] + 31) / 32;
-  k_mask_z<<<dim3((pl + 255) / 256, nw, c->Nt), 256, 0, st>>>(c->d_mask, c->nwords, c->d_mz, c->N[0], c->N[1],
-                                                               plane_ops(c->N[0], c->N[1], c->N[2]) != nullptr, c->N[2], nw);
+  const dim3 grid((pl + 255) / 256, nw, std::min(c->Nt, 65535));
+  k_mask_z<<<grid, 256, 0, st>>>(c->d_mask, c->nwords, c->d_mz, c->N[0], c->N[1],
+                                 plane_ops(c->N[0], c->N[1], c->N[2]) != nullptr, c->N[2], nw, c->Nt);
   MSLR_CUDA_TRY(cudaGetLastError());
   return MSLR_OK;
 }
