@@ -884,7 +884,9 @@ int normal_op_spec(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool sub
 // (register-line form) one or two lanes of chunks, timed on the bound context
 // (A'A applied to A'y).  Larger chunks mean fewer launches; the chunk's
 // k-space should stay in L2.  The three-kernel form's clusters hold one coil
-// per CTA, so groups have at most eight coils.
+// per CTA, so its groups have at most eight coils.  The shape that the context
+// has is timed first: its groups of equal size may have 5 or 7 coils, which the
+// list has not (75 × 64 × 45, 5 coils: 0.33 ms, in groups of 3 and 2 0.36).
 int tune_sense_chunks(Ctx* c, cudaStream_t st) {
   const bool three = c->spec && (c->spec_three || c->xy_tc);
   if (!three && !c->line) return MSLR_OK;
@@ -892,30 +894,35 @@ int tune_sense_chunks(Ctx* c, cudaStream_t st) {
   const int max_lanes = !three && c->sn_stream ? 2 : 1;
   float best = 1e30f;
   int bch = c->spec_ch, bfr = c->spec_fr, bl = c->spec_lanes;
-  for (int ch : {2, 3, 4, 6, 8}) {
-    if (ch > c->Nc) continue;
-    for (int fr = 1; fr <= 4; ++fr) {
-      if ((int64_t)fr * ch > (int64_t)c->F * c->Nc || fr > c->Nt || fr * ch > 24) continue;
-      c->spec_ch = ch;
-      c->spec_fr = fr;
-      for (int lanes = 1; lanes <= max_lanes; ++lanes) {
-        if (!three) c->spec_lanes = lanes;
-        float ms = 0.f;
-        int rc = time_ms(st, 2, &ms, [&] { return normal_op(c, c->d_ahy, 1, E, c->d_G, false, st); });
-        if (rc) return rc;
-        if (ms < best) {
-          best = ms;
-          bch = ch;
-          bfr = fr;
-          bl = c->spec_lanes;
-        }
+  auto time_shape = [&](int ch, int fr) {
+    c->spec_ch = ch;
+    c->spec_fr = fr;
+    for (int lanes = 1; lanes <= max_lanes; ++lanes) {
+      if (!three) c->spec_lanes = lanes;
+      float ms = 0.f;
+      const int rc = time_ms(st, 2, &ms, [&] { return normal_op(c, c->d_ahy, 1, E, c->d_G, false, st); });
+      if (rc) return rc;
+      if (ms < best) {
+        best = ms;
+        bch = ch;
+        bfr = fr;
+        bl = c->spec_lanes;
       }
+    }
+    return (int)MSLR_OK;
+  };
+  int rc = time_shape(bch, bfr);
+  for (int ch : {2, 3, 4, 6, 8, 9, 12, 18}) {
+    if (ch > c->Nc || (three && ch > 8)) continue;
+    for (int fr = 1; fr <= 4 && !rc; ++fr) {
+      if ((int64_t)fr * ch > (int64_t)c->F * c->Nc || fr > c->Nt || fr * ch > 24) continue;
+      rc = time_shape(ch, fr);
     }
   }
   c->spec_ch = bch;
   c->spec_fr = bfr;
   c->spec_lanes = bl;
-  return MSLR_OK;
+  return rc;
 }
 
 int autotune(Ctx* c, cudaStream_t st) {
