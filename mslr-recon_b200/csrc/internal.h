@@ -99,7 +99,7 @@ struct Ctx {
   int spec_lanes = 1;
   cudaStream_t sn_stream = nullptr;
   cudaEvent_t sn_fork = nullptr, sn_join = nullptr;
-  cf* d_xsum = nullptr;   // (Nt, nvox) summed image Σ_k X_k
+  cf* d_xsum = nullptr;   // (Nt, nvox) summed image Σ_k X_k, when first needed
   // register-line SENSE kernels (sense_line.cu): every axis a 5-smooth length of 8..96
   bool line = false;
   uint32_t* d_mz = nullptr;   // sample bits over z: (Nt, ⌈Nz/32⌉, Ny·Nx)
@@ -200,6 +200,9 @@ int normal_op_spec(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool sub
 // ---- sense_line.cu (tuned form, 5-smooth axes) -------------------------------------
 bool sense_line_setup(Ctx* c);
 int sense_line_bind(Ctx* c, cudaStream_t st);
+// Whether normal_op_line can take the call: false when there is no memory for
+// the summed image.
+int normal_op_line_ready(Ctx* c, const cf* X, int ns, const cf* g, bool* ready);
 int normal_op_line(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool subtract,
                    cudaStream_t st);
 int sense_forward_line(Ctx* c, const cf* x, cf* y, cudaStream_t st);

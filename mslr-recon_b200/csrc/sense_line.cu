@@ -516,6 +516,30 @@ int for_chunks(Ctx* c, cudaStream_t st, Fn&& fn) {
   return MSLR_OK;
 }
 
+// Whether the normal operator reads a copy or the sum of its images.  One image
+// is read where it is, unless the result lies over it and a second coil group
+// would read what the first has written (with one group, a chunk's frames are
+// read before they are written, and by no other chunk).
+bool needs_sum(const Ctx* c, const cf* X, int ns, const cf* g) {
+  if (ns > 1) return true;
+  int ch, fr;
+  bool lanes;
+  chunk_of(c, &ch, &fr, &lanes);
+  const int64_t series = (int64_t)c->Nt * c->nvox;
+  return X < g + series && g < X + series && (ch < c->Nc || g != X);
+}
+
+// The buffer for it, a whole image series, made when first needed (by a
+// context of several scales when it is bound); a stream may be capturing.
+int sum_buffer(Ctx* c) {
+  if (c->d_xsum) return MSLR_OK;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  MSLR_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+  const int rc = dalloc(c, (void**)&c->d_xsum, (size_t)c->Nt * c->nvox * sizeof(cf));
+  MSLR_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+  return rc;
+}
+
 }  // namespace
 
 bool sense_line_setup(Ctx* c) {
@@ -539,8 +563,7 @@ bool sense_line_setup(Ctx* c) {
   if (!cudaGetDevice(&dev) && !cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) && nsm > 0)
     c->nsm = nsm;
   const int nw = (c->N[2] + 31) / 32;
-  if (dalloc(c, (void**)&c->d_mz, (size_t)c->Nt * nw * c->N[0] * c->N[1] * sizeof(uint32_t)) ||
-      (!c->d_xsum && dalloc(c, (void**)&c->d_xsum, (size_t)c->Nt * c->nvox * sizeof(cf)))) {
+  if (dalloc(c, (void**)&c->d_mz, (size_t)c->Nt * nw * c->N[0] * c->N[1] * sizeof(uint32_t))) {
     cudaGetLastError();
     return false;
   }
@@ -566,21 +589,24 @@ int sense_line_bind(Ctx* c, cudaStream_t st) {
   k_mask_z<<<grid, 256, 0, st>>>(c->d_mask, c->nwords, c->d_mz, c->N[0], c->N[1],
                                  plane_ops(c->N[0], c->N[1], c->N[2]) != nullptr, c->N[2], nw, c->Nt);
   MSLR_CUDA_TRY(cudaGetLastError());
+  // what every iteration over several scales needs; without it they go another way
+  if (c->Ns > 1 && sum_buffer(c)) cudaGetLastError();
+  return MSLR_OK;
+}
+
+int normal_op_line_ready(Ctx* c, const cf* X, int ns, const cf* g, bool* ready) {
+  *ready = true;
+  if (!needs_sum(c, X, ns, g) || !sum_buffer(c)) return MSLR_OK;
+  cudaGetLastError();
+  if (ns == 1) return MSLR_ERR_NOMEM;   // (the other forms can't write over their input either)
+  *ready = false;
   return MSLR_OK;
 }
 
 int normal_op_line(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool subtract, cudaStream_t st) {
   const float scale = (float)(1.0 / (double)c->nvox);
   const cf* xs = X;
-  // One image is read where it is, unless the result lies over it and a second
-  // coil group would read what the first has written (with one group, a chunk's
-  // frames are read before they are written, and by no other chunk).
-  int ch, fr;
-  bool lanes;
-  chunk_of(c, &ch, &fr, &lanes);
-  const int64_t series = (int64_t)c->Nt * c->nvox;
-  const bool over = X < g + series && g < X + series;
-  if (ns > 1 || (over && (ch < c->Nc || g != X))) {
+  if (needs_sum(c, X, ns, g)) {
     if (int rc = image_sum(c, X, ns, sstride, c->d_xsum, st)) return rc;
     xs = c->d_xsum;
   }

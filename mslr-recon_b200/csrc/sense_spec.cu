@@ -807,11 +807,10 @@ int normal_op_spec(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool sub
                    cudaStream_t st) {
   const SpecOps* o = find_ops(c->N[0], c->N[1], c->N[2]);
   if (!o) return fail(MSLR_ERR_UNSUPPORTED, "no specialised SENSE kernels for this shape");
-  if (c->line && !c->spec_three && !c->xy_tc) return normal_op_line(c, X, ns, sstride, g, subtract, st);
   c->prof_kernels = 3;
   float scale = (float)(1.0 / (double)c->nvox);
   const int Nc = c->Nc, Ny = c->N[1], Nz = c->N[2];
-  const int Ch = std::max(1, std::min(Nc, c->spec_ch));             // coils per group
+  const int Ch = std::max(1, std::min(std::min(Nc, c->spec_ch), 8));   // coils per group, a cluster
   int F = std::max(1, c->spec_fr);                                  // frames per chunk
   while (F > 1 && (int64_t)F * Ch > (int64_t)c->F * Nc) --F;        // within the k-space buffer
   int nwords = c->nwords;
