@@ -225,15 +225,18 @@ const LineOps* line_ops(int n) {
 template <int VEC> struct Vals;
 template <> struct Vals<1> { using type = float2; };
 template <> struct Vals<2> { using type = float4; };
-__device__ __forceinline__ void mac_c(float2& a, const float2 s, const float2 v) {   // a += conj(s)·v
-  a.x = fmaf(s.x, v.x, fmaf(s.y, v.y, a.x));
-  a.y = fmaf(s.x, v.y, fmaf(-s.y, v.x, a.y));
+// a += conj(s)·v, the product formed first: the running sum is then rounded once
+// a coil and not twice (normal operator at 32 × 32 × 24 × 8 × 64: 1.49e-6 -> 1.40e-6
+// against 64 bits, 0.2 to 0.5 % of its time)
+__device__ __forceinline__ void mac_c(float2& a, const float2 s, const float2 v) {
+  a.x += fmaf(s.x, v.x, s.y * v.y);
+  a.y += fmaf(s.x, v.y, -(s.y * v.x));
 }
 __device__ __forceinline__ void mac_c(float4& a, const float4 s, const float4 v) {
-  a.x = fmaf(s.x, v.x, fmaf(s.y, v.y, a.x));
-  a.y = fmaf(s.x, v.y, fmaf(-s.y, v.x, a.y));
-  a.z = fmaf(s.z, v.z, fmaf(s.w, v.w, a.z));
-  a.w = fmaf(s.z, v.w, fmaf(-s.w, v.z, a.w));
+  a.x += fmaf(s.x, v.x, s.y * v.y);
+  a.y += fmaf(s.x, v.y, -(s.y * v.x));
+  a.z += fmaf(s.z, v.z, s.w * v.w);
+  a.w += fmaf(s.z, v.w, -(s.w * v.z));
 }
 __device__ __forceinline__ float2 axpy(float k, float2 a, float2 b) { return make_float2(fmaf(k, a.x, b.x), fmaf(k, a.y, b.y)); }
 __device__ __forceinline__ float4 axpy(float k, float4 a, float4 b) {
