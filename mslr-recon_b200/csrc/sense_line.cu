@@ -248,7 +248,7 @@ __device__ __forceinline__ float2 minus(float2 v) { return make_float2(-v.x, -v.
 __device__ __forceinline__ float4 minus(float4 v) { return make_float4(-v.x, -v.y, -v.z, -v.w); }
 
 template <int VEC, int CH>
-__global__ void __launch_bounds__(256) k_csum(const cf* __restrict__ T_, const cf* __restrict__ smod_, int nf, int ch,
+__global__ void __launch_bounds__(256, 4) k_csum(const cf* __restrict__ T_, const cf* __restrict__ smod_, int nf, int ch,
                                               int64_t nvox, cf* __restrict__ out_, const cf* __restrict__ ahy_,
                                               int t0, float scale, int add) {
   using V = typename Vals<VEC>::type;
