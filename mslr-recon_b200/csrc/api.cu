@@ -84,7 +84,6 @@ static void free_ctx(mslr_ctx* c) {
   if (c->d_ckpt) cudaFree(c->d_ckpt);
   if (c->d_gbuf) cudaFree(c->d_gbuf);
   if (c->d_vjpw) cudaFree(c->d_vjpw);
-  if (c->d_xsum) cudaFree(c->d_xsum);
   if (c->d_mz) cudaFree(c->d_mz);
   if (c->d_pthr) cudaFree(c->d_pthr);
   if (c->sn_stream) cudaStreamDestroy(c->sn_stream);

@@ -99,7 +99,6 @@ struct Ctx {
   int spec_lanes = 1;
   cudaStream_t sn_stream = nullptr;
   cudaEvent_t sn_fork = nullptr, sn_join = nullptr;
-  cf* d_xsum = nullptr;   // (Nt, nvox) summed image Σ_k X_k, when first needed
   // register-line SENSE kernels (sense_line.cu): every axis a 5-smooth length of 8..96
   bool line = false;
   uint32_t* d_mz = nullptr;   // sample bits over z: (Nt, ⌈Nz/32⌉, Ny·Nx)
@@ -127,7 +126,7 @@ struct Ctx {
   // POGM
   cf* d_U = nullptr;   // (Ns, Nt, nvox)
   cf* d_Z = nullptr;   // (Ns, Nt, nvox) pre-prox iterate z_i
-  cf* d_G = nullptr;   // (Nt, nvox) gradient
+  cf* d_G = nullptr;   // (Nt, nvox) gradient; either is also the summed image Σ_k X_k of a normal operator
   cf* d_Gold = nullptr;  // (Nt, nvox) previous gradient (only when bsig != 1)
   cf* d_Y = nullptr;     // (Ns, Nt, nvox) y_i of mom = :pgm / :fpgm (allocated on first use)
   double* d_part = nullptr;   // reduction partials
@@ -200,9 +199,6 @@ int normal_op_spec(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool sub
 // ---- sense_line.cu (tuned form, 5-smooth axes) -------------------------------------
 bool sense_line_setup(Ctx* c);
 int sense_line_bind(Ctx* c, cudaStream_t st);
-// Whether normal_op_line can take the call: false when there is no memory for
-// the summed image.
-int normal_op_line_ready(Ctx* c, const cf* X, int ns, const cf* g, bool* ready);
 int normal_op_line(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool subtract,
                    cudaStream_t st);
 int sense_forward_line(Ctx* c, const cf* x, cf* y, cudaStream_t st);

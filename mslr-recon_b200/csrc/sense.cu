@@ -428,11 +428,7 @@ int sense_adjoint(Ctx* c, const cf* y, cf* x, cudaStream_t st) {
 
 int normal_op(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool subtract,
               cudaStream_t st) {
-  if (c->line && !(c->spec && (c->spec_three || c->xy_tc))) {
-    bool ready;
-    if (int rc = normal_op_line_ready(c, X, ns, g, &ready)) return rc;
-    if (ready) return normal_op_line(c, X, ns, sstride, g, subtract, st);
-  }
+  if (c->line && !(c->spec && (c->spec_three || c->xy_tc))) return normal_op_line(c, X, ns, sstride, g, subtract, st);
   if (c->spec) return normal_op_spec(c, X, ns, sstride, g, subtract, st);
   if (c->fast) return normal_op_fast(c, X, ns, sstride, g, subtract, st);
   const Dims d = dims_of(c);

@@ -532,17 +532,6 @@ bool needs_sum(const Ctx* c, const cf* X, int ns, const cf* g) {
   return X < g + series && g < X + series && (ch < c->Nc || g != X);
 }
 
-// The buffer for it, a whole image series, made when first needed (by a
-// context of several scales when it is bound); a stream may be capturing.
-int sum_buffer(Ctx* c) {
-  if (c->d_xsum) return MSLR_OK;
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  MSLR_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
-  const int rc = dalloc(c, (void**)&c->d_xsum, (size_t)c->Nt * c->nvox * sizeof(cf));
-  MSLR_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
-  return rc;
-}
-
 }  // namespace
 
 bool sense_line_setup(Ctx* c) {
@@ -592,17 +581,6 @@ int sense_line_bind(Ctx* c, cudaStream_t st) {
   k_mask_z<<<grid, 256, 0, st>>>(c->d_mask, c->nwords, c->d_mz, c->N[0], c->N[1],
                                  plane_ops(c->N[0], c->N[1], c->N[2]) != nullptr, c->N[2], nw, c->Nt);
   MSLR_CUDA_TRY(cudaGetLastError());
-  // what every iteration over several scales needs; without it they go another way
-  if (c->Ns > 1 && sum_buffer(c)) cudaGetLastError();
-  return MSLR_OK;
-}
-
-int normal_op_line_ready(Ctx* c, const cf* X, int ns, const cf* g, bool* ready) {
-  *ready = true;
-  if (!needs_sum(c, X, ns, g) || !sum_buffer(c)) return MSLR_OK;
-  cudaGetLastError();
-  if (ns == 1) return MSLR_ERR_NOMEM;   // (the other forms can't write over their input either)
-  *ready = false;
   return MSLR_OK;
 }
 
@@ -610,8 +588,13 @@ int normal_op_line(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool sub
   const float scale = (float)(1.0 / (double)c->nvox);
   const cf* xs = X;
   if (needs_sum(c, X, ns, g)) {
-    if (int rc = image_sum(c, X, ns, sstride, c->d_xsum, st)) return rc;
-    xs = c->d_xsum;
+    // Into a buffer of the POGM state that holds nothing between calls: the
+    // gradient, or, when that is the result, z, which a step writes after it.
+    // (Whatever uses those two also uses T, so calls that may overlap on the
+    // GPU are none fewer.)
+    cf* sum = g == c->d_G ? c->d_Z : c->d_G;
+    if (int rc = image_sum(c, X, ns, sstride, sum, st)) return rc;
+    xs = sum;
   }
   c->prof_kernels = 4;
   return for_chunks(c, st, [&](const Pass& p) {

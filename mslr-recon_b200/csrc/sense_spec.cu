@@ -810,7 +810,7 @@ int normal_op_spec(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool sub
   c->prof_kernels = 3;
   float scale = (float)(1.0 / (double)c->nvox);
   const int Nc = c->Nc, Ny = c->N[1], Nz = c->N[2];
-  const int Ch = std::max(1, std::min(std::min(Nc, c->spec_ch), 8));   // coils per group, a cluster
+  const int Ch = std::max(1, std::min(Nc, c->spec_ch));             // coils per group
   int F = std::max(1, c->spec_fr);                                  // frames per chunk
   while (F > 1 && (int64_t)F * Ch > (int64_t)c->F * Nc) --F;        // within the k-space buffer
   int nwords = c->nwords;
