@@ -33,9 +33,8 @@ sys.path.insert(0, ROOT)
 
 WORKLOAD = "metric"
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch of
-# each kernel of the SENSE chunk (6 coils x 2 frames at 90x90x60) from the ncu
-# capture recorded in profiles/sense_line_kernels_90x90x60.md; ncu
-# flushes L2 before each launch, so these are cold-cache upper bounds (the
+# each kernel of the SENSE chunk (6 coils x 2 frames at 90x90x60) from an ncu
+# capture; ncu flushes L2 before each launch, so these are cold-cache upper bounds (the
 # timed loop finds most of the chunk's k-space in L2).
 TRAFFIC_PER_LAUNCH = {"pfwd": 32954880, "zmask": 47483648, "padj": 46829056, "csum": 81330176}
 

@@ -169,9 +169,9 @@ int mslr_normal_op(mslr_ctx* ctx, const void* X, int32_t ns_in, void* g,
  * subtract_data = 1 once, recording CUDA events on `stream` around every
  * kernel of every chunk, and returns in kernel_ms[0..3] the average device
  * time per launch of the chunk's kernels and in launches_per_kernel[0..3]
- * their launch counts.  Four-pass form (the default): [0] forward plane pass
+ * their launch counts.  Register-line form (the default): [0] forward plane pass
  * (coil maps × summed image, DFT_y, DFT_x), [1] z pass with the k-space mask,
- * [2] inverse plane pass with × conj(coil map), [3] coil combine.  Three-kernel
+ * [2] inverse plane pass, [3] coil combine with × conj(coil map).  Three-kernel
  * form (MSLR_SENSE_PATH=3, or the tensor-core plane pass): [0] forward z pass,
  * [1] plane pass, [2] adjoint z pass with the coil combine, [3] zero.  Both
  * arrays must hold 4 entries.  Synchronises `stream`.  MSLR_ERR_UNSUPPORTED
@@ -370,10 +370,9 @@ int mslr_pogm_grad(mslr_ctx* ctx, const void* X_true, int32_t niter, double L, d
 
 /* Autotuner (tuned and TF32 forms; no counterpart in the reference).  Times,
  * on the bound context, the launch shapes the library can choose freely —
- * coils per group × frames per chunk of the SENSE normal operator, its lanes
- * (one or two streams) and z-mask CTA variant (two per SM, one per SM, or
- * two per SM of fewer warps), the
- * split-K count of each single-patch scale's Gram, and the eigen stage's CTA
+ * coils per group × frames per chunk of the SENSE normal operator (the shape
+ * that the context starts with among them) and its lanes (one or two streams),
+ * the split-K count of each single-patch scale's Gram, and the eigen stage's CTA
  * variant of each scale with Gram side <= 384 (384 threads, two per SM, or
  * 1024 threads) — and keeps the fastest.  Runs at the end of mslr_bind when
  * the environment has MSLR_AUTOTUNE=1.  The choices change the order of
@@ -381,8 +380,8 @@ int mslr_pogm_grad(mslr_ctx* ctx, const void* X_true, int32_t niter, double L, d
  * before the first POGM step (it uses the POGM buffers as scratch), or the
  * captured iteration is captured again.  mslr_get_tuning writes {coils per
  * group, frames per chunk, split count of scale 0 .. Ns−1 (0: heuristic),
- * lanes, z-mask CTAs per SM, z-mask warps per CTA, eigen CTA threads of
- * scale 0 .. Ns−1}. */
+ * lanes, 2, 4, eigen CTA threads of scale 0 .. Ns−1}; the constants stand where
+ * the variant of the z pass stood, which has none any more. */
 int mslr_autotune(mslr_ctx* ctx, void* stream);
 int mslr_get_tuning(const mslr_ctx* ctx, int32_t* values, int32_t cap, int32_t* count);
 

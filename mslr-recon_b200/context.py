@@ -339,7 +339,8 @@ class MSLRContext:
 
     def tuning(self):
         """{'coils_per_group', 'frames_per_chunk', 'gram_splits': [per scale, 0 = heuristic],
-        'lanes', 'zmask_ctas_per_sm', 'zmask_warps', 'eig_threads': [per scale]}"""
+        'lanes', 'zmask_ctas_per_sm', 'zmask_warps', 'eig_threads': [per scale]}.  The two of
+        the z pass are always 2 and 4: it has no variants to choose from."""
         n = C.c_int32()
         vals = (C.c_int32 * 64)()
         self._chk(lib.mslr_get_tuning(self._h, vals, 64, C.byref(n)))

@@ -597,7 +597,7 @@ int mslr_get_tuning(const mslr_ctx* ctx, int32_t* values, int32_t cap, int32_t* 
   std::vector<int32_t> v = {ctx->spec_ch, ctx->spec_fr};
   for (const auto& g : ctx->scales) v.push_back(g.nsplit_tuned > 0 ? g.nsplit_tuned : 0);
   v.push_back(ctx->spec_lanes);
-  // the z pass: two or more resident CTAs per SM of four warps, not tuned
+  // the z pass has no variants to choose from: two entries that keep their place
   v.push_back(2);
   v.push_back(4);
   for (const auto& g : ctx->scales) v.push_back(g.n > 384 || g.eig_big ? 1024 : 384);

@@ -37,11 +37,11 @@
 // Split stage (9 <= n <= 384): three launches (two for the values alone) instead
 // of one, so that each phase has the shape it needs — phase 1 and the WY
 // blocks' T factors (k_tri_reg: the matrix in registers, n <= 128; k_tri_big:
-// panels), phases 2–3 (four CTAs per SM, all patches resident at once), and
-// phases 4–5 as k_wy_apply: 32 eigenvectors of one patch per CTA, held in
-// registers through every block update.  Phase 1 measured against k_eig's:
-// one patch of side 64 351 → 88 µs, 40 of 128 834 → 244 µs, 2250 of 128 8.0 →
-// 3.9 ms, 486 of 300 12.7 → 8.8 ms.
+// panels), phases 2–3 (k_pairs: two, four or eight CTAs per SM by side and
+// number of patches), and phases 4–5 as k_wy_apply: 64 eigenvectors of one patch
+// per CTA, held in registers through every block update.  Phase 1 measured
+// against k_eig's: one patch of side 64 351 → 71 µs, 40 of 128 834 → 219 µs, 2250
+// of 128 8.0 → 3.5 ms, 486 of 300 12.7 → 8.7 ms.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -1122,7 +1122,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
 // doubled components that a packed FMA would take directly (those are moves,
 // for which the FMAs leave issue slots), and the reflector's scalars that only
 // the vector phases need are worked out by their warps alone: 148 matrices of
-// side 128 252 -> 227 us, 216 of side 64 99 -> 94.
+// side 128 252 -> 227 us, 216 of side 64 99 -> 94 (by the profiler now 221 and 89,
+// 218 and 89 without the scaling).
 // CU columns per lane: tiles of 32 rows × 4·CU columns, one per warp.  Eight is
 // what 16 warps' registers hold at NT = 4; with four the smaller sides have
 // twice the warps, so the latencies of a tile pass overlap.

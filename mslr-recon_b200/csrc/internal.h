@@ -233,7 +233,7 @@ struct EigSegment {
   double* nuc = nullptr;   // when set: per-patch Σ √λ above the threshold only (no vectors, no W)
   double* lam_out = nullptr;   // when set: every eigenpair — V (row-major, G = V Λ Vᴴ) in zv
                                // and the eigenvalues (descending, np × n) here; threshold unused
-  double* side = nullptr;      // np × 6n FP64 scratch; when set (and 33 <= n <= 384), the stage
+  double* side = nullptr;      // np × 6n FP64 scratch; when set (and 9 <= n <= 384), the stage
                                // runs as three launches (tridiagonalise, eigenpairs of T, V = Q Z)
 };
 // Adds the number of kernels launched to *launches when given.

@@ -101,7 +101,8 @@ __device__ __forceinline__ void line_dft(const Ld& ld, const Tmp& tmp, const St&
 }
 
 // The plane [rows][cols] of g into shared memory with rows of RS values, every
-// copy in flight at once (8-byte copies: odd row strides); waits and synchronises.
+// copy in flight at once (8-byte copies: odd row strides); waits for the thread's
+// own copies, so that a barrier has to follow.
 template <int ROWS, int COLS, int RS, int THREADS>
 __device__ __forceinline__ void plane_in(cf* W, const cf* g) {
   constexpr int NW = THREADS / 32;

@@ -16,11 +16,11 @@
 // its waves alternate between the two; the plane passes are bound by latency
 // with 9 warps per SM (issue slots 35–45% busy, barrier, shared-memory and
 // load stalls), for which packed FP32 pairs cut the instructions by a third.
-// Measured at 90×90×60, 18 coils, 300 frames: 54.0 → 31.5 ms for the normal
+// Measured at 90×90×60, 18 coils, 300 frames: 54.0 → 30.9 ms for the normal
 // operator against two Stockham passes per axis through shared memory
 // (per 24 coil images: plane passes 80 / 83 → 50 / 46 µs, z pass 86 → 41 µs,
 // coil sum 25 → 30 µs with the maps' product moved into it); 75×64×45, 12
-// coils, 40 frames: 11.0 → 1.62 ms against generic passes.
+// coils, 40 frames: 11.0 → 1.47 ms against generic passes.
 #pragma once
 #include "fft_line.cuh"
 #include "internal.h"
