@@ -41,3 +41,5 @@ def test_more_than_2_31_patches():
     v[..., 1] = torch.arange(Nz, device="cuda")[:, None, None]
     P = R.img2patches(img, (1, 1, 1), (1, 1, 1))
     assert torch.equal(P.view(-1), img.view(-1))
+    del P, img, v
+    torch.cuda.empty_cache()   # 34 GB
