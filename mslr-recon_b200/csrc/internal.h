@@ -198,6 +198,7 @@ int normal_op_spec(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool sub
 
 // ---- sense_line.cu (tuned form, 5-smooth axes) -------------------------------------
 bool sense_line_setup(Ctx* c);
+bool sense_line_fixed(const Ctx* c);   // one launch a pass: no chunk shape to choose
 int sense_line_bind(Ctx* c, cudaStream_t st);
 int normal_op_line(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool subtract,
                    cudaStream_t st);

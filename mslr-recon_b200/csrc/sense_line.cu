@@ -475,10 +475,31 @@ struct Pass {   // one chunk of one coil group
 // L2.  Small images take several units of spec_fr frames per launch.
 constexpr double kChunkBytes = 24e6;
 
+// Up to this much k-space in all, every coil and frame goes in one launch a pass
+// on one stream: a launch is then little more than its latency, and three groups
+// of coils, or two lanes of which each has half the frames, are as many times
+// that.  16³, normal operator: 16 coils × 1 frame 74.5 → 28.2 us (three groups of
+// 6), 32 coils 147.5 → 28.1; 4 coils × 15 frames (2 MB, four chunks) 82.9 → 29.5;
+// 32 × 32 × 24 × 8 × 10 (16 MB) 34.2 → 29.5, at 32 MB 38.2 → 42.9.  With more than
+// one group, 12 coils at 64 MB 108.2 → 91.7, 16 coils 133.7 → 88, at 128 MB 146 →
+// 225 and 194 → 223.
+constexpr double kOneLaunchBytes = 16e6, kOneLaunchBytesGroups = 64e6;
+int coil_groups(int nc) { return nc <= 8 ? 1 : (nc + 5) / 6; }   // of equal size, at most 6 coils (8 when that is all)
+bool one_launch(const Ctx* c) {   // (the buffer holds it: F = Nt)
+  const double most = coil_groups(c->Nc) > 1 ? kOneLaunchBytesGroups : kOneLaunchBytes;
+  return (double)c->nvox * sizeof(cf) * c->Nc * c->Nt <= most;
+}
+
 // Coils per group and frames per launch of the next operator: within the
 // k-space buffer, which two lanes share when both fit; the launches of a
 // group equally large, and an even number of them on two lanes.
 void chunk_of(const Ctx* c, int* ch, int* fr, bool* lanes) {
+  if (one_launch(c)) {
+    *ch = c->Nc;
+    *fr = c->Nt;
+    *lanes = false;
+    return;
+  }
   *ch = std::max(1, std::min(c->Nc, c->spec_ch));
   const int64_t cap = (int64_t)c->F * c->Nc;
   const double img = (double)c->nvox * sizeof(cf) * *ch;
@@ -560,9 +581,8 @@ bool sense_line_setup(Ctx* c) {
     cudaGetLastError();
     return false;
   }
-  // coil groups of equal size, at most six coils (eight when that is all)
   if (!c->spec_three && !c->xy_tc) {
-    const int groups = c->Nc <= 8 ? 1 : (c->Nc + 5) / 6;
+    const int groups = one_launch(c) ? 1 : coil_groups(c->Nc);
     c->spec_ch = (c->Nc + groups - 1) / groups;
     c->spec_fr = 2;
   }
@@ -575,6 +595,8 @@ bool sense_line_setup(Ctx* c) {
   cudaGetLastError();
   return true;
 }
+
+bool sense_line_fixed(const Ctx* c) { return one_launch(c); }
 
 int sense_line_bind(Ctx* c, cudaStream_t st) {
   const int pl = c->N[0] * c->N[1], nw = (c->N[2] + 31) / 32;

@@ -888,7 +888,7 @@ int normal_op_spec(Ctx* c, const cf* X, int ns, int64_t sstride, cf* g, bool sub
 // list has not (75 × 64 × 45, 5 coils: 0.33 ms, in groups of 3 and 2 0.36).
 int tune_sense_chunks(Ctx* c, cudaStream_t st) {
   const bool three = c->spec && (c->spec_three || c->xy_tc);
-  if (!three && !c->line) return MSLR_OK;
+  if (!three && (!c->line || sense_line_fixed(c))) return MSLR_OK;
   const int64_t E = (int64_t)c->Nt * c->nvox;
   const int max_lanes = !three && c->sn_stream ? 2 : 1;
   float best = 1e30f;

@@ -1,7 +1,7 @@
 """The normal operator with its result over its input: out of a call on X is
-what it is with a buffer of its own, bit for bit, for one image series (more
-and fewer coils than a coil group holds; a compiled plane, other lines, and an
-image without line kernels) and for a stack of two."""
+what it is with a buffer of its own, bit for bit, for one image series (one
+coil group and several; a compiled plane, other lines, and an image without
+line kernels) and for a stack of two."""
 import numpy as np
 import pytest
 
@@ -9,13 +9,14 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("ns", [1, 2])
-@pytest.mark.parametrize("N,Nc", [((12, 15, 10), 12), ((12, 15, 10), 5), ((32, 32, 24), 13), ((14, 15, 10), 12)])
-def test_result_over_the_input(N, Nc, ns):
+@pytest.mark.parametrize("N,Nc,Nt", [((12, 15, 10), 12, 5), ((12, 15, 10), 12, 400), ((12, 15, 10), 5, 5),
+                                     ((32, 32, 24), 13, 26), ((14, 15, 10), 12, 5)])
+def test_result_over_the_input(N, Nc, Nt, ns):
     import torch
     import mslr_recon_b200 as M
     rng = np.random.default_rng(Nc)
     Nx, Ny, Nz = N
-    nvox, Nt = Nx * Ny * Nz, 5
+    nvox = Nx * Ny * Nz
     cn = lambda *s: torch.from_numpy((rng.standard_normal(s) + 1j * rng.standard_normal(s)).astype(np.complex64)).cuda()
     idx = np.stack([np.sort(rng.choice(nvox, nvox // 3, replace=False)) for _ in range(Nt)]).astype(np.int32)
     with M.MSLRContext(N, Nc, Nt, nvox // 3, [list(N)], [list(N)]) as ctx:
