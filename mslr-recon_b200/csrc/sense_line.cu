@@ -554,12 +554,26 @@ bool needs_sum(const Ctx* c, const cf* X, int ns, const cf* g) {
   return X < g + series && g < X + series && (ch < c->Nc || g != X);
 }
 
+// One frame of a small image without a compiled plane: six launches here, three
+// in sense_fast.cu, each little more than its latency (that form takes three a
+// frame, so from two frames on this one is no slower).  Normal operator here and
+// there: 8³, one coil 37.7 and 26.6 us; 16³, 4 coils 29.3 and 27.3; 24 × 20 × 18, 8
+// coils 31 and 28; 48 × 45 × 40, 2 coils 33 and 30; but 32 × 30 × 27, 8 coils 31 and
+// 48, 48 × 45 × 40, 4 coils 34 and 46, 12³, 16 coils 28 and 32 (8³ 28 and 25), and
+// large planes, 96 × 96 × 8, one coil 29 and 143.
+bool few_launches_win(const Ctx* c) {
+  const int64_t points = c->nvox * c->Nc;
+  return c->Nt == 1 && c->fast && c->N[0] * c->N[1] <= 4096 &&
+         points <= (c->Nc <= 2 ? 330000 : c->Nc <= 8 ? 105000 : 12000);
+}
+
 }  // namespace
 
 bool sense_line_setup(Ctx* c) {
   for (int d = 0; d < 3; ++d)
     if (!line_ops(c->N[d])) return false;
   const PlaneOps* po = plane_ops(c->N[0], c->N[1], c->N[2]);
+  if (!po && few_launches_win(c)) return false;
   if (po) {
     if (raise_dyn_smem(po->pfwd, (int)po->smem) || raise_dyn_smem(po->padj, (int)po->smem)) {
       cudaGetLastError();

@@ -37,11 +37,28 @@ def test_one_launch_a_pass(N, Nc, Nt, passes):
             assert ctx.launch_count() - before <= most
 
 
-@pytest.mark.parametrize("Nc,Nt", [(8, 43), (8, 44), (12, 115), (12, 116)])
-def test_both_sides_of_the_border(Nc, Nt):
-    """20 x 18 x 16 voxels: 15.9 and 16.2 MB, 63.6 and 64.1."""
+@pytest.mark.parametrize("N,Nc", [((8, 8, 8), 1), ((8, 8, 8), 16), ((16, 16, 16), 8), ((80, 8, 8), 4), ((48, 45, 40), 2)])
+def test_one_frame_of_a_small_image(N, Nc):
+    """Three launches, not one a pass of the lines."""
     import torch
-    ctx, smaps, y, idx, x = bound((20, 18, 16), Nc, Nt, np.random.default_rng(Nt))
+    ctx, _, y, _, x = bound(N, Nc, 1, np.random.default_rng(2))
+    with ctx:
+        xd, yd = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+        for call in (lambda: ctx.normal(xd), lambda: ctx.forward(xd), lambda: ctx.adjoint(yd)):
+            before = ctx.launch_count()
+            call()
+            assert ctx.launch_count() - before <= 3
+
+
+@pytest.mark.parametrize("N,Nc,Nt", [((20, 18, 16), 8, 43), ((20, 18, 16), 8, 44), ((20, 18, 16), 12, 115),
+                                     ((20, 18, 16), 12, 116), ((8, 8, 8), 1, 1), ((8, 8, 8), 1, 2), ((8, 8, 8), 20, 1), ((8, 8, 8), 24, 1), ((24, 20, 18), 8, 1),
+                                     ((24, 20, 18), 9, 1), ((20, 24, 50), 4, 1), ((20, 24, 54), 4, 1), ((64, 64, 40), 2, 1),
+                                     ((64, 72, 16), 2, 1)])
+def test_both_sides_of_each_border(N, Nc, Nt):
+    """15.9 and 16.2 MB, 63.6 and 64.1; one and two frames; one frame of 8 and 9
+    coils, on planes of 4096 points and more, and of fewer and more points."""
+    import torch
+    ctx, smaps, y, idx, x = bound(N, Nc, Nt, np.random.default_rng(Nt))
     s64, x64, y64 = smaps.astype(np.complex128), x.astype(np.complex128), y.astype(np.complex128)
     fwd = O.sense_forward(x64, s64, idx)
     with ctx:
