@@ -32,9 +32,9 @@
 // two CTAs run one tile's chain under the other's.  With chunks of 32 and one
 // CTA per SM, and tall rebuilds stored a row per lane (32 lines a store), 486
 // patches of 1000 × 300 took 3.34 ms to rebuild, 1.78 for their Grams and 0.60
-// for W; now 1.93, 1.42 and 0.44.  A Gram of at most 64 rows takes half of each
-// operand and half the columns of an MMA; with few patches its longer chain of
-// chunks then costs what it did (one 216 × 64: 17.4 -> 17.7 us, its rebuild
+// for W; now 1.93, 1.42 and 0.44.  Grams whose tiles have an SM each still go in
+// chunks of 32 (gram_umma_launch).  A Gram of at most 64 rows takes half of each
+// operand and half the columns of an MMA (one 216 × 64: 17.4 -> 15.2 us, its rebuild
 // 12.8 -> 10.7; 240 of 343 × 50: 48 -> 31 and 65 -> 42).
 // A stage is reused only after the tcgen05.commit of
 // the MMAs that read it has arrived on the stage's mbarrier.  The epilogue
@@ -60,18 +60,20 @@ namespace {
 
 constexpr int kTM = 128;          // output rows per CTA (TMEM lanes)
 constexpr int kTN = 128;          // output columns per CTA
-constexpr int kKc = 16;           // K elements per chunk
 constexpr int kThr = 256;
-constexpr int kTile = kTM * kKc;  // bf16 per planar tile
-constexpr int kPairs = kTile / 2 / kThr;   // (k, k+1) pairs per thread per operand: 4
 constexpr int kTmemCols = 256;
+// K elements per chunk (KC): 16, two CTAs per SM, or 32, one CTA (see gram_umma_launch)
+constexpr int tile_words(int KC) { return kTM * KC / 2; }         // bf16 pairs of a planar tile
+constexpr int pairs_of(int KC) { return tile_words(KC) / kThr; }   // per thread and operand: 4 or 8
+constexpr int ctas_of(int KC) { return KC == 16 ? 2 : 1; }
 
 enum { AR_H, AR_L, AI_H, AI_L, BR_H, BR_L, BI_H, BI_L, NOPS };
 
+template <int KC>
 struct USmem {
-  uint32_t op[2][NOPS][kTile / 2];   // two stages × 8 tiles of 128 × 16 bf16 (as bf16 pairs)
+  uint32_t op[2][NOPS][tile_words(KC)];   // two stages × 8 tiles of 128 × KC bf16 (as bf16 pairs)
   int rowA[kTM], rowB[kTN];
-  int kof[2][kKc];
+  int kof[2][KC];
   uint64_t bar[2];
   uint32_t tmem;
 };
@@ -82,16 +84,18 @@ __device__ __forceinline__ unsigned su32(const void* p) {
 
 // word index of the bf16 pair (r, k..k+1), k even, in a K-major unswizzled tile:
 // 8-row × 8-element core matrices of 128 bytes, k-adjacent cores 128 B apart
-// (LBO), 8-row groups 256 B apart (SBO)
+// (LBO), 8-row groups KC / 8 of them apart (SBO)
+template <int KC>
 __device__ __forceinline__ int pair_word(int r, int k) {
-  return ((r >> 3) * 2 + (k >> 3)) * 32 + (r & 7) * 4 + ((k & 7) >> 1);
+  return ((r >> 3) * (KC / 8) + (k >> 3)) * 32 + (r & 7) * 4 + ((k & 7) >> 1);
 }
 
-// shared-memory matrix descriptor (sm_100 layout): start, LBO = 128 B, SBO = 256 B,
-// version 1, no swizzle
+// shared-memory matrix descriptor (sm_100 layout): start, LBO = 128 B, SBO =
+// KC / 8 · 128 B, version 1, no swizzle
+template <int KC>
 __device__ __forceinline__ uint64_t sdesc(const void* p) {
   const uint64_t a = su32(p);
-  return ((a >> 4) & 0x3FFFull) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(256 >> 4) << 32) |
+  return ((a >> 4) & 0x3FFFull) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)((KC / 8 * 128) >> 4) << 32) |
          (1ull << 46);
 }
 
@@ -184,21 +188,23 @@ __device__ __forceinline__ void split_pair_f16(float x0, float x1, uint32_t& hi,
 // TF32 operands (the TF32 form): one FP32 plane per real / imaginary part,
 // each value rounded to TF32 (to nearest, ties away), in K-major unswizzled
 // core matrices of 8 rows × 4 values (128 bytes): k-adjacent cores 128 B apart
-// (LBO), 8-row groups 512 B apart (SBO).  A chunk of 16 K values is two
-// 8-value MMA steps.  Planes per stage: Ar, Ai, Br, Bi of 2048 words each.
-constexpr int kTfPlane = kTile;   // words per TF32 plane (128 rows × 16 values)
+// (LBO), 8-row groups KC / 4 of them apart (SBO).  A chunk of KC values is KC / 8
+// 8-value MMA steps.  Planes per stage: Ar, Ai, Br, Bi of 128 · KC words each.
+constexpr int tf_plane(int KC) { return kTM * KC; }   // words per TF32 plane
 
 __device__ __forceinline__ uint32_t to_tf32(float x) {
   uint32_t r;
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
   return r;
 }
+template <int KC>
 __device__ __forceinline__ int tf_word(int r, int k) {
-  return ((r >> 3) * 4 + (k >> 2)) * 32 + (r & 7) * 4 + (k & 3);
+  return ((r >> 3) * (KC / 4) + (k >> 2)) * 32 + (r & 7) * 4 + (k & 3);
 }
+template <int KC>
 __device__ __forceinline__ uint64_t sdesc_tf(const void* p) {
   const uint64_t a = su32(p);
-  return ((a >> 4) & 0x3FFFull) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(512 >> 4) << 32) |
+  return ((a >> 4) & 0x3FFFull) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)((KC / 4 * 128) >> 4) << 32) |
          (1ull << 46);
 }
 // instruction descriptor: TF32 × TF32 → F32, both K-major, M = 128; N is added by with_n
@@ -212,28 +218,32 @@ __device__ __forceinline__ void umma_tf(uint32_t dtmem, uint64_t a, uint64_t b, 
       "l"(a), "l"(b), "r"(id), "r"(acc ? 1u : 0u));
 }
 
-// Registers of one operand chunk: thread t holds pairs q = t + 256 i, i < 4, of
-// the 128 × 16 tile; pair q is (row r, k..k+1) of core c = q / 32, so pair i
-// lies in rows 32 i … 32 i + 31.  A Gram's tile of at most 64 rows takes the
-// first half only (NI = 2): what the stage holds beyond reaches no output.
+// Registers of one operand chunk: thread t holds pairs q = t + 256 i, i < KC / 4,
+// of the 128 × KC tile; pair q is (row r, k..k+1) of core c = q / 32, so pair i
+// lies in the i-th of KC / 4 equal groups of rows.  A Gram's tile of at most 64
+// rows takes the first half only (NI = KC / 8): what the stage holds beyond
+// reaches no output.
+template <int KC>
 struct Chunk {
-  cf v[kPairs][2];
+  cf v[pairs_of(KC)][2];
 };
 
+template <int KC>
 __device__ __forceinline__ void pair_rk(int i, int& r, int& k) {
+  constexpr int CK = KC / 8;   // cores along K
   const int q = threadIdx.x + kThr * i;
   const int c = q >> 5, w = q & 31;
-  r = (c >> 1) * 8 + (w >> 2);
-  k = (c & 1) * 8 + (w & 3) * 2;
+  r = (c / CK) * 8 + (w >> 2);
+  k = (c % CK) * 8 + (w & 3) * 2;
 }
 
-template <int NI>
-__device__ __forceinline__ void load_chunk(Chunk& ch, const cf* __restrict__ base, const int* row,
+template <int KC, int NI>
+__device__ __forceinline__ void load_chunk(Chunk<KC>& ch, const cf* __restrict__ base, const int* row,
                                            const int* kof) {
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
     int r, k;
-    pair_rk(i, r, k);
+    pair_rk<KC>(i, r, k);
     const int ro = row[r];
 #pragma unroll
     for (int d = 0; d < 2; ++d) {
@@ -244,14 +254,14 @@ __device__ __forceinline__ void load_chunk(Chunk& ch, const cf* __restrict__ bas
 }
 
 // chunk → planar hi / lo tiles (re_h, re_l, im_h, im_l), conjugated when conj
-template <bool F16, int NI>
-__device__ __forceinline__ void store_chunk(const Chunk& ch, uint32_t* rh, uint32_t* rl,
+template <int KC, bool F16, int NI>
+__device__ __forceinline__ void store_chunk(const Chunk<KC>& ch, uint32_t* rh, uint32_t* rl,
                                             uint32_t* ih, uint32_t* il, bool conj) {
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
     int r, k;
-    pair_rk(i, r, k);
-    const int w = pair_word(r, k);
+    pair_rk<KC>(i, r, k);
+    const int w = pair_word<KC>(r, k);
     const cf a = ch.v[i][0], b = ch.v[i][1];
     const float ai = conj ? -a.y : a.y, bi = conj ? -b.y : b.y;
     uint32_t h, l;
@@ -267,35 +277,34 @@ __device__ __forceinline__ void store_chunk(const Chunk& ch, uint32_t* rh, uint3
 }
 
 // One operand chunk into stage `stage` (B operand when isB), conjugated when conj.
-template <int MODE, int NI>
-__device__ __forceinline__ void store_operand(const Chunk& ch, uint32_t* stage, bool isB, bool conj) {
+template <int KC, int MODE, int NI>
+__device__ __forceinline__ void store_operand(const Chunk<KC>& ch, uint32_t* stage, bool isB, bool conj) {
   if constexpr (MODE == kTf32) {
-    uint32_t* re = stage + (isB ? 2 : 0) * kTfPlane;
-    uint32_t* im = stage + (isB ? 3 : 1) * kTfPlane;
+    uint32_t* re = stage + (isB ? 2 : 0) * tf_plane(KC);
+    uint32_t* im = stage + (isB ? 3 : 1) * tf_plane(KC);
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
       int r, k;
-      pair_rk(i, r, k);
-      const int w = tf_word(r, k);
+      pair_rk<KC>(i, r, k);
+      const int w = tf_word<KC>(r, k);
       const cf a = ch.v[i][0], b = ch.v[i][1];
       *reinterpret_cast<uint2*>(re + w) = make_uint2(to_tf32(a.x), to_tf32(b.x));
       *reinterpret_cast<uint2*>(im + w) = make_uint2(to_tf32(conj ? -a.y : a.y), to_tf32(conj ? -b.y : b.y));
     }
   } else {
-    const int o = isB ? BR_H : AR_H;
-    store_chunk<MODE == kF16, NI>(ch, stage + (o + 0) * (kTile / 2), stage + (o + 1) * (kTile / 2),
-                stage + (o + 2) * (kTile / 2), stage + (o + 3) * (kTile / 2), conj);
+    uint32_t* o = stage + (isB ? BR_H : AR_H) * tile_words(KC);
+    store_chunk<KC, MODE == kF16, NI>(ch, o, o + tile_words(KC), o + 2 * tile_words(KC), o + 3 * tile_words(KC), conj);
   }
 }
 
-// The 12 MMAs of stage st, one 16-element K step.
-template <bool GRAM, bool F16>
-__device__ __forceinline__ void issue_step(const USmem& s, int st, uint32_t dre, uint32_t dim, bool acc,
+// The 12 MMAs of a 16-element K step of stage st.
+template <int KC, bool GRAM, bool F16>
+__device__ __forceinline__ void issue_step(const USmem<KC>& s, int st, int step, uint32_t dre, uint32_t dim, bool acc,
                                            bool bSameAsA, int cols) {
-  const uint32_t* o = &s.op[st][0][0];
-  auto A = [&](int k) { return sdesc(o + k * (kTile / 2)); };
+  const uint32_t* o = &s.op[st][0][0] + step * 64;   // two cores a step
+  auto A = [&](int k) { return sdesc<KC>(o + k * tile_words(KC)); };
   const int bro = bSameAsA ? AR_H : BR_H;   // B operands: same tiles as A on diagonal Gram tiles
-  auto B = [&](int k) { return sdesc(o + (bro + (k - BR_H)) * (kTile / 2)); };
+  auto B = [&](int k) { return sdesc<KC>(o + (bro + (k - BR_H)) * tile_words(KC)); };
   const uint32_t P = with_n(idesc(false, F16), cols), N = with_n(idesc(true, F16), cols);
   // real part
   umma(dre, A(AR_H), B(BR_H), P, acc);
@@ -323,16 +332,16 @@ __device__ __forceinline__ void issue_step(const USmem& s, int st, uint32_t dre,
 }
 
 // All MMAs of the chunk in stage st (first: the accumulators start from zero).
-template <bool GRAM, int MODE>
-__device__ __forceinline__ void issue_chunk(const USmem& s, int st, uint32_t dre, uint32_t dim,
+template <int KC, bool GRAM, int MODE>
+__device__ __forceinline__ void issue_chunk(const USmem<KC>& s, int st, uint32_t dre, uint32_t dim,
                                             bool first, bool bSameAsA, int cols) {
   if constexpr (MODE == kTf32) {
     const uint32_t* o = &s.op[st][0][0];
     const int br = bSameAsA ? 0 : 2, bi = bSameAsA ? 1 : 3;
     const uint32_t P = with_n(idesc_tf(false), cols), N = with_n(idesc_tf(true), cols);
 #pragma unroll
-    for (int t = 0; t < kKc / 8; ++t) {
-      auto D = [&](int pl) { return sdesc_tf(o + pl * kTfPlane + t * 64); };   // +2 cores = 256 B
+    for (int t = 0; t < KC / 8; ++t) {
+      auto D = [&](int pl) { return sdesc_tf<KC>(o + pl * tf_plane(KC) + t * 64); };   // +2 cores = 256 B
       const bool acc = !first || t > 0;
       // Gram:    Re += Ar·Brᵀ + Ai·Biᵀ   Im += Ai·Brᵀ − Ar·Biᵀ
       // rebuild: Re += Ar·Brᵀ − Ai·Biᵀ   Im += Ar·Biᵀ + Ai·Brᵀ
@@ -347,7 +356,9 @@ __device__ __forceinline__ void issue_chunk(const USmem& s, int st, uint32_t dre
       }
     }
   } else {
-    issue_step<GRAM, MODE == kF16>(s, st, dre, dim, !first, bSameAsA, cols);
+#pragma unroll
+    for (int t = 0; t < KC / 16; ++t)
+      issue_step<KC, GRAM, MODE == kF16>(s, st, t, dre, dim, !first || t > 0, bSameAsA, cols);
   }
 }
 
@@ -367,20 +378,21 @@ struct Pending {
   // After a timed-out wait: thread 0 waits, with the default poll count, for
   // every commit still pending, so that no MMA reads shared memory or writes
   // tensor memory after the kernel frees them and returns.
-  __device__ void drain(USmem& s) const {
+  template <int KC>
+  __device__ void drain(USmem<KC>& s) const {
     if (c0 >= 0) mbar_wait(&s.bar[0], (unsigned)((c0 >> 1) & 1), kWaitPolls);
     if (c1 >= 0) mbar_wait(&s.bar[1], (unsigned)((c1 >> 1) & 1), kWaitPolls);
   }
 };
 
 // Main loop shared by both kernels: nch chunks; kofs(c, buf) fills s.kof[buf]
-// for chunk c (threads < kKc; chunks 0 and 1 are in place).  Returns false when
+// for chunk c (threads < KC; chunks 0 and 1 are in place).  Returns false when
 // a wait timed out.
 //
 // One chunk of the main loop: its operands, already in registers, into stage
 // c mod 2; the loads that `next` issues run under its MMAs.
-template <bool GRAM, int MODE, class Store, class Next>
-__device__ __forceinline__ void chunk_step(USmem& s, int c, bool& ok, Pending& pend, bool bSameAsA, int cols, int polls,
+template <int KC, bool GRAM, int MODE, class Store, class Next>
+__device__ __forceinline__ void chunk_step(USmem<KC>& s, int c, bool& ok, Pending& pend, bool bSameAsA, int cols, int polls,
                                            const Store& store, const Next& next) {
   const int st = c & 1;
   if (c >= 2 && ok) {
@@ -395,13 +407,14 @@ __device__ __forceinline__ void chunk_step(USmem& s, int c, bool& ok, Pending& p
   next();
   if (threadIdx.x == 0 && ok) {
     tc_fence_after();
-    issue_chunk<GRAM, MODE>(s, st, s.tmem, s.tmem + kTN, c == 0, bSameAsA, cols);
+    issue_chunk<KC, GRAM, MODE>(s, st, s.tmem, s.tmem + kTN, c == 0, bSameAsA, cols);
     umma_commit(&s.bar[st]);
     pend.committed(c);
   }
 }
 
-__device__ __forceinline__ bool mainloop_end(USmem& s, int nch, bool ok, Pending& pend, int polls) {
+template <int KC>
+__device__ __forceinline__ bool mainloop_end(USmem<KC>& s, int nch, bool ok, Pending& pend, int polls) {
   if (nch > 0 && ok) {
     const int l = nch - 1;
     if (mbar_wait(&s.bar[l & 1], (unsigned)((l >> 1) & 1), polls)) pend.observed(l);
@@ -415,8 +428,8 @@ __device__ __forceinline__ bool mainloop_end(USmem& s, int nch, bool ok, Pending
 }
 
 // Two operands, cols rows of B; load(c, buf) brings chunk c of both to registers.
-template <bool GRAM, int MODE, class KOfs, class Load>
-__device__ __forceinline__ bool mainloop(USmem& s, int nch, Chunk& ca, Chunk& cb, bool conjA, bool conjB,
+template <int KC, bool GRAM, int MODE, class KOfs, class Load>
+__device__ __forceinline__ bool mainloop(USmem<KC>& s, int nch, Chunk<KC>& ca, Chunk<KC>& cb, bool conjA, bool conjB,
                                          int cols, const KOfs& kofs, const Load& load, int polls) {
   bool ok = true;
   Pending pend;
@@ -424,11 +437,11 @@ __device__ __forceinline__ bool mainloop(USmem& s, int nch, Chunk& ca, Chunk& cb
   __syncthreads();
   for (int c = 0; c < nch; ++c) {
     if (c > 0 && c + 1 < nch) kofs(c + 1, (c + 1) & 1);
-    chunk_step<GRAM, MODE>(
+    chunk_step<KC, GRAM, MODE>(
         s, c, ok, pend, false, cols, polls,
         [&](uint32_t* stage) {
-          store_operand<MODE, kPairs>(ca, stage, false, conjA);
-          store_operand<MODE, kPairs>(cb, stage, true, conjB);
+          store_operand<KC, MODE, pairs_of(KC)>(ca, stage, false, conjA);
+          store_operand<KC, MODE, pairs_of(KC)>(cb, stage, true, conjB);
         },
         [&] {
           if (c + 1 < nch) load(c + 1, (c + 1) & 1);
@@ -439,19 +452,19 @@ __device__ __forceinline__ bool mainloop(USmem& s, int nch, Chunk& ca, Chunk& cb
 
 // One operand on both sides (a Gram's diagonal tiles): with the registers of
 // the second, two chunks of loads are under way.  load(x, c, buf): chunk c into x.
-template <int MODE, int NI, class KOfs, class Load>
-__device__ __forceinline__ bool mainloop_same(USmem& s, int nch, Chunk& c0, Chunk& c1, bool conj, int rows,
+template <int KC, int MODE, int NI, class KOfs, class Load>
+__device__ __forceinline__ bool mainloop_same(USmem<KC>& s, int nch, Chunk<KC>& c0, Chunk<KC>& c1, bool conj, int rows,
                                               const KOfs& kofs, const Load& load, int polls) {
   bool ok = true;
   Pending pend;
   if (nch > 0) load(c0, 0, 0);
   if (nch > 1) load(c1, 1, 1);
   __syncthreads();
-  auto step = [&](Chunk& x, int c) {
+  auto step = [&](Chunk<KC>& x, int c) {
     if (c + 2 < nch) kofs(c + 2, c & 1);
-    chunk_step<true, MODE>(
+    chunk_step<KC, true, MODE>(
         s, c, ok, pend, true, rows, polls,
-        [&](uint32_t* stage) { store_operand<MODE, NI>(x, stage, false, conj); },
+        [&](uint32_t* stage) { store_operand<KC, MODE, NI>(x, stage, false, conj); },
         [&] {
           if (c + 2 < nch) load(x, c + 2, c & 1);
         });
@@ -463,7 +476,8 @@ __device__ __forceinline__ bool mainloop_same(USmem& s, int nch, Chunk& c0, Chun
   return mainloop_end(s, nch, ok, pend, polls);
 }
 
-__device__ __forceinline__ void tmem_alloc(USmem& s) {
+template <int KC>
+__device__ __forceinline__ void tmem_alloc(USmem<KC>& s) {
   if ((threadIdx.x >> 5) == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
                      su32(&s.tmem)),
@@ -478,7 +492,8 @@ __device__ __forceinline__ void tmem_alloc(USmem& s) {
   }
 }
 
-__device__ __forceinline__ void tmem_free(USmem& s) {
+template <int KC>
+__device__ __forceinline__ void tmem_free(USmem<KC>& s) {
   tc_fence_before();
   __syncthreads();
   if ((threadIdx.x >> 5) == 0)
@@ -491,8 +506,8 @@ __device__ __forceinline__ void tmem_free(USmem& s) {
 // row and two rows per access: 16 consecutive columns leave in one store where
 // lane = row would touch 32 lines.  Uses the operand stages, which no MMA reads
 // any more; put(row, column, value) for this lane's share.
-template <class Put>
-__device__ __forceinline__ void by_columns(USmem& s, const cf (&v)[16], const Put& put) {
+template <int KC, class Put>
+__device__ __forceinline__ void by_columns(USmem<KC>& s, const cf (&v)[16], const Put& put) {
   cf* t = reinterpret_cast<cf*>(&s.op[0][0][0]) + (threadIdx.x >> 5) * (32 * 17);
   const int lane = threadIdx.x & 31;
   __syncwarp();
@@ -509,12 +524,13 @@ __device__ __forceinline__ void by_columns(USmem& s, const cf (&v)[16], const Pu
 // ---------------------------------------------------------------------------
 // kcols (or null): the patch's contraction stops at kcols[ip] values (the
 // eigenvectors beyond the rank are zero).
-template <int MODE>
-__global__ void __launch_bounds__(kThr, 2)
+template <int MODE, int KC>
+__global__ void __launch_bounds__(kThr, ctas_of(KC))
     k_gram_umma(const cf* __restrict__ img, PatchMap m, cf* __restrict__ out, int nsplit,
                 int lchunk, const int* __restrict__ kcols, DevWait dw) {
   extern __shared__ __align__(1024) unsigned char smraw[];
-  USmem& s = *reinterpret_cast<USmem*>(smraw);
+  USmem<KC>& s = *reinterpret_cast<USmem<KC>*>(smraw);
+  constexpr int kPairs = pairs_of(KC);
   int t = blockIdx.x, ta = 0;
   while (t > ta) {
     t -= ta + 1;
@@ -530,7 +546,7 @@ __global__ void __launch_bounds__(kThr, 2)
   const int l_begin = split * lchunk;
   const int l_end = min(kcols ? kcols[ip] : m.L, l_begin + lchunk);
   const int n = m.n;
-  const int nch = l_end > l_begin ? (l_end - l_begin + kKc - 1) / kKc : 0;
+  const int nch = l_end > l_begin ? (l_end - l_begin + KC - 1) / KC : 0;
   tmem_alloc(s);
   for (int r = threadIdx.x; r < kTM; r += kThr) {
     const int a = a0 + r, b = b0 + r;
@@ -538,8 +554,8 @@ __global__ void __launch_bounds__(kThr, 2)
     s.rowB[r] = (b < n) ? (int)(m.tall ? (int64_t)b * ts : patch_off(m, b)) : -1;
   }
   auto kofs = [&](int c, int buf) {
-    if (threadIdx.x < kKc) {
-      const int l = l_begin + c * kKc + threadIdx.x;
+    if (threadIdx.x < KC) {
+      const int l = l_begin + c * KC + threadIdx.x;
       s.kof[buf][threadIdx.x] = (l < l_end) ? (int)(m.tall ? patch_off(m, l) : (int64_t)l * ts) : -1;
     }
   };
@@ -549,23 +565,23 @@ __global__ void __launch_bounds__(kThr, 2)
   tc_fence_after();
   const cf* base = img + org;
   const bool cj = m.tall != 0;
-  Chunk ca, cb;
+  Chunk<KC> ca, cb;
   const int ra = min(kTM, n - a0);
   bool ok;
   if (diag) {
     auto one = [&](auto ni) {
       constexpr int NI = decltype(ni)::value;
-      return mainloop_same<MODE, NI>(
-          s, nch, ca, cb, cj, ra, kofs, [&](Chunk& x, int, int buf) { load_chunk<NI>(x, base, s.rowA, s.kof[buf]); },
-          dw.polls);
+      return mainloop_same<KC, MODE, NI>(
+          s, nch, ca, cb, cj, ra, kofs,
+          [&](Chunk<KC>& x, int, int buf) { load_chunk<KC, NI>(x, base, s.rowA, s.kof[buf]); }, dw.polls);
     };
     ok = ra <= kTM / 2 ? one(std::integral_constant<int, kPairs / 2>{}) : one(std::integral_constant<int, kPairs>{});
   } else {
     auto load = [&](int, int buf) {
-      load_chunk<kPairs>(ca, base, s.rowA, s.kof[buf]);
-      load_chunk<kPairs>(cb, base, s.rowB, s.kof[buf]);
+      load_chunk<KC, kPairs>(ca, base, s.rowA, s.kof[buf]);
+      load_chunk<KC, kPairs>(cb, base, s.rowB, s.kof[buf]);
     };
-    ok = mainloop<true, MODE>(s, nch, ca, cb, cj, cj, kTN, kofs, load, dw.polls);
+    ok = mainloop<KC, true, MODE>(s, nch, ca, cb, cj, cj, kTN, kofs, load, dw.polls);
   }
   cf* G = out + ((nsplit > 1) ? (int64_t)split * n * n : ip * (int64_t)n * n);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -609,14 +625,15 @@ __global__ void __launch_bounds__(kThr, 2)
     k_rebuild_umma(const cf* __restrict__ img, const cf* __restrict__ W, PatchMap m,
                    cf* __restrict__ out, int direct, DevWait dw) {
   extern __shared__ __align__(1024) unsigned char smraw[];
-  USmem& s = *reinterpret_cast<USmem*>(smraw);
+  constexpr int KC = 16, kPairs = pairs_of(KC);
+  USmem<KC>& s = *reinterpret_cast<USmem<KC>*>(smraw);
   const int a0 = blockIdx.x * kTM, l0 = blockIdx.y * kTN;
   const int64_t ip = blockIdx.z;
   const int n = m.n;
   const cf* Wp = W + ip * (int64_t)n * n;
   const int64_t org = patch_origin(m, ip);
   const int64_t ts = tstride(m);
-  const int nch = (n + kKc - 1) / kKc;
+  const int nch = (n + KC - 1) / KC;
   tmem_alloc(s);
   // A rows a: the stored W column a holds conj(W[a][·]); conjugated back on conversion.
   // B rows l: M[·][l] — tall: conj(img[b·ts + org + off(l)]); wide: img[l·ts + org + off(b)]
@@ -627,8 +644,8 @@ __global__ void __launch_bounds__(kThr, 2)
   }
   // the K offsets of A (b) and B (frame or voxel of b) differ: A uses kof + its own rows
   auto kofs = [&](int c, int buf) {
-    if (threadIdx.x < kKc) {
-      const int b = c * kKc + threadIdx.x;
+    if (threadIdx.x < KC) {
+      const int b = c * KC + threadIdx.x;
       s.kof[buf][threadIdx.x] = (b < n) ? (int)(m.tall ? (int64_t)b * ts : patch_off(m, b)) : -1;
     }
   };
@@ -638,22 +655,22 @@ __global__ void __launch_bounds__(kThr, 2)
   tc_fence_after();
   // A's element (a, b) is at Wp[a·n + b] (rows a·n in rowA, K offset b itself);
   // B's element (l, b) at org + rowB[l] + kof[b].
-  Chunk ca, cb;
+  Chunk<KC> ca, cb;
   auto load = [&](int c, int buf) {
 #pragma unroll
     for (int i = 0; i < kPairs; ++i) {
       int r, k;
-      pair_rk(i, r, k);
+      pair_rk<KC>(i, r, k);
       const int ro = s.rowA[r];
 #pragma unroll
       for (int d = 0; d < 2; ++d) {
-        const int b = c * kKc + k + d;
+        const int b = c * KC + k + d;
         ca.v[i][d] = (ro >= 0 && b < n) ? __ldg(Wp + ro + b) : make_float2(0.f, 0.f);
       }
     }
-    load_chunk<kPairs>(cb, img + org, s.rowB, s.kof[buf]);
+    load_chunk<KC, kPairs>(cb, img + org, s.rowB, s.kof[buf]);
   };
-  const bool ok = mainloop<false, MODE>(s, nch, ca, cb, true, m.tall != 0, min(kTN, m.L - l0), kofs, load, dw.polls);
+  const bool ok = mainloop<KC, false, MODE>(s, nch, ca, cb, true, m.tall != 0, min(kTN, m.L - l0), kofs, load, dw.polls);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int a = a0 + (warp & 3) * 32 + lane;
   // on a time-out the output tile is written as zeros and the error raised
@@ -713,10 +730,12 @@ int umma_prepare() {
   MSLR_CUDA_TRY(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(mu);
   if (dev < 64 && done[dev]) return MSLR_OK;
-  for (const void* k : {reinterpret_cast<const void*>(&k_gram_umma<kBf16>), reinterpret_cast<const void*>(&k_gram_umma<kTf32>),
-                        reinterpret_cast<const void*>(&k_gram_umma<kF16>), reinterpret_cast<const void*>(&k_rebuild_umma<kBf16>),
+  for (const void* k : {reinterpret_cast<const void*>(&k_gram_umma<kBf16, 16>), reinterpret_cast<const void*>(&k_gram_umma<kTf32, 16>),
+                        reinterpret_cast<const void*>(&k_gram_umma<kF16, 16>), reinterpret_cast<const void*>(&k_rebuild_umma<kBf16>),
                         reinterpret_cast<const void*>(&k_rebuild_umma<kTf32>)})
-    MSLR_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(USmem)));
+    MSLR_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(USmem<16>)));
+  for (const void* k : {reinterpret_cast<const void*>(&k_gram_umma<kBf16, 32>), reinterpret_cast<const void*>(&k_gram_umma<kTf32, 32>)})
+    MSLR_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(USmem<32>)));
   if (dev < 64) done[dev] = true;
   return MSLR_OK;
 }
@@ -727,12 +746,24 @@ int gram_umma_launch(const cf* img, const PatchMap& m, int64_t np, cf* out_or_pa
   const int T = (m.n + kTM - 1) / kTM;
   const int ntri = T * (T + 1) / 2;
   const dim3 grid(ntri, (unsigned)np, nsplit);
-  if (tf32)
-    k_gram_umma<kTf32><<<grid, kThr, sizeof(USmem), st>>>(img, m, out_or_part, nsplit, lchunk, kcols, dw);
-  else if (kcols)
-    k_gram_umma<kF16><<<grid, kThr, sizeof(USmem), st>>>(img, m, out_or_part, nsplit, lchunk, kcols, dw);
-  else
-    k_gram_umma<kBf16><<<grid, kThr, sizeof(USmem), st>>>(img, m, out_or_part, nsplit, lchunk, nullptr, dw);
+  // No more tiles than SMs: each has its SM to itself, and nothing runs under
+  // its chain of chunks, which should then be the shorter one of 32 elements, half
+  // the barriers and waits (the sums are the same, bit for bit).  One of 216 × 64
+  // 16.9 -> 14.7 us, 140 of 1000 × 64 71 -> 50, 140 of 512 × 128 48 -> 39, one of
+  // 1000 × 300 89 -> 78, 49 of 1000 × 200 (147 tiles) 93.6 -> 89.3, one of 100 000 ×
+  // 128 7.03 -> 5.11 ms, of 500 000 × 300 43.0 -> 36.1.  With two tiles per SM the
+  // shorter chunks are faster (486 of 1000 × 300: see above).
+  constexpr int kSms = 148;
+  if (!kcols && (int64_t)ntri * np * nsplit <= kSms) {
+    if (tf32) k_gram_umma<kTf32, 32><<<grid, kThr, sizeof(USmem<32>), st>>>(img, m, out_or_part, nsplit, lchunk, kcols, dw);
+    else k_gram_umma<kBf16, 32><<<grid, kThr, sizeof(USmem<32>), st>>>(img, m, out_or_part, nsplit, lchunk, kcols, dw);
+  } else if (tf32) {
+    k_gram_umma<kTf32, 16><<<grid, kThr, sizeof(USmem<16>), st>>>(img, m, out_or_part, nsplit, lchunk, kcols, dw);
+  } else if (kcols) {
+    k_gram_umma<kF16, 16><<<grid, kThr, sizeof(USmem<16>), st>>>(img, m, out_or_part, nsplit, lchunk, kcols, dw);
+  } else {
+    k_gram_umma<kBf16, 16><<<grid, kThr, sizeof(USmem<16>), st>>>(img, m, out_or_part, nsplit, lchunk, nullptr, dw);
+  }
   MSLR_CUDA_TRY(cudaGetLastError());
   return MSLR_OK;
 }
@@ -742,9 +773,9 @@ int rebuild_umma_launch(const cf* img, const cf* W, const PatchMap& m, int64_t n
   if (int rc = umma_prepare()) return rc;
   const dim3 grid((m.n + kTM - 1) / kTM, (m.L + kTN - 1) / kTN, (unsigned)np);
   if (tf32)
-    k_rebuild_umma<kTf32><<<grid, kThr, sizeof(USmem), st>>>(img, W, m, out, direct, dw);
+    k_rebuild_umma<kTf32><<<grid, kThr, sizeof(USmem<16>), st>>>(img, W, m, out, direct, dw);
   else
-    k_rebuild_umma<kBf16><<<grid, kThr, sizeof(USmem), st>>>(img, W, m, out, direct, dw);
+    k_rebuild_umma<kBf16><<<grid, kThr, sizeof(USmem<16>), st>>>(img, W, m, out, direct, dw);
   MSLR_CUDA_TRY(cudaGetLastError());
   return MSLR_OK;
 }
