@@ -121,6 +121,56 @@ __device__ __forceinline__ int sturm_less_f(const float* d, const float* e2, int
   return cnt;
 }
 
+// Which of several equal eigenvalues (to ctol) number e is, counted from the
+// first, or -1 when it stands alone; lam[0 … r) descending.
+__device__ __forceinline__ int tie_of(const double* lam, int r, int e, double ctol) {
+  int t = 0;
+  while (t < e && lam[e - t - 1] - lam[e - t] <= ctol) ++t;
+  return t > 0 || (e + 1 < r && lam[e] - lam[e + 1] <= ctol) ? t : -1;
+}
+
+// Twist of the vector of the t-th of several equal eigenvalues.  They come from
+// blocks of T that nothing couples (an unreduced T has none: a diagonal Gram, a
+// patch with zero voxels), so the smallest |γ| of all rows is the same row for
+// each of them.  The t-th takes the t-th block that has the eigenvalue, the row
+// of the smallest |γ| in it, and rows b0 … b1 of that block alone.  How far the
+// block's own eigenvalue is from λ̂ is the Rayleigh correction γ / ‖z‖², z its
+// vector: z_j = −up(j) z_{j+1} above the twist, −down(j) z_{j−1} below.
+struct Twist {
+  int k, b0, b1;
+};
+template <class Gamma, class Up, class Down>
+__device__ __noinline__ Twist tied_twist(int n, int t, const double* ee, double tnorm, Gamma gamma, Up up, Down down) {
+  const double tau = 2e-12 * tnorm, cut = 1e-15 * tnorm;
+  double best = 1e308;
+  int bk = 0, b0 = 0;
+  for (int k = 0; k < n; ++k) {
+    const double g = gamma(k);
+    if (g < best) {
+      best = g;
+      bk = k;
+    }
+    if (k == n - 1 || fabs(ee[k]) <= cut) {
+      if (best <= tau * n) {   // ‖z‖² <= n at the row of the largest |z_j|
+        double z = 1.0, s = 1.0;
+        for (int j = bk - 1; j >= b0; --j) {
+          z *= -up(j);
+          s = fma(z, z, s);
+        }
+        z = 1.0;
+        for (int j = bk + 1; j <= k; ++j) {
+          z *= -down(j);
+          s = fma(z, z, s);
+        }
+        if (best <= tau * s && t-- == 0) return {bk, b0, k};
+      }
+      best = 1e308;
+      b0 = k + 1;
+    }
+  }
+  return {-1, 0, n - 1};
+}
+
 struct Seg {
   int n;
   int64_t first;   // first block of the segment
@@ -915,16 +965,28 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
         kb = j;
       }
     }
+    int b0 = 0, b1 = n - 1;
+    if (const int t = tie_of(lam, r, tid, 1e-12 * fmax(tnorm, 1e-300)); t >= 0) {
+      const Twist w = tied_twist(
+          n, t, ee, tnorm,
+          [=](int k) { return fabs(dp[(int64_t)k * zs] + zd[(int64_t)k * zs] - (dd[k] - lm)); },
+          [=](int j) { return ee[j] / dp[(int64_t)j * zs]; }, [=](int j) { return ee[j - 1] / zd[(int64_t)j * zs]; });
+      if (w.k >= 0) {
+        kb = w.k;
+        b0 = w.b0;
+        b1 = w.b1;
+      }
+    }
     double nrm = 1.0, zp = 1.0;
     for (int j = kb - 1; j >= 0; --j) {   // z_j = −e_j z_{j+1} / D+_j
-      zp = -ee[j] * zp / dp[(int64_t)j * zs];
+      zp = j < b0 ? 0.0 : -ee[j] * zp / dp[(int64_t)j * zs];
       zd[(int64_t)j * zs] = zp;
       nrm += zp * zp;
     }
     zd[(int64_t)kb * zs] = 1.0;
     zp = 1.0;
     for (int j = kb + 1; j < n; ++j) {    // z_j = −e_{j−1} z_{j−1} / D−_j
-      zp = -ee[j - 1] * zp / zd[(int64_t)j * zs];
+      zp = j > b1 ? 0.0 : -ee[j - 1] * zp / zd[(int64_t)j * zs];
       zd[(int64_t)j * zs] = zp;
       nrm += zp * zp;
     }
@@ -2116,6 +2178,21 @@ __global__ void __launch_bounds__(TH, MINB) k_pairs(EigArgs g) {
           kb = k;
         }
         if (k + 1 < n) el = ee[k] * dp[(int64_t)k * zs];
+      }
+    }
+    if (const int t = tie_of(lam, r, tid, 1e-12 * fmax(tnorm, 1e-300)); t >= 0) {
+      const Twist w = tied_twist(
+          n, t, ee, tnorm,
+          [=](int k) {
+            const double em = k + 1 < n ? ee[k] * zd[(int64_t)(k + 1) * zs] : 0.0;
+            const double el = k > 0 ? ee[k - 1] * dp[(int64_t)(k - 1) * zs] : 0.0;
+            return fabs(dd[k] - lm - el - em);
+          },
+          [=](int j) { return dp[(int64_t)j * zs]; }, [=](int j) { return zd[(int64_t)j * zs]; });
+      if (w.k >= 0) {   // nothing goes past the block's ends
+        kb = w.k;
+        if (w.b0 > 0) dp[(int64_t)(w.b0 - 1) * zs] = 0.0;
+        if (w.b1 + 1 < n) zd[(int64_t)(w.b1 + 1) * zs] = 0.0;
       }
     }
     double nrm = 1.0;
