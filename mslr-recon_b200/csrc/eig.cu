@@ -289,6 +289,27 @@ __device__ __forceinline__ void col_sums(float* cr, float* ci, int lane) {
   ci[0] += __shfl_xor_sync(0xffffffffu, ci[0], 1);
 }
 
+// The power of two that takes a matrix's largest diagonal entry, which bounds a
+// Gram's entries, into [1, 2), and its inverse, with which d and e are scaled
+// back; reflectors and τ do not depend on it.  As it is when the entry is zero
+// or not finite.
+struct PowerOfTwo {
+  float up;
+  double down;
+  __device__ __forceinline__ explicit PowerOfTwo(float dmax) {
+    const int ex = __float_as_int(dmax) >> 23;   // (dmax >= 0)
+    const int k = dmax > 0.f && ex < 255 ? min(max(ex, 1), 253) : 127;
+    up = __int_as_float((254 - k) << 23);
+    down = __hiloint2double((k - 127 + 1023) << 20, 0);
+  }
+};
+
+// What is left of a column below its subdiagonal (and the subdiagonal's
+// imaginary part) is dropped, the column taken as it is, when its square is
+// at most this: 1e-16 of the scaled matrix, far below FP32's rounding of it.
+// Above, neither |u₁|² nor the sums with u lose bits to denormals.
+constexpr float kNoColumn = 1e-32f;
+
 // An off-diagonal tile (I, J), J < I, whose 32 columns all lie inside the
 // matrix (rows past n, in the last tile row, are masked per lane): the same
 // arithmetic as the general tile path without its per-element tests; the
@@ -535,6 +556,22 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
   const int i = tid;   // row owned by this thread (n <= kT)
   const int warp = tid >> 5, lane = tid & 31, nwarp = kT >> 5;
   // ---- 1. tridiagonalisation with delayed rank-2 updates ---------------------
+  // The matrix scaled by a power of two first (PowerOfTwo): columns of an unscaled
+  // one, squared, leave FP32 from 1e19 up and below 1e-19, where a pass over the
+  // triangle costs one step of n.
+  double down;
+  {
+    float q = i < n ? fabsf(__ldcg(&A[(int64_t)i * n + i].x)) : 0.f;
+    for (int o = 16; o > 0; o >>= 1) q = fmaxf(q, __shfl_xor_sync(0xffffffffu, q, o));
+    if (lane == 0) red1[warp] = q;
+    __syncthreads();
+    float dmax = 0.f;
+    for (int w = 0; w < nwarp; ++w) dmax = fmaxf(dmax, red1[w]);
+    const PowerOfTwo p(dmax);
+    down = p.down;
+    for (int c = warp; c < n; c += nwarp)
+      for (int r = c + lane; r < n; r += 32) A[(int64_t)c * n + r] = cscale(__ldcg(A + (int64_t)c * n + r), p.up);
+  }
   for (int q = tid; q < npad; q += kT) {
     sv[q] = make_float2(0.f, 0.f);
     svp[q] = make_float2(0.f, 0.f);
@@ -563,7 +600,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
     if (i >= k && i < n) {
       x = (k == 0) ? __ldcg(A + i) : scol[i];
       x = csub(x, cadd(cmul(vpi, cconj(wpk)), cmul(wpi, cconj(vpk))));
-      if (i == k) dd[k] = (double)x.x;
+      if (i == k) dd[k] = (double)x.x * down;
     }
     if (i == k + 1) s_x = x;
     const float xn = block_sum((i >= k + 2 && i < n) ? cabs2(x) : 0.f, red0);
@@ -572,7 +609,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
     {
       const float ar = s_x.x, ai = s_x.y;
       float bt;
-      if (xn == 0.f && ai == 0.f) {
+      if (xn + ai * ai <= kNoColumn) {   // (false for NaN)
         bt = ar;
         tr = ti = 0.f;
         sr = 1.f;
@@ -587,8 +624,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
         si = -zi / den;
       }
       if (i == k + 1) {
-        ee[k] = (double)bt;
-        ee2[k] = (double)bt * (double)bt;
+        ee[k] = (double)bt * down;
+        ee2[k] = ee[k] * ee[k];
         taur[k] = tr;
         taui[k] = ti;
       }
@@ -772,7 +809,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_eig(EigArgs g) {
     cf x = __ldcg(A + (int64_t)(n - 1) * n + (n - 1));
     const cf vpk = svp[n - 1], wpk = swp[n - 1];
     x = csub(x, cadd(cmul(vpk, cconj(wpk)), cmul(wpk, cconj(vpk))));
-    dd[n - 1] = (double)x.x;
+    dd[n - 1] = (double)x.x * down;
     ee[n - 1] = 0.0;
     ee2[n - 1] = 0.0;
   }
@@ -1201,27 +1238,6 @@ struct TriVec {
   float red0[4], redt[NT * NTC];
   cf x1;
 };
-
-// The power of two that takes a matrix's largest diagonal entry, which bounds a
-// Gram's entries, into [1, 2), and its inverse, with which d and e are scaled
-// back; reflectors and τ do not depend on it.  As it is when the entry is zero
-// or not finite.
-struct PowerOfTwo {
-  float up;
-  double down;
-  __device__ __forceinline__ explicit PowerOfTwo(float dmax) {
-    const int ex = __float_as_int(dmax) >> 23;   // (dmax >= 0)
-    const int k = dmax > 0.f && ex < 255 ? min(max(ex, 1), 253) : 127;
-    up = __int_as_float((254 - k) << 23);
-    down = __hiloint2double((k - 127 + 1023) << 20, 0);
-  }
-};
-
-// What is left of a column below its subdiagonal (and the subdiagonal's
-// imaginary part) is dropped, the column taken as it is, when its square is
-// at most this: 1e-16 of the scaled matrix, far below FP32's rounding of it.
-// Above, neither |u₁|² nor the sums with u lose bits to denormals.
-constexpr float kNoColumn = 1e-32f;
 
 // zlarfg with α = (ar, ai) and ‖x‖² = xn: Hᴴ (α, x) = (β, 0), H = I − τ v vᴴ, β
 // real, v = (1, x / u₁), u₁ = α − β.  The root and its reciprocal come from one

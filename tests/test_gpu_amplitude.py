@@ -15,7 +15,7 @@ from oracle import mslr_oracle as O
 
 pytestmark = pytest.mark.gpu
 
-SIDES = [20, 64, 90, 100, 128, 130, 300, 301]
+SIDES = [5, 8, 20, 64, 90, 100, 128, 130, 300, 301, 400]
 POWERS = [-30, -20, -13, 14, 20, 40]
 
 
@@ -79,6 +79,24 @@ def test_columns_of_very_different_size(n):
     rng = np.random.default_rng(11 * n)
     X = cn(rng, n + 40, n)
     X[:, n // 2:] *= 1e-11
+    X = X.astype(np.complex64)
+    out = M.SVST(torch.from_numpy(X).cuda(), 2.0).cpu().numpy()
+    ref = O.svst(X.astype(np.complex128), 2.0)
+    assert np.linalg.norm(out - ref) <= 9.2e-5 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("tiny", [1e-12, 1e-17, 1e-20, 1e-35])
+@pytest.mark.parametrize("n", SIDES)
+def test_rows_that_have_faded(n, tiny):
+    """Rows down to 1e-35, as thresholded voxels outside the object have: the
+    squares of what couples them leave FP32."""
+    import torch
+    import mslr_recon_b200 as M
+    rng = np.random.default_rng(13 * n)
+    X = cn(rng, n, n + 70)
+    X[n - 2] *= 1e-13
+    X[n - 1] *= tiny
+    X[:, ::7] *= tiny
     X = X.astype(np.complex64)
     out = M.SVST(torch.from_numpy(X).cuda(), 2.0).cpu().numpy()
     ref = O.svst(X.astype(np.complex128), 2.0)
